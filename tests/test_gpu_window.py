@@ -1,0 +1,73 @@
+"""The window probe (kernels/window_probe.cuh) against the oracle at the sizes
+where it can go wrong: every slice width a remainder can take, hash counts of
+each unroll and of none, segments from 16 to 1,024 cells, hash partitions,
+multi-member groups, batches at the key count where it takes over, and keys
+that all fall into one bucket. Counts are whole numbers: equality."""
+import numpy as np
+import pytest
+
+import helpers
+from helpers import build_index, dna, sample_reads
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    dict(colors=250, H=2, b=8, k=25),                     # 16 chunks, ragged last field
+    dict(colors=300, H=4, b=8, k=31, seg=16),             # 16 + 2 + 1 chunks, short segments
+    dict(colors=700, H=3, b=4, k=25, groups="0,1,2;7,9"),
+    dict(colors=260, H=8, b=16, k=31, max_size="256KiB"),  # hash partitions
+    dict(colors=300, H=5, b=32, k=25, max_size="1MiB"),
+    dict(colors=600, H=16, b=8, k=31),
+    dict(colors=270, H=32, b=8, k=21),
+    dict(colors=300, H=4, b=8, k=31, seg=256),            # four-chunk slices
+    dict(colors=300, H=3, b=8, k=31, seg=1024),           # one-chunk slices
+    dict(colors=300, H=4, b=8, k=31, seg=4096),           # no window fits: the wide probe
+]
+
+
+def _index(d, colors, **opts):
+    lengths = [2000 if c % 3 == 0 else (4000 if c % 3 == 1 else 9000) for c in range(colors)]
+    (d / "g").mkdir()
+    lines = []
+    for c, n in enumerate(lengths):
+        p = d / "g" / f"g{c}.fa"
+        helpers.write_fasta(p, [dna(n, 31 + c)])
+        lines.append(f"g{c}\t{p}")
+    (d / "fof.tsv").write_text("\n".join(lines) + "\n")
+    build_index(d / "fof.tsv", d / "index", min_docs=1, **opts)
+    return d / "index", [dna(n, 31 + c) for c, n in enumerate(lengths)]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(f"{k}{v}" for k, v in c.items()))
+def test_window_probe_matches_oracle(gpu, oracle, tmp_path, case):
+    import zindex_b200 as zx
+
+    ix, genomes = _index(tmp_path, **case)
+    rng = np.random.default_rng(5)
+    batches = [sample_reads(genomes, rng, 3000, 150, n_runs=0.1),
+               sample_reads(genomes, rng, 1, 150),
+               [b"A" * 9000] * 20 + sample_reads(genomes, rng, 400, 150),  # one k-mer over and over
+               [genomes[2][:2000]] * 200]
+    with zx.Index(ix) as index:
+        for recover in (True, False):
+            for reads in batches:
+                bases, offsets = zx.pack_records(reads)
+                want, want_total = oracle.query_records(ix, bases, offsets, recover=recover)
+                got, total = index.query_records(bases, offsets, recover=recover)
+                assert total == want_total
+                np.testing.assert_array_equal(got, want)
+
+
+def test_window_probe_around_its_threshold(gpu, oracle, tmp_path):
+    """Batches growing through the key count from which windows are used."""
+    import zindex_b200 as zx
+
+    ix, genomes = _index(tmp_path, colors=256, H=4, b=8, k=31)
+    rng = np.random.default_rng(6)
+    with zx.Index(ix) as index:
+        for reads in (10, 50, 100, 130, 150, 200, 400, 800):
+            bases, offsets = zx.pack_records(sample_reads(genomes, rng, reads, 151))
+            want, want_total = oracle.query_records(ix, bases, offsets)
+            got, total = index.query_records(bases, offsets)
+            assert total == want_total
+            np.testing.assert_array_equal(got, want)

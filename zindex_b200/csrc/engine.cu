@@ -16,6 +16,7 @@
 #include "kernels/record_hits.cuh"
 #include "kernels/strobes.cuh"
 #include "kernels/wide_probe.cuh"
+#include "kernels/window_probe.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -145,8 +146,10 @@ FusedFn fused_for(int mode, const QueryLaunch& l) {
 constexpr size_t kSmallColors = 1024;
 
 using WideFn = void (*)(const DevIndex*, const ColorLoc*, const uint64_t*,
-                       const unsigned long long*, int, uint32_t, uint32_t*, uint64_t*,
+                       const unsigned long long*, int, uint32_t, uint64_t*,
                        unsigned long long*, WideRound);
+using WindowFn = void (*)(const DevIndex*, WinPlan, const uint64_t*, const unsigned long long*,
+                         const uint32_t*, uint64_t*, unsigned long long*);
 using DenseExtractFn = void (*)(BatchView, SeedParams, uint64_t*, unsigned long long*, int,
                                 WideRound);
 
@@ -163,6 +166,17 @@ WideFn wide_fn(int J, int HQ, int T) {
   if (J == 2) return HQ == 8 ? wide_probe_kernel<2, 1, 8, 2> : wide_probe_kernel<2, 2, 4, 2>;
   if (J == 3) return wide_probe_kernel<3, 1, 4, 2>;
   return wide_probe_kernel<4, 1, 4, 2>;
+}
+
+// Window probe by hash count: exact unrolls of the common ones.
+WindowFn window_fn(int hashes) {
+  switch (hashes) {
+    case 2: return window_probe_kernel<2>;
+    case 3: return window_probe_kernel<3>;
+    case 4: return window_probe_kernel<4>;
+    case 8: return window_probe_kernel<8>;
+    default: return window_probe_kernel<0>;
+  }
 }
 
 DenseExtractFn dense_extract_for(int mode) {
@@ -874,9 +888,74 @@ void Engine::load(const std::string& dir, const OpenOptions& options) {
   DevIndex norec = host_ix_;
   norec.rec = DevRecovery{nullptr, nullptr, nullptr, 0};
   cuda_check(cudaMemcpy(d_ix_norec_, &norec, sizeof(DevIndex), cudaMemcpyHostToDevice), "upload");
+  plan_windows();
   launch_ = default_launch();
   ws_ = make_workspace();
   load_s_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
+}
+
+void Engine::plan_windows() {
+  // Buckets of the ordered rounds: about two per segment of the largest
+  // class, 2^14 (so that the sort's counters are not contended) to 2^18.
+  uint64_t most = 1;
+  order_.seed = m_.seed;
+  for (uint32_t c = 0; c < host_ix_.classes; ++c) {
+    const DevClass& C = host_ix_.cls[c];
+    most = std::max<uint64_t>(most, C.slots / C.seg - (uint64_t)m_.hashes + 1);
+    order_.parts = std::max(order_.parts, C.partitions);
+  }
+  int pbits = 0;
+  while ((1u << pbits) < order_.parts) ++pbits;
+  order_.fbits = 14;
+  while (order_.fbits + pbits < kMaxOrderBits && (1ull << order_.fbits) < 2 * most) ++order_.fbits;
+  if (order_.fbits + pbits > kMaxOrderBits || !wide_eligible(8)) return;
+
+  // Slices of every class: the widest power of two (up to 16 chunks, a lane
+  // each) whose window of H segments and one bucket fits the block's shared
+  // memory, the remainder cut where the sum of (width + 2) per slice is
+  // least (2: a slice's own hashing of a seed, in chunks).
+  const int H = m_.hashes;
+  const uint32_t tile = WinSmem::tile_bytes(H);
+  std::vector<WinSlice> slices;
+  uint32_t weights = 0;
+  uint64_t row_chunks = 0, chunk_rows = 0;  // chunks of a seed's row, of all rows
+  for (uint32_t c = 0; c < host_ix_.classes; ++c) {
+    const DevClass& C = host_ix_.cls[c];
+    const uint64_t count = C.slots / C.seg - (uint64_t)H + 1;
+    const uint64_t span = (count + (1ull << order_.fbits) - 1) >> order_.fbits;
+    int top = 4;
+    while (top >= 0 && tile / ((C.seg << top) * 16) < (uint64_t)H + span) --top;
+    if (top < 0) return;  // segments too long for a window: the wide probe runs every round
+    std::vector<uint32_t> cost(C.fp_chunks + 1, 0), width(C.fp_chunks + 1, 0);
+    for (uint32_t left = 1; left <= C.fp_chunks; ++left) {
+      cost[left] = ~0u;
+      for (int lw = 0; lw <= top; ++lw) {
+        const uint32_t w = 1u << lw, rest = left > w ? cost[left - w] : 0;
+        if (w + 2 + rest < cost[left]) {
+          cost[left] = w + 2 + rest;
+          width[left] = (uint32_t)lw;
+        }
+      }
+    }
+    for (uint32_t k = 0; k < C.fp_chunks;) {
+      const uint32_t lw = width[C.fp_chunks - k], w = 1u << lw;
+      const uint32_t n = std::min(w, C.fp_chunks - k);
+      slices.push_back(WinSlice{c, k, n, lw, w + 2, weights});
+      weights += w + 2;
+      k += n;
+    }
+    row_chunks += C.fp_chunks;
+    chunk_rows += (uint64_t)C.fp_chunks * C.slots * C.partitions;
+  }
+  dev_alloc(&d_win_slices_, slices.size(), "window slices");
+  allocations_.push_back(d_win_slices_);
+  cuda_check(cudaMemcpy(d_win_slices_, slices.data(), slices.size() * sizeof(WinSlice),
+                        cudaMemcpyHostToDevice),
+             "upload");
+  win_slices_ = (uint32_t)slices.size();
+  win_weights_ = weights;
+  // Windows pay once a round's row reads are a few times the rows copied.
+  win_min_keys_ = std::max<uint64_t>(1, 4 * chunk_rows / (row_chunks * (uint64_t)H));
 }
 
 uint64_t Engine::gather_sector_bytes_per_seed() const {
@@ -1330,7 +1409,7 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
     cuda_check(cudaGetLastError(), "reduce_counters_kernel");
   };
   if (wide_form(l)) {
-    run_wide(ws, bv, tiles_bound, recover, counts, total, 0, s);
+    run_wide(ws, bv, tiles_bound, nbases, recover, counts, total, 0, s);
     if (timed) cuda_check(cudaEventRecord(ev_end_, s), "cudaEventRecord");
     return;
   }
@@ -1371,8 +1450,8 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   if (timed) cuda_check(cudaEventRecord(ev_end_, s), "cudaEventRecord");
 }
 
-void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, bool recover,
-                      uint64_t* counts, unsigned long long* total, uint32_t segments,
+void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, uint64_t max_keys,
+                      bool recover, uint64_t* counts, unsigned long long* total, uint32_t segments,
                       cudaStream_t s, double prune_ratio) {
   // Rounds of up to kSplitTiles tiles; per round the extraction kernel
   // appends the tiles' seeds to one dense list (segmented: each segment's
@@ -1399,7 +1478,6 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
   // A tile holds at most 256 seeds: one probe round.
   const int wblocks = l.blocks > 0 ? std::min(l.blocks, blocks_cap)
                                    : (int)std::min<uint64_t>(blocks_cap, std::max<uint64_t>(tiles_bound, 1));
-  const uint32_t colors = (uint32_t)m_.colors.size();
   const uint64_t rounds = (tiles_bound + kSplitTiles - 1) / kSplitTiles;
   // Several rounds: extraction (compute-bound) of round r + 1 runs on the
   // auxiliary stream beside the probe (memory-bound) of round r, the rounds
@@ -1431,6 +1509,8 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
     const bool ordered = l.order && !segments;
     if (ordered) ensure_order_capacity(ws, b);
     sg.interleave = !segments && l.order == 2 ? 1u : 0u;
+    const bool windows = l.order == 1 && !segments && win_slices_ && max_keys >= win_min_keys_;
+    if (windows) sg.max_keys = win_min_keys_;
     if (overlap && r >= 2)
       cuda_check(cudaStreamWaitEvent(xs, ws.wide_probe[b], 0), "cudaStreamWaitEvent");
     if (segments)
@@ -1441,16 +1521,16 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
     cuda_check(cudaGetLastError(), "extract_dense_kernel");
     const uint64_t* probe_keys = keys;
     if (ordered) {
-      // Counting sort of the round's keys by their first hash's top bits
-      // (row-address order of every class), the key count read on the device.
+      // Counting sort of the round's keys by partition and their first
+      // hash's top bits (row-address order of every class), the key count
+      // read on the device.
       const int ogrid = sms_ * 8;
-      cuda_check(cudaMemsetAsync(ws.wide_hist[b], 0, kOrderBuckets * 4, xs), "memset");
-      order_count_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + b, host_ix_.seed,
-                                                ws.wide_hist[b]);
+      cuda_check(cudaMemsetAsync(ws.wide_hist[b], 0, order_.buckets() * 4ull, xs), "memset");
+      order_count_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + b, order_, ws.wide_hist[b]);
       cuda_check(cudaGetLastError(), "order_count_kernel");
-      order_scan_kernel<<<1, 1024, 0, xs>>>(ws.wide_hist[b]);
+      order_scan_kernel<<<1, 1024, 0, xs>>>(ws.wide_hist[b], order_.buckets());
       cuda_check(cudaGetLastError(), "order_scan_kernel");
-      order_scatter_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + b, host_ix_.seed,
+      order_scatter_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + b, order_,
                                                   ws.wide_hist[b], ws.wide_keys_alt[b]);
       cuda_check(cudaGetLastError(), "order_scatter_kernel");
       probe_keys = ws.wide_keys_alt[b];
@@ -1464,15 +1544,26 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
       cuda_check(cudaEventRecord(ws.wide_ext[b], xs), "cudaEventRecord");
       cuda_check(cudaStreamWaitEvent(s, ws.wide_ext[b], 0), "cudaStreamWaitEvent");
     }
-    wfn<<<wblocks, l.warps * 32, smem, s>>>(recover ? d_ix_rec_ : d_ix_norec_, d_color_loc_,
-                                            probe_keys, ws.wide_cursor + b, l.smem_counters,
-                                            wteam, ws.partial, counts, segments ? nullptr : total,
-                                            sg);
+    const DevIndex* dix = recover ? d_ix_rec_ : d_ix_norec_;
+    wfn<<<wblocks, l.warps * 32, smem, s>>>(dix, d_color_loc_, probe_keys, ws.wide_cursor + b,
+                                            l.smem_counters, wteam, counts,
+                                            segments ? nullptr : total, sg);
     cuda_check(cudaGetLastError(), "wide_probe_kernel");
-    if (l.smem_counters && !segments) {
-      reduce_counters_kernel<<<std::max(1u, (colors + 255) / 256), 256, 0, s>>>(
-          ws.partial, wblocks, colors, counts);
-      cuda_check(cudaGetLastError(), "reduce_counters_kernel");
+    if (windows) {
+      WindowFn winfn = window_fn(m_.hashes);
+      cuda_check(cudaFuncSetAttribute(winfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kWinBlockBytes),
+                 "cudaFuncSetAttribute");
+      const WinPlan plan{d_win_slices_, win_slices_, win_weights_, order_, win_min_keys_};
+      const int wgrid = l.blocks > 0 ? std::min(l.blocks, 2 * sms_) : 2 * sms_;
+      winfn<<<wgrid, kWinThreads, kWinBlockBytes, s>>>(dix, plan, probe_keys, ws.wide_cursor + b,
+                                                       ws.wide_hist[b], counts, total);
+      cuda_check(cudaGetLastError(), "window_probe_kernel");
+      if (recover && host_ix_.rec.bits) {
+        recover_kernel<<<sms_ * 8, 256, 0, s>>>(dix, d_color_loc_, probe_keys, ws.wide_cursor + b,
+                                                win_min_keys_, counts);
+        cuda_check(cudaGetLastError(), "recover_kernel");
+      }
     }
     if (overlap) cuda_check(cudaEventRecord(ws.wide_probe[b], s), "cudaEventRecord");
   }
@@ -1481,7 +1572,7 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
 void Engine::ensure_order_capacity(Workspace& ws, int b) {
   if (ws.wide_keys_alt[b]) return;
   dev_alloc(&ws.wide_keys_alt[b], (uint64_t)kSplitTiles * kTileWindows, "round keys in order");
-  dev_alloc(&ws.wide_hist[b], kOrderBuckets, "round order buckets");
+  dev_alloc(&ws.wide_hist[b], order_.buckets(), "round order buckets");
   ws.release_graphs();
 }
 
@@ -1616,7 +1707,7 @@ void Engine::query_segments(Workspace& ws, const uint8_t* bases, uint64_t nbases
     BatchView bv{PackedView{ws.packed, ws.invalid}, offsets, ws.tiles, ws.tile_first + records,
                  ws.fstate};
     const uint64_t tiles_bound = nbases / kTileWindows + records + nbases / kFindereTask + 1;
-    run_wide(ws, bv, tiles_bound, recover, counts, totals, segments, s, prune_ratio);
+    run_wide(ws, bv, tiles_bound, nbases, recover, counts, totals, segments, s, prune_ratio);
     return;
   }
   QueryLaunch l = fused_launch(launch_);

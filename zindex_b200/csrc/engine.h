@@ -19,6 +19,7 @@
 namespace zx {
 struct ColorLoc;
 struct BatchView;
+struct WinSlice;
 }
 
 namespace zx {
@@ -280,9 +281,13 @@ class Engine {
   // per-round cursors already in ws).
   // prune_ratio > 0 (segmented per-record reports): threshold pruning of the
   // colours that cannot reach count / total >= prune_ratio.
-  void run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, bool recover,
-                uint64_t* counts, unsigned long long* total, uint32_t segments, cudaStream_t s,
-                double prune_ratio = 0.0);
+  // max_keys: no more seeds than this in the batch (its bases).
+  void run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, uint64_t max_keys,
+                bool recover, uint64_t* counts, unsigned long long* total, uint32_t segments,
+                cudaStream_t s, double prune_ratio = 0.0);
+  // Buckets of the ordered rounds and the window probe's slices of the rows
+  // (kernels/window_probe.cuh).
+  void plan_windows();
   // Device tables of a segmented launch for `segments` requests.
   void ensure_segment_capacity(Workspace& ws, uint32_t segments);
   // Randstrobemer seeds of a planned batch (strobes.cuh): candidates, then
@@ -307,6 +312,10 @@ class Engine {
   DevIndex* d_ix_rec_ = nullptr;    // with recovery
   DevIndex* d_ix_norec_ = nullptr;  // recovery disabled
   ColorLoc* d_color_loc_ = nullptr;  // colour -> class, member, group (wide probe)
+  OrderKey order_;
+  WinSlice* d_win_slices_ = nullptr;  // none: no window probe for this index
+  uint32_t win_slices_ = 0, win_weights_ = 0;
+  uint64_t win_min_keys_ = ~0ull;
   std::vector<void*> allocations_;
   uint64_t resident_bytes_ = 0;
   std::unique_ptr<Workspace> ws_;

@@ -27,6 +27,14 @@ struct SeedParams {
   uint32_t strobe_min, strobe_max;
 };
 
+// Buckets of a key sort: hash partition, then the top fbits of the first hash.
+struct OrderKey {
+  uint64_t seed = 0;
+  uint32_t parts = 1;  // largest partition count of a class (a power of two)
+  int fbits = 16;      // bits of the first hash
+  __host__ __device__ uint32_t buckets() const { return parts << fbits; }
+};
+
 struct Tile {
   uint32_t record;  // record index in the batch
   uint32_t w0;      // first window start (record coordinates)

@@ -37,11 +37,11 @@ namespace zx {
 constexpr int kWideSeeds = 256;      // seeds per descriptor round of a block
 constexpr int kWidePlanes = 6;       // register planes: counts up to 63 per field
 constexpr uint32_t kWideFlush = 63;  // seeds between plane flushes
-// Ordered rounds: a counting sort of a round's dense key list by the top
-// kOrderBits bits of each key's first hash (every class's row index grows
-// with the first hash). Keys keep no particular order within a bucket.
-constexpr int kOrderBits = 16;
-constexpr uint32_t kOrderBuckets = 1u << kOrderBits;
+// Ordered rounds: a counting sort of a round's dense key list by hash
+// partition and the top bits of each key's first hash (every class's row
+// index grows with the first hash within a partition). Keys keep no
+// particular order within a bucket.
+constexpr int kMaxOrderBits = 18;  // buckets: 1 MiB of counters
 
 // Colour location for recovered-origin point probes: cls_member = class |
 // member index << 8 (member index within a multi-member group, 0 for
@@ -99,6 +99,9 @@ struct WideRound {
   // min_ratio (> 0 turns on threshold pruning); tile_hi ends the round.
   double min_ratio = 0.0;
   uint32_t tile_hi = 0;
+  // Unsegmented: a round of this many keys or more is left to the window
+  // probe (window_probe.cuh).
+  uint64_t max_keys = ~0ull;
 };
 
 // Smallest count c with c / total >= ratio in IEEE double division: the
@@ -187,51 +190,87 @@ __global__ void extract_dense_kernel(BatchView bv, SeedParams sp, uint64_t* __re
   }
 }
 
-__device__ __forceinline__ uint32_t order_bucket(uint64_t key, uint64_t seed) {
-  return (uint32_t)(mixsplit(key, seed) >> (64 - kOrderBits));
+// Partition part of a key's bucket: a class of P partitions holds the key in
+// partition order_partition(...) % P.
+__device__ __forceinline__ uint32_t order_partition(uint64_t key, const OrderKey& o) {
+  return o.parts > 1 ? partition_id(key, o.seed, o.parts) : 0u;
+}
+
+__device__ __forceinline__ uint32_t order_bucket(uint64_t key, const OrderKey& o) {
+  return (order_partition(key, o) << o.fbits) |
+         (uint32_t)(mixsplit(key, o.seed) >> (64 - o.fbits));
 }
 
 // Ordered rounds, step 1: keys per bucket (hist zeroed before).
 __global__ void order_count_kernel(const uint64_t* __restrict__ keys,
-                                   const unsigned long long* __restrict__ nkeys, uint64_t seed,
+                                   const unsigned long long* __restrict__ nkeys, OrderKey o,
                                    uint32_t* __restrict__ hist) {
   const uint64_t n = *nkeys;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x)
-    atomicAdd(hist + order_bucket(keys[i], seed), 1u);
+    atomicAdd(hist + order_bucket(keys[i], o), 1u);
 }
 
 // Step 2 (one block of 1,024 threads): the buckets' first places, in place.
-__global__ void order_scan_kernel(uint32_t* __restrict__ hist) {
-  __shared__ uint32_t part[1024];
-  const uint32_t T = blockDim.x, tid = threadIdx.x, per = kOrderBuckets / T;
-  uint32_t sum = 0;
-  for (uint32_t j = 0; j < per; ++j) sum += hist[tid * per + j];
-  part[tid] = sum;
-  __syncthreads();
-  for (uint32_t off = 1; off < T; off <<= 1) {
-    const uint32_t v = tid >= off ? part[tid - off] : 0u;
+// The table goes through in stretches of 16,384 buckets, 16 consecutive ones
+// per thread in four 16-byte loads: a thread-strided walk of the same table
+// waited on one load at a time (107 us for 65,536 buckets on a B200).
+__global__ void __launch_bounds__(1024) order_scan_kernel(uint32_t* __restrict__ hist,
+                                                          uint32_t buckets) {
+  __shared__ uint32_t part[32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t run = 0;
+  for (uint32_t b0 = 0; b0 < buckets; b0 += 16384) {
+    const uint32_t at = b0 + tid * 16;
+    uint4 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      v[q] = at + q * 4 < buckets ? *reinterpret_cast<const uint4*>(hist + at + q * 4)
+                                  : make_uint4(0, 0, 0, 0);
+    uint32_t sum = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sum += v[q].x + v[q].y + v[q].z + v[q].w;
+    uint32_t incl = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+      if (lane >= d) incl += u;
+    }
+    if (lane == 31) part[warp] = incl;
     __syncthreads();
-    part[tid] += v;
+    uint32_t before = 0, all = 0;
+    for (uint32_t i = 0; i < 32; ++i) {
+      const uint32_t p = part[i];
+      if (i < warp) before += p;
+      all += p;
+    }
     __syncthreads();
-  }
-  uint32_t run = tid ? part[tid - 1] : 0u;
-  for (uint32_t j = 0; j < per; ++j) {
-    const uint32_t c = hist[tid * per + j];
-    hist[tid * per + j] = run;
-    run += c;
+    uint32_t first = run + before + incl - sum;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (at + q * 4 >= buckets) break;
+      uint4 f;
+      f.x = first;
+      f.y = f.x + v[q].x;
+      f.z = f.y + v[q].y;
+      f.w = f.z + v[q].z;
+      first = f.w + v[q].w;
+      *reinterpret_cast<uint4*>(hist + at + q * 4) = f;
+    }
+    run += all;
   }
 }
 
-// Step 3: every key to its bucket's next place in out[].
+// Step 3: every key to its bucket's next place in out[]; next[b] ends as the
+// end of bucket b.
 __global__ void order_scatter_kernel(const uint64_t* __restrict__ keys,
-                                     const unsigned long long* __restrict__ nkeys, uint64_t seed,
+                                     const unsigned long long* __restrict__ nkeys, OrderKey o,
                                      uint32_t* __restrict__ next, uint64_t* __restrict__ out) {
   const uint64_t n = *nkeys;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t k = keys[i];
-    out[atomicAdd(next + order_bucket(k, seed), 1u)] = k;
+    out[atomicAdd(next + order_bucket(k, o), 1u)] = k;
   }
 }
 
@@ -258,6 +297,40 @@ struct WideCounters {
   }
 };
 
+// Adds the recovered origins of a key that its filters do not hit (an origin
+// counts once per seed whether or not a filter hits it too): the origin's own
+// field is read again in the key's H cells, and its membership bit for a
+// multi-member group. row_of(ci, r) is the row index of cell r in class ci.
+template <class RowOf>
+__device__ __forceinline__ void count_recovered(const DevIndex& ix, const RecHit& rec,
+                                                const ColorLoc* __restrict__ color_loc, uint32_t fp,
+                                                const WideCounters& cnt, RowOf&& row_of) {
+  const int H = ix.hashes, b = ix.bits;
+  for (uint32_t o = 0; o < rec.len; ++o) {
+    const uint32_t c = rec.at(o);
+    const ColorLoc loc = color_loc[c];
+    bool hit = false;
+    if (loc.cls_member != 0xFFFFFFFFu) {
+      const uint32_t ci = loc.cls_member & 0xFFu, mi = loc.cls_member >> 8, g = loc.group;
+      const DevClass& C = ix.cls[ci];
+      uint64_t fx = 0;
+      for (int r = 0; r < H; ++r)
+        fx ^= row_bits(C.data + (uint64_t)row_of(ci, r) * C.row_stride, g * (uint32_t)b, (uint32_t)b);
+      hit = (uint32_t)fx == fp;
+      const uint32_t gc = __ldg(C.group_color + g);
+      if (hit && (gc & kMultiGroup)) {
+        const uint32_t* mg = C.multi + 3 * (gc & ~kMultiGroup);
+        const uint32_t off = __ldg(mg), w = __ldg(mg + 1);
+        uint64_t mx = 0;
+        for (int r = 0; r < H; ++r)
+          mx ^= row_bits(C.data + (uint64_t)row_of(ci, r) * C.row_stride, off, w);
+        hit = (mx >> mi) & 1u;
+      }
+    }
+    if (!hit) cnt.add(c, 1);
+  }
+}
+
 // Group of dense bit p of a chunk (chunk-local group 0 = first field): word
 // p % b of the chunk, field p / b of that word.
 __device__ __forceinline__ uint32_t wide_group(uint32_t g0, uint32_t p, int b, int lb) {
@@ -273,9 +346,9 @@ __global__ void __launch_bounds__(MAXT, MINB)
     wide_probe_kernel(const DevIndex* __restrict__ gix, const ColorLoc* __restrict__ color_loc,
                       const uint64_t* __restrict__ keys,
                       const unsigned long long* __restrict__ nkeys, int smem_counters,
-                      uint32_t team_threads, uint32_t* __restrict__ partial,
-                      uint64_t* __restrict__ counts, unsigned long long* __restrict__ total,
-                      WideRound sg) {
+                      uint32_t team_threads, uint64_t* __restrict__ counts,
+                      unsigned long long* __restrict__ total, WideRound sg) {
+  if (!sg.nseg && *nkeys >= sg.max_keys) return;
   extern __shared__ __align__(16) uint8_t smem[];
   DevIndex* six = reinterpret_cast<DevIndex*>(smem);
   uint8_t* p = smem + FusedSmem::ix_bytes;
@@ -295,7 +368,6 @@ __global__ void __launch_bounds__(MAXT, MINB)
   WideCounters cnt{scount, counts};
   const int H = ix.hashes, Hp = (H + 3) & ~3, b = ix.bits, lb = log2_bits(b);
   const uint32_t ones = field_ones(b), hi = ones << (b - 1);
-  const uint32_t fmask = b == 32 ? 0xFFFFFFFFu : (1u << b) - 1u;
   const uint32_t per_seed = classes * (uint32_t)Hp;
   const uint32_t T = blockDim.x, tid = threadIdx.x;
   // Teams of TT threads (the whole block for wide rows; fewer threads for
@@ -488,29 +560,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
           my[ci * Hp + r] = row0 + (uint32_t)r * seg + (((uint32_t)h ^ (uint32_t)(h >> 33)) & (seg - 1));
       }
       const RecHit rec = recovery_lookup(ix.rec, recovery_hash(key, ix.seed));
-      for (uint32_t o = 0; o < rec.len; ++o) {
-        const uint32_t c = rec.at(o);
-        const ColorLoc loc = color_loc[c];
-        bool hit = false;
-        if (loc.cls_member != 0xFFFFFFFFu) {
-          const uint32_t ci = loc.cls_member & 0xFFu, mi = loc.cls_member >> 8, g = loc.group;
-          const DevClass& C = ix.cls[ci];
-          const uint32_t* rr = my + ci * Hp;
-          uint64_t fx = 0;
-          for (int r = 0; r < H; ++r)
-            fx ^= row_bits(C.data + (uint64_t)rr[r] * C.row_stride, g * (uint32_t)b, (uint32_t)b);
-          hit = (uint32_t)fx == (fp & fmask);
-          const uint32_t gc = __ldg(C.group_color + g);
-          if (hit && (gc & kMultiGroup)) {
-            const uint32_t* mg = C.multi + 3 * (gc & ~kMultiGroup);
-            const uint32_t off = __ldg(mg), w = __ldg(mg + 1);
-            uint64_t mx = 0;
-            for (int r = 0; r < H; ++r) mx ^= row_bits(C.data + (uint64_t)rr[r] * C.row_stride, off, w);
-            hit = (mx >> mi) & 1u;
-          }
-        }
-        if (!hit) cnt.add(c, 1);
-      }
+      count_recovered(ix, rec, color_loc, fp, cnt,
+                      [&](uint32_t ci, int r) { return my[ci * Hp + r]; });
     }
     if (tid == 0 && !sg.nseg) seeds += n;
     __syncthreads();
@@ -609,7 +660,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
   __syncthreads();
   if (scount)
     for (uint32_t c = threadIdx.x; c < colors; c += blockDim.x)
-      partial[(uint64_t)blockIdx.x * colors + c] = scount[c];
+      if (scount[c])
+        atomicAdd(reinterpret_cast<unsigned long long*>(counts + c), (unsigned long long)scount[c]);
 }
 
 }  // namespace zx
