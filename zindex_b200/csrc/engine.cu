@@ -149,7 +149,8 @@ using WideFn = void (*)(const DevIndex*, const ColorLoc*, const uint64_t*,
                        const unsigned long long*, int, uint32_t, uint64_t*,
                        unsigned long long*, WideRound);
 using WindowFn = void (*)(const DevIndex*, WinPlan, const uint64_t*, const unsigned long long*,
-                         const uint32_t*, uint64_t*, unsigned long long*);
+                         const uint32_t*, unsigned long long*, uint64_t*,
+                         unsigned long long*);
 using DenseExtractFn = void (*)(BatchView, SeedParams, uint64_t*, unsigned long long*, int,
                                 WideRound);
 
@@ -912,8 +913,9 @@ void Engine::plan_windows() {
 
   // Slices of every class: the widest power of two (up to 16 chunks, a lane
   // each) whose window of H segments and one bucket fits the block's shared
-  // memory, the remainder cut where the sum of (width + 2) per slice is
-  // least (2: a slice's own hashing of a seed, in chunks).
+  // memory, the remainder cut where the sum of (width + 4) per slice is
+  // least (4: a slice's own hashing of a seed, in chunks; on a B200 a seed
+  // costs 18, 11, 8 and 6 cycles of a block in slices of 16, 8, 4 and 1).
   const int H = m_.hashes;
   const uint32_t tile = WinSmem::tile_bytes(H);
   std::vector<WinSlice> slices;
@@ -931,8 +933,8 @@ void Engine::plan_windows() {
       cost[left] = ~0u;
       for (int lw = 0; lw <= top; ++lw) {
         const uint32_t w = 1u << lw, rest = left > w ? cost[left - w] : 0;
-        if (w + 2 + rest < cost[left]) {
-          cost[left] = w + 2 + rest;
+        if (w + 4 + rest < cost[left]) {
+          cost[left] = w + 4 + rest;
           width[left] = (uint32_t)lw;
         }
       }
@@ -940,8 +942,8 @@ void Engine::plan_windows() {
     for (uint32_t k = 0; k < C.fp_chunks;) {
       const uint32_t lw = width[C.fp_chunks - k], w = 1u << lw;
       const uint32_t n = std::min(w, C.fp_chunks - k);
-      slices.push_back(WinSlice{c, k, n, lw, w + 2, weights});
-      weights += w + 2;
+      slices.push_back(WinSlice{c, k, n, lw, w + 4, weights});
+      weights += w + 4;
       k += n;
     }
     row_chunks += C.fp_chunks;
@@ -1516,8 +1518,8 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
     if (segments)
       cuda_check(cudaMemsetAsync(sg.cursor, 0, segments * 8ull, xs), "memset");
     else
-      cuda_check(cudaMemsetAsync(ws.wide_cursor + b, 0, 8, xs), "memset");
-    efn<<<egrid, ewarps * 32, esmem, xs>>>(rb, sp_, keys, ws.wide_cursor + b, ewarps, sg);
+      cuda_check(cudaMemsetAsync(ws.wide_cursor + 2 * b, 0, 16, xs), "memset");
+    efn<<<egrid, ewarps * 32, esmem, xs>>>(rb, sp_, keys, ws.wide_cursor + 2 * b, ewarps, sg);
     cuda_check(cudaGetLastError(), "extract_dense_kernel");
     const uint64_t* probe_keys = keys;
     if (ordered) {
@@ -1526,11 +1528,11 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
       // read on the device.
       const int ogrid = sms_ * 8;
       cuda_check(cudaMemsetAsync(ws.wide_hist[b], 0, order_.buckets() * 4ull, xs), "memset");
-      order_count_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + b, order_, ws.wide_hist[b]);
+      order_count_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + 2 * b, order_, ws.wide_hist[b]);
       cuda_check(cudaGetLastError(), "order_count_kernel");
       order_scan_kernel<<<1, 1024, 0, xs>>>(ws.wide_hist[b], order_.buckets());
       cuda_check(cudaGetLastError(), "order_scan_kernel");
-      order_scatter_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + b, order_,
+      order_scatter_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + 2 * b, order_,
                                                   ws.wide_hist[b], ws.wide_keys_alt[b]);
       cuda_check(cudaGetLastError(), "order_scatter_kernel");
       probe_keys = ws.wide_keys_alt[b];
@@ -1545,7 +1547,7 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
       cuda_check(cudaStreamWaitEvent(s, ws.wide_ext[b], 0), "cudaStreamWaitEvent");
     }
     const DevIndex* dix = recover ? d_ix_rec_ : d_ix_norec_;
-    wfn<<<wblocks, l.warps * 32, smem, s>>>(dix, d_color_loc_, probe_keys, ws.wide_cursor + b,
+    wfn<<<wblocks, l.warps * 32, smem, s>>>(dix, d_color_loc_, probe_keys, ws.wide_cursor + 2 * b,
                                             l.smem_counters, wteam, counts,
                                             segments ? nullptr : total, sg);
     cuda_check(cudaGetLastError(), "wide_probe_kernel");
@@ -1556,11 +1558,12 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
                  "cudaFuncSetAttribute");
       const WinPlan plan{d_win_slices_, win_slices_, win_weights_, order_, win_min_keys_};
       const int wgrid = l.blocks > 0 ? std::min(l.blocks, 2 * sms_) : 2 * sms_;
-      winfn<<<wgrid, kWinThreads, kWinBlockBytes, s>>>(dix, plan, probe_keys, ws.wide_cursor + b,
-                                                       ws.wide_hist[b], counts, total);
+      winfn<<<wgrid, kWinThreads, kWinBlockBytes, s>>>(dix, plan, probe_keys, ws.wide_cursor + 2 * b,
+                                                       ws.wide_hist[b], ws.wide_cursor + 2 * b + 1,
+                                                       counts, total);
       cuda_check(cudaGetLastError(), "window_probe_kernel");
       if (recover && host_ix_.rec.bits) {
-        recover_kernel<<<sms_ * 8, 256, 0, s>>>(dix, d_color_loc_, probe_keys, ws.wide_cursor + b,
+        recover_kernel<<<sms_ * 8, 256, 0, s>>>(dix, d_color_loc_, probe_keys, ws.wide_cursor + 2 * b,
                                                 win_min_keys_, counts);
         cuda_check(cudaGetLastError(), "recover_kernel");
       }
@@ -1658,7 +1661,7 @@ void Engine::ensure_split_capacity(Workspace& ws) {
   if (ws.split_keys) return;
   dev_alloc(&ws.split_keys, kSplitTiles * kTileWindows, "split key slots");
   dev_alloc(&ws.split_counts, kSplitTiles, "split key counts");
-  dev_alloc(&ws.wide_cursor, 2, "dense key cursors");
+  dev_alloc(&ws.wide_cursor, 4, "dense key cursors");
   ws.release_graphs();
 }
 

@@ -70,7 +70,9 @@ struct Workspace {
   // Split minimizer queries: key slots of one round of tiles.
   uint64_t* split_keys = nullptr;
   uint32_t* split_counts = nullptr;
-  unsigned long long* wide_cursor = nullptr;  // wide-row queries: keys in the dense lists (2)
+  // Wide-row queries, per key list (2): its keys, then the window probe's
+  // next work item.
+  unsigned long long* wide_cursor = nullptr;
   // Segmented wide-row queries, per key list: keys of each segment and the
   // first probe round of each segment (2 x cap_segments each).
   unsigned long long* wide_seg_cursor = nullptr;
