@@ -12,6 +12,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
+#include "kernels/key_order.cuh"
 #include "kernels/query_kernels.cuh"
 #include "kernels/record_hits.cuh"
 #include "kernels/strobes.cuh"
@@ -488,7 +489,8 @@ Workspace::~Workspace() {
                  rec_counts, rec_totals, rec_hits, rec_first, rec_scan_tmp, hit_colors,
                  hit_counts, split_keys, split_counts, wide_cursor, wide_keys2,
                  wide_seg_cursor, wide_round_first, wide_keys_alt[0], wide_keys_alt[1],
-                 wide_hist[0], wide_hist[1], strobe_anchors, strobe_hashes, strobe_slots,
+                 wide_hist[0], wide_hist[1], wide_next[0], wide_next[1], round_keys[0],
+                 round_keys[1], strobe_anchors, strobe_hashes, strobe_slots,
                  strobe_count};
   for (void* p : dev)
     if (p) cudaFree(p);
@@ -881,13 +883,25 @@ void Engine::load(const std::string& dir, const OpenOptions& options) {
     cuda_check(cudaMemcpy(d_origins, rr.origins.data(), rr.origins.size() * 4,
                           cudaMemcpyHostToDevice),
                "upload");
-    host_ix_.rec = DevRecovery{d_dir, d_ranges, d_origins, bits};
+    uint32_t* d_filter = nullptr;
+    if (n <= 1ull << kRecFilterBits) {
+      std::vector<uint32_t> filter((1ull << kRecFilterBits) / 32, 0);
+      for (uint32_t h : rr.hashes) {
+        const uint32_t at = h & ((1u << kRecFilterBits) - 1);
+        filter[at >> 5] |= 1u << (at & 31);
+      }
+      dev_alloc(&d_filter, filter.size(), "recovery filter");
+      allocations_.push_back(d_filter);
+      cuda_check(cudaMemcpy(d_filter, filter.data(), filter.size() * 4, cudaMemcpyHostToDevice),
+                 "upload");
+    }
+    host_ix_.rec = DevRecovery{d_dir, d_ranges, d_origins, bits, d_filter};
   }
   dev_alloc(&d_ix_rec_, 1, "index table");
   dev_alloc(&d_ix_norec_, 1, "index table");
   cuda_check(cudaMemcpy(d_ix_rec_, &host_ix_, sizeof(DevIndex), cudaMemcpyHostToDevice), "upload");
   DevIndex norec = host_ix_;
-  norec.rec = DevRecovery{nullptr, nullptr, nullptr, 0};
+  norec.rec = DevRecovery{nullptr, nullptr, nullptr, 0, nullptr};
   cuda_check(cudaMemcpy(d_ix_norec_, &norec, sizeof(DevIndex), cudaMemcpyHostToDevice), "upload");
   plan_windows();
   launch_ = default_launch();
@@ -896,37 +910,55 @@ void Engine::load(const std::string& dir, const OpenOptions& options) {
 }
 
 void Engine::plan_windows() {
-  // Buckets of the ordered rounds: about two per segment of the largest
-  // class, 2^14 (so that the sort's counters are not contended) to 2^18.
-  uint64_t most = 1;
+  const int H = m_.hashes;
+  uint64_t most = 1;  // bases of the largest class
   order_.seed = m_.seed;
   for (uint32_t c = 0; c < host_ix_.classes; ++c) {
     const DevClass& C = host_ix_.cls[c];
-    most = std::max<uint64_t>(most, C.slots / C.seg - (uint64_t)m_.hashes + 1);
+    most = std::max<uint64_t>(most, C.slots / C.seg - (uint64_t)H + 1);
     order_.parts = std::max(order_.parts, C.partitions);
   }
   int pbits = 0;
   while ((1u << pbits) < order_.parts) ++pbits;
-  order_.fbits = 14;
+  // The widest slice (log2 of chunks, at most 16: a lane each) whose window
+  // of H segments and one bucket fits a block's shared memory; negative:
+  // none.
+  const uint32_t tile = WinSmem::tile_bytes(H);
+  auto widest = [&](const DevClass& C, int fbits) {
+    const uint64_t count = C.slots / C.seg - (uint64_t)H + 1;
+    const uint64_t span = (count + (1ull << fbits) - 1) >> fbits;
+    int top = 4;
+    while (top >= 0 && tile / ((C.seg << top) * 16) < (uint64_t)H + span) --top;
+    return top;
+  };
+  // Buckets of the ordered rounds: about two per segment of the largest
+  // class, at least 2^10 and at most 2^18 over the partitions; 2^13, which a
+  // block sorts in shared memory, where that leaves every class slices of
+  // eight chunks or what finer buckets would leave it (half the slice width
+  // costs the probe about a tenth, the sort through global counters more
+  // than half of the probe).
+  order_.fbits = 10;
   while (order_.fbits + pbits < kMaxOrderBits && (1ull << order_.fbits) < 2 * most) ++order_.fbits;
+  if (order_.fbits + pbits > kBlockOrderBits && pbits < kBlockOrderBits) {
+    const int coarse = kBlockOrderBits - pbits;
+    bool keep = true;
+    for (uint32_t c = 0; c < host_ix_.classes; ++c)
+      keep &= widest(host_ix_.cls[c], coarse) >= std::min(3, widest(host_ix_.cls[c], order_.fbits));
+    if (keep) order_.fbits = coarse;
+  }
+  block_order_ = order_.fbits + pbits <= kBlockOrderBits;
   if (order_.fbits + pbits > kMaxOrderBits || !wide_eligible(8)) return;
 
-  // Slices of every class: the widest power of two (up to 16 chunks, a lane
-  // each) whose window of H segments and one bucket fits the block's shared
-  // memory, the remainder cut where the sum of (width + 4) per slice is
-  // least (4: a slice's own hashing of a seed, in chunks; on a B200 a seed
-  // costs 18, 11, 8 and 6 cycles of a block in slices of 16, 8, 4 and 1).
-  const int H = m_.hashes;
-  const uint32_t tile = WinSmem::tile_bytes(H);
+  // Slices of every class: as wide as fits, the remainder cut where the sum
+  // of (width + 4) per slice is least (4: a slice's own hashing of a seed, in
+  // chunks; on a B200 a seed costs 18, 11, 8 and 6 cycles of a block in slices
+  // of 16, 8, 4 and 1).
   std::vector<WinSlice> slices;
   uint32_t weights = 0;
   uint64_t row_chunks = 0, chunk_rows = 0;  // chunks of a seed's row, of all rows
   for (uint32_t c = 0; c < host_ix_.classes; ++c) {
     const DevClass& C = host_ix_.cls[c];
-    const uint64_t count = C.slots / C.seg - (uint64_t)H + 1;
-    const uint64_t span = (count + (1ull << order_.fbits) - 1) >> order_.fbits;
-    int top = 4;
-    while (top >= 0 && tile / ((C.seg << top) * 16) < (uint64_t)H + span) --top;
+    const int top = widest(C, order_.fbits);
     if (top < 0) return;  // segments too long for a window: the wide probe runs every round
     std::vector<uint32_t> cost(C.fp_chunks + 1, 0), width(C.fp_chunks + 1, 0);
     for (uint32_t left = 1; left <= C.fp_chunks; ++left) {
@@ -1192,15 +1224,20 @@ std::unique_ptr<Workspace> Engine::make_workspace() {
   return ws;
 }
 
-void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, bool segmented) {
+void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, bool segmented,
+                             uint64_t round_bases) {
   const uint64_t colors = m_.colors.size();
   // Split minimizer and wide-row queries: key slots allocated before any graph capture.
-  if (kernel_mode(launch_) == 4 || wide_form(launch_)) ensure_split_capacity(ws);
-  const bool rounds = nbases / kTileWindows + records + nbases / kFindereTask + 1 > kSplitTiles;
-  if (wide_form(launch_) && rounds) ensure_wide_pipeline(ws);
-  if (wide_form(launch_) && launch_.order && !segmented) {
-    ensure_order_capacity(ws, 0);
-    if (rounds) ensure_order_capacity(ws, 1);
+  const bool wide = wide_form(launch_);
+  const bool whole = wide && !segmented && ensure_round_capacity(ws, std::min(nbases, round_bases));
+  if (kernel_mode(launch_) == 4 || (wide && !whole)) ensure_split_capacity(ws);
+  const bool rounds =
+      !whole && nbases / kTileWindows + records + nbases / kFindereTask + 1 > kSplitTiles;
+  if (wide) ensure_cursors(ws);
+  if (wide && rounds) ensure_wide_pipeline(ws);
+  if (wide && launch_.order && !segmented) {
+    ensure_order_capacity(ws, 0, whole);
+    if (rounds) ensure_order_capacity(ws, 1, whole);
   }
   if (nbases > ws.cap_bases || !ws.bases) {
     uint64_t cap = std::max<uint64_t>({nbases, ws.cap_bases * 3 / 2, 4096});
@@ -1461,7 +1498,6 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
   // counters are added up (segmented: each block adds its counters to the
   // segment it leaves).
   const QueryLaunch& l = launch_;
-  ensure_split_capacity(ws);
   const size_t smem = fused_smem_bytes(l);
   const int blocks_cap = max_blocks(l);
   int J, HQ;
@@ -1480,7 +1516,12 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
   // A tile holds at most 256 seeds: one probe round.
   const int wblocks = l.blocks > 0 ? std::min(l.blocks, blocks_cap)
                                    : (int)std::min<uint64_t>(blocks_cap, std::max<uint64_t>(tiles_bound, 1));
-  const uint64_t rounds = (tiles_bound + kSplitTiles - 1) / kSplitTiles;
+  // One round when its key lists hold every base of the batch; else rounds of
+  // kSplitTiles tiles.
+  const bool whole = !segments && ensure_round_capacity(ws, max_keys);
+  const uint64_t round_tiles = whole ? std::max<uint64_t>(tiles_bound, 1) : kSplitTiles;
+  const uint64_t rounds = (tiles_bound + round_tiles - 1) / round_tiles;
+  if (!whole) ensure_split_capacity(ws);
   // Several rounds: extraction (compute-bound) of round r + 1 runs on the
   // auxiliary stream beside the probe (memory-bound) of round r, the rounds
   // alternating between two key lists; events order each list's reuse.
@@ -1493,10 +1534,10 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
   }
   for (uint64_t r = 0; r < rounds; ++r) {
     const int b = overlap ? (int)(r & 1) : 0;
-    uint64_t* keys = b ? ws.wide_keys2 : ws.split_keys;
+    uint64_t* keys = whole ? ws.round_keys[0] : (b ? ws.wide_keys2 : ws.split_keys);
     BatchView rb = bv;
-    rb.tile_lo = (uint32_t)(r * kSplitTiles);
-    rb.tile_hi = (uint32_t)std::min<uint64_t>((r + 1) * kSplitTiles, tiles_bound);
+    rb.tile_lo = (uint32_t)(r * round_tiles);
+    rb.tile_hi = (uint32_t)std::min<uint64_t>((r + 1) * round_tiles, tiles_bound);
     WideRound sg;
     if (segments) {
       sg.seg_tiles = ws.seg_tiles;
@@ -1508,10 +1549,16 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
       sg.tile_hi = rb.tile_hi;
       sg.min_ratio = prune_ratio;
     }
-    const bool ordered = l.order && !segments;
-    if (ordered) ensure_order_capacity(ws, b);
+    if (whole) {
+      sg.key_cap = ws.cap_round_keys;
+      sg.err = ws.error;
+    }
+    // (Seeds far fewer than the rows share none worth bringing together.)
+    const bool ordered =
+        !segments && (l.order == 2 || (l.order == 1 && (!win_slices_ || max_keys >= win_min_keys_ / 8)));
+    if (ordered) ensure_order_capacity(ws, b, whole);
     sg.interleave = !segments && l.order == 2 ? 1u : 0u;
-    const bool windows = l.order == 1 && !segments && win_slices_ && max_keys >= win_min_keys_;
+    const bool windows = ordered && l.order == 1 && win_slices_ && max_keys >= win_min_keys_;
     if (windows) sg.max_keys = win_min_keys_;
     if (overlap && r >= 2)
       cuda_check(cudaStreamWaitEvent(xs, ws.wide_probe[b], 0), "cudaStreamWaitEvent");
@@ -1522,20 +1569,65 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
     efn<<<egrid, ewarps * 32, esmem, xs>>>(rb, sp_, keys, ws.wide_cursor + 2 * b, ewarps, sg);
     cuda_check(cudaGetLastError(), "extract_dense_kernel");
     const uint64_t* probe_keys = keys;
+    const uint32_t* bucket_end = ws.wide_hist[b];  // end of each bucket in the sorted list
+    const DevIndex* dix = recover ? d_ix_rec_ : d_ix_norec_;
     if (ordered) {
       // Counting sort of the round's keys by partition and their first
       // hash's top bits (row-address order of every class), the key count
       // read on the device.
-      const int ogrid = sms_ * 8;
+      uint64_t* sorted = whole ? ws.round_keys[1] : ws.wide_keys_alt[b];
       cuda_check(cudaMemsetAsync(ws.wide_hist[b], 0, order_.buckets() * 4ull, xs), "memset");
-      order_count_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + 2 * b, order_, ws.wide_hist[b]);
-      cuda_check(cudaGetLastError(), "order_count_kernel");
-      order_scan_kernel<<<1, 1024, 0, xs>>>(ws.wide_hist[b], order_.buckets());
-      cuda_check(cudaGetLastError(), "order_scan_kernel");
-      order_scatter_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + 2 * b, order_,
-                                                  ws.wide_hist[b], ws.wide_keys_alt[b]);
-      cuda_check(cudaGetLastError(), "order_scatter_kernel");
-      probe_keys = ws.wide_keys_alt[b];
+      if (block_order_) {
+        const uint32_t buckets = order_.buckets();
+        const int ogrid = sms_ * 2;
+        unsigned long long* n = ws.wide_cursor + 2 * b;
+        const bool look = windows && recover && host_ix_.rec.bits;
+        const size_t csmem = 
+            buckets * 4ull + (look ? kRecQueueBytes : 0) + (look && host_ix_.rec.filter ? kRecFilterBytes : 0);
+        cuda_check(cudaFuncSetAttribute(block_count_kernel,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem),
+                   "cudaFuncSetAttribute");
+        block_count_kernel<<<ogrid, kOrderThreads, csmem, xs>>>(
+            dix, d_color_loc_, keys, n, order_, look ? win_min_keys_ : ~0ull, ws.wide_hist[b],
+            counts);
+        cuda_check(cudaGetLastError(), "block_count_kernel");
+        order_scan_kernel<<<1, 1024, 0, xs>>>(ws.wide_hist[b], buckets);
+        cuda_check(cudaGetLastError(), "order_scan_kernel");
+        cuda_check(cudaFuncSetAttribute(tile_scatter_kernel,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)sizeof(TileSmem)),
+                   "cudaFuncSetAttribute");
+        // By the upper half of the bucket bits into the other list, then by
+        // all of them back into this one.
+        int half = 0;
+        while ((1u << (2 * half)) < buckets) ++half;
+        const uint64_t* from = keys;
+        uint64_t* to = sorted;
+        for (int shift : {half, 0}) {
+          const uint32_t bins = buckets >> shift;
+          order_bins_kernel<<<(bins + 255) / 256, 256, 0, xs>>>(ws.wide_hist[b], bins, shift,
+                                                                ws.wide_next[b]);
+          cuda_check(cudaGetLastError(), "order_bins_kernel");
+          tile_scatter_kernel<<<ogrid, kTileThreads, sizeof(TileSmem), xs>>>(
+              from, n, order_, shift, ws.wide_next[b], to);
+          cuda_check(cudaGetLastError(), "tile_scatter_kernel");
+          from = sorted;
+          to = keys;
+        }
+        sorted = keys;
+        bucket_end = ws.wide_hist[b] + 1;
+      } else {
+        const int ogrid = sms_ * 8;
+        order_count_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + 2 * b, order_,
+                                                  ws.wide_hist[b]);
+        cuda_check(cudaGetLastError(), "order_count_kernel");
+        order_scan_kernel<<<1, 1024, 0, xs>>>(ws.wide_hist[b], order_.buckets());
+        cuda_check(cudaGetLastError(), "order_scan_kernel");
+        order_scatter_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + 2 * b, order_,
+                                                    ws.wide_hist[b], sorted);
+        cuda_check(cudaGetLastError(), "order_scatter_kernel");
+      }
+      probe_keys = sorted;
     }
     if (segments) {
       wide_rounds_kernel<<<1, 1024, 0, xs>>>(sg.cursor, segments,
@@ -1546,7 +1638,6 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
       cuda_check(cudaEventRecord(ws.wide_ext[b], xs), "cudaEventRecord");
       cuda_check(cudaStreamWaitEvent(s, ws.wide_ext[b], 0), "cudaStreamWaitEvent");
     }
-    const DevIndex* dix = recover ? d_ix_rec_ : d_ix_norec_;
     wfn<<<wblocks, l.warps * 32, smem, s>>>(dix, d_color_loc_, probe_keys, ws.wide_cursor + 2 * b,
                                             l.smem_counters, wteam, counts,
                                             segments ? nullptr : total, sg);
@@ -1559,10 +1650,10 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
       const WinPlan plan{d_win_slices_, win_slices_, win_weights_, order_, win_min_keys_};
       const int wgrid = l.blocks > 0 ? std::min(l.blocks, 2 * sms_) : 2 * sms_;
       winfn<<<wgrid, kWinThreads, kWinBlockBytes, s>>>(dix, plan, probe_keys, ws.wide_cursor + 2 * b,
-                                                       ws.wide_hist[b], ws.wide_cursor + 2 * b + 1,
+                                                       bucket_end, ws.wide_cursor + 2 * b + 1,
                                                        counts, total);
       cuda_check(cudaGetLastError(), "window_probe_kernel");
-      if (recover && host_ix_.rec.bits) {
+      if (!block_order_ && recover && host_ix_.rec.bits) {
         recover_kernel<<<sms_ * 8, 256, 0, s>>>(dix, d_color_loc_, probe_keys, ws.wide_cursor + 2 * b,
                                                 win_min_keys_, counts);
         cuda_check(cudaGetLastError(), "recover_kernel");
@@ -1572,11 +1663,44 @@ void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, 
   }
 }
 
-void Engine::ensure_order_capacity(Workspace& ws, int b) {
-  if (ws.wide_keys_alt[b]) return;
-  dev_alloc(&ws.wide_keys_alt[b], (uint64_t)kSplitTiles * kTileWindows, "round keys in order");
-  dev_alloc(&ws.wide_hist[b], order_.buckets(), "round order buckets");
+void Engine::ensure_order_capacity(Workspace& ws, int b, bool whole) {
+  if (!ws.wide_hist[b]) {
+    dev_alloc(&ws.wide_hist[b], order_.buckets() + 4ull, "round order buckets");
+    if (block_order_)
+      dev_alloc(&ws.wide_next[b], order_.buckets(), "round order places");
+    ws.release_graphs();
+  }
+  if (!whole && !ws.wide_keys_alt[b]) {
+    dev_alloc(&ws.wide_keys_alt[b], (uint64_t)kSplitTiles * kTileWindows, "round keys in order");
+    ws.release_graphs();
+  }
+}
+
+bool Engine::ensure_round_capacity(Workspace& ws, uint64_t keys) {
+  if (keys > kRoundKeys) return false;
+  const int lists = launch_.order ? 2 : 1;
+  bool have = true;
+  for (int i = 0; i < lists; ++i) have &= ws.round_keys[i] && ws.cap_round_keys >= keys;
+  if (have) return true;
+  // No memory for it: the smaller lists of kSplitTiles tiles a round.
+  const uint64_t cap = std::max<uint64_t>(keys + std::min<uint64_t>(keys / 4, 1ull << 24), 1ull << 20);
   ws.release_graphs();
+  ws.cap_round_keys = 0;
+  for (int i = 0; i < 2; ++i) {
+    if (ws.round_keys[i]) cudaFree(ws.round_keys[i]);
+    ws.round_keys[i] = nullptr;
+  }
+  for (int i = 0; i < lists; ++i)
+    if (cudaMalloc((void**)&ws.round_keys[i], cap * 8) != cudaSuccess) {
+      cudaGetLastError();
+      for (int j = 0; j < 2; ++j) {
+        if (ws.round_keys[j]) cudaFree(ws.round_keys[j]);
+        ws.round_keys[j] = nullptr;
+      }
+      return false;
+    }
+  ws.cap_round_keys = cap;
+  return true;
 }
 
 void Engine::ensure_strobe_capacity(Workspace& ws, uint64_t nbases, uint64_t tiles) {
@@ -1661,6 +1785,11 @@ void Engine::ensure_split_capacity(Workspace& ws) {
   if (ws.split_keys) return;
   dev_alloc(&ws.split_keys, kSplitTiles * kTileWindows, "split key slots");
   dev_alloc(&ws.split_counts, kSplitTiles, "split key counts");
+  ws.release_graphs();
+}
+
+void Engine::ensure_cursors(Workspace& ws) {
+  if (ws.wide_cursor) return;
   dev_alloc(&ws.wide_cursor, 4, "dense key cursors");
   ws.release_graphs();
 }
@@ -2137,7 +2266,10 @@ void Engine::query_host(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   for (uint64_t c = 0; c < chunks; ++c)
     check(offsets[bounds[c]] <= offsets[bounds[c + 1]] && offsets[bounds[c + 1]] <= nbases, kEInval,
           "offsets must be non-decreasing");
-  ensure_capacity(ws, nbases, records + chunks);
+  uint64_t most = 0;  // bases of the largest chunk
+  for (uint64_t c = 0; c < chunks; ++c)
+    most = std::max(most, offsets[bounds[c + 1]] - offsets[bounds[c]]);
+  ensure_capacity(ws, nbases, records + chunks, false, most);
   ensure_host_capacity(ws, nbases, records + chunks);
   const uint64_t colors = m_.colors.size();
   cudaStream_t s = ws.stream;

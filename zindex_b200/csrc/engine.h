@@ -77,10 +77,14 @@ struct Workspace {
   // first probe round of each segment (2 x cap_segments each).
   unsigned long long* wide_seg_cursor = nullptr;
   uint32_t* wide_round_first = nullptr;
-  // Ordered wide-row rounds, per key list: the keys in bucket order and the
-  // buckets' counts / next places.
+  // Ordered wide-row rounds, per key list: the keys in bucket order, the
+  // buckets' counts / places and, sorted by blocks, a pass's next places.
   uint64_t* wide_keys_alt[2] = {};
   uint32_t* wide_hist[2] = {};
+  uint32_t* wide_next[2] = {};
+  // Wide-row queries of one round: the whole batch's keys, and in order.
+  uint64_t* round_keys[2] = {};
+  uint64_t cap_round_keys = 0;
   // Randstrobemer queries: candidate bits and strobe hashes per base, each
   // tile's linked seeds (kStrobeSlot per tile) and their numbers.
   uint32_t* strobe_anchors = nullptr;
@@ -255,7 +259,9 @@ class Engine {
   void release();  // frees every device allocation and event of the engine
   // Device buffers of a query of nbases / records (segmented queries do not
   // sort their rounds: no ordered-round buffers).
-  void ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, bool segmented = false);
+  // round_bases: most bases queried at once (a host query's largest chunk).
+  void ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, bool segmented = false,
+                       uint64_t round_bases = ~0ull);
   // Homopolymer compression on the device (lib.rs:211-222 per ACGT run):
   // replaces (bases, offsets) by the compressed batch in the workspace.
   void compress_homopolymers(Workspace& ws, const uint8_t*& bases, uint64_t nbases,
@@ -274,8 +280,13 @@ class Engine {
   // Wide-row queries of several rounds: the second key list, the auxiliary
   // stream and the events of the extraction / probe pipeline.
   void ensure_wide_pipeline(Workspace& ws);
-  // Ordered wide-row rounds: sort buffers of key list b (0 or 1).
-  void ensure_order_capacity(Workspace& ws, int b);
+  // Ordered wide-row rounds: sort buffers of key list b (0 or 1); whole: the
+  // sorted keys go to the round lists.
+  void ensure_order_capacity(Workspace& ws, int b, bool whole);
+  // Key lists of a batch in one round (up to kRoundKeys keys); false: too many
+  // keys or no memory, and the batch runs in rounds of kSplitTiles tiles.
+  bool ensure_round_capacity(Workspace& ws, uint64_t keys);
+  void ensure_cursors(Workspace& ws);
   // Wide-row form over the planned tiles of a packed batch: rounds of up to
   // kSplitTiles tiles, each a dense extraction and a wide probe. segments = 0:
   // one query into counts / *total; segments > 0: a segmented query, request
@@ -315,6 +326,7 @@ class Engine {
   DevIndex* d_ix_norec_ = nullptr;  // recovery disabled
   ColorLoc* d_color_loc_ = nullptr;  // colour -> class, member, group (wide probe)
   OrderKey order_;
+  bool block_order_ = false;  // buckets fit a block's shared memory (kernels/key_order.cuh)
   WinSlice* d_win_slices_ = nullptr;  // none: no window probe for this index
   uint32_t win_slices_ = 0, win_weights_ = 0;
   uint64_t win_min_keys_ = ~0ull;

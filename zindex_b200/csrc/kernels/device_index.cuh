@@ -39,7 +39,11 @@ struct DevRecovery {
   const uint2* ranges;       // {start, length} postings
   const uint32_t* origins;   // posting storage
   uint32_t bits;             // log2(capacity); 0 when the map is empty
+  // Bit h % 2^kRecFilterBits set for every hash h of the map: a small map's
+  // lookups that end here need no random read. Null for a larger map.
+  const uint32_t* filter;
 };
+constexpr int kRecFilterBits = 20;  // 128 KiB, of use up to about as many hashes
 
 struct __align__(16) DevIndex {
   DevClass cls[kMaxClasses];

@@ -20,34 +20,67 @@ namespace zx {
 // Byte -> 2-bit code, 4 for anything that is not A/C/G/T.
 __device__ __forceinline__ uint32_t dev_code(uint8_t b) { return encode_base(b); }
 
+// Four bases of a word (first in the low byte) -> their 2-bit codes as one
+// byte, first base on top, and a bit per base that is not A/C/G/T. Of the
+// upper-case letters bits 1 and 2, XORed with bits 2 and 3, are the code; a
+// letter is valid when it is the one its code stands for.
+__device__ __forceinline__ uint32_t pack4(uint32_t x, uint32_t& inv) {
+  const uint32_t u = x & 0xDFDFDFDFu;
+  const uint32_t c = ((u >> 1) ^ (u >> 2)) & 0x03030303u;
+  const uint32_t pair = (c | (c >> 4)) & 0x00330033u;
+  const uint32_t bad = u ^ __byte_perm(0x54474341u, 0, pair | (pair >> 8));
+  // Bit 7 of every byte of `bad` that is not zero, gathered in four bits.
+  const uint32_t nz = (((bad & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | bad) & 0x80808080u;
+  inv = ((nz >> 7) * 0x10204080u) >> 28;
+  return (c * 0x40100401u) >> 24;
+}
+
 // K0: ASCII bases -> packed 2-bit words + invalid masks. Word w covers bases
-// 32w..32w+31; positions past `n` are marked invalid.
+// 32w..32w+31; positions past `n` are marked invalid. Bound by its reads and
+// writes (1.375 bytes a base); a byte-by-byte decode took 171 us for 150 MB on
+// a B200.
 __device__ __forceinline__ void pack_word(const uint8_t* __restrict__ bases, uint64_t n,
                                           uint64_t* __restrict__ packed,
                                           uint32_t* __restrict__ invalid, uint64_t w) {
-  {
-    uint64_t base = w * 32, v = 0;
-    uint32_t inv = 0;
-    if (base + 32 <= n && (((uintptr_t)(bases + base)) & 15) == 0) {
-      uint4 a = *reinterpret_cast<const uint4*>(bases + base);
-      uint4 b = *reinterpret_cast<const uint4*>(bases + base + 16);
-      uint32_t x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        uint32_t c = dev_code((uint8_t)(x[i >> 2] >> (8 * (i & 3))));
-        inv |= (uint32_t)(c > 3) << i;
-        v |= (uint64_t)(c & 3) << (62 - 2 * i);
-      }
+  const uint64_t base = w * 32;
+  uint64_t v = 0;
+  uint32_t inv = 0;
+  if (base + 32 <= n) {
+    const uint8_t* p = bases + base;
+    uint32_t x[8];
+    if (((uintptr_t)p & 15) == 0) {
+      const uint4 a = *reinterpret_cast<const uint4*>(p);
+      const uint4 b = *reinterpret_cast<const uint4*>(p + 16);
+      x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+      x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
     } else {
-      for (int i = 0; i < 32; ++i) {
-        uint32_t c = base + i < n ? dev_code(bases[base + i]) : 4;
-        inv |= (uint32_t)(c > 3) << i;
-        v |= (uint64_t)(c & 3) << (62 - 2 * i);
+      // Any alignment: the aligned words that hold the 32 bytes, shifted.
+      const uint32_t* q = reinterpret_cast<const uint32_t*>((uintptr_t)p & ~(uintptr_t)3);
+      const uint32_t shift = 8u * ((uint32_t)(uintptr_t)p & 3u);
+      uint32_t lo = q[0];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t hi = i < 7 || shift ? q[i + 1] : 0u;
+        x[i] = __funnelshift_r(lo, hi, shift);
+        lo = hi;
       }
     }
-    packed[w] = v;
-    invalid[w] = inv;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      uint32_t bad;
+      const uint32_t codes = pack4(x[i], bad);
+      v |= (uint64_t)codes << (56 - 8 * i);
+      inv |= bad << (4 * i);
+    }
+  } else {
+    for (int i = 0; i < 32; ++i) {
+      const uint32_t c = base + i < n ? dev_code(bases[base + i]) : 4;
+      inv |= (uint32_t)(c > 3) << i;
+      v |= (uint64_t)(c & 3) << (62 - 2 * i);
+    }
   }
+  packed[w] = v;
+  invalid[w] = inv;
 }
 
 __global__ void pack_kernel(const uint8_t* __restrict__ bases, uint64_t n,
@@ -129,6 +162,41 @@ __device__ __forceinline__ uint32_t warp_append(uint64_t* buf, uint32_t count, b
   return count + __popc(ballot);
 }
 
+// 32 consecutive windows of at most 32 bases, one per lane, from the two or
+// three words that the whole warp shares.
+//
+// Whether lane l's window p0 + l .. p0 + l + k - 1 is all A/C/G/T, for the
+// first n lanes (p0 + n + k - 2 is a base of the batch).
+__device__ __forceinline__ bool short_valid(const PackedView& pv, uint64_t p0, uint32_t n, int k,
+                                            int lane) {
+  const uint64_t q = p0 >> 5;
+  const uint32_t off = (uint32_t)(p0 & 31), end = off + n + (uint32_t)k - 2;  // last base
+  const uint32_t i0 = __ldg(pv.invalid + q), i1 = end >= 32 ? __ldg(pv.invalid + q + 1) : 0u;
+  const uint32_t i2 = end >= 64 ? __ldg(pv.invalid + q + 2) : 0u;
+  const uint32_t r = off + (uint32_t)lane;
+  const uint32_t inv = r < 32 ? __funnelshift_r(i0, i1, r) : __funnelshift_r(i1, i2, r - 32);
+  return (uint32_t)lane < n && (inv & (k == 32 ? ~0u : (1u << k) - 1u)) == 0;
+}
+
+// Canonical value of lane l's window (meaningful where it is valid).
+__device__ __forceinline__ uint64_t short_canonical(const PackedView& pv, uint64_t p0, uint32_t n,
+                                                    int k, int lane) {
+  const uint64_t q = p0 >> 5;
+  const uint32_t off = (uint32_t)(p0 & 31), end = off + n + (uint32_t)k - 2;
+  const uint64_t w0 = __ldg(pv.packed + q), w1 = end >= 32 ? __ldg(pv.packed + q + 1) : 0ull;
+  const uint64_t w2 = end >= 64 ? __ldg(pv.packed + q + 2) : 0ull;
+  const uint32_t r = off + (uint32_t)lane;
+  const uint64_t hi = r < 32 ? w0 : w1, lo = r < 32 ? w1 : w2;
+  const bool half = r & 16;  // 2r bits: one 32-bit word and 2 (r & 15) bits
+  const uint32_t x0 = half ? (uint32_t)hi : (uint32_t)(hi >> 32);
+  const uint32_t x1 = half ? (uint32_t)(lo >> 32) : (uint32_t)hi;
+  const uint32_t x2 = half ? (uint32_t)lo : (uint32_t)(lo >> 32);
+  const uint32_t sh = 2 * (r & 15);
+  const uint64_t v = ((uint64_t)__funnelshift_l(x1, x0, sh) << 32) | __funnelshift_l(x2, x1, sh);
+  const uint64_t f = k == 32 ? v : v >> (64 - 2 * k), c = revcomp(f, k);
+  return f < c ? f : c;
+}
+
 // Canonical k-mers (k <= 32) of windows [w0, w0+nw) of the record starting at
 // global base `rb`: one window per lane per round, in window order.
 __device__ __forceinline__ uint32_t tile_kmers_short(const PackedView& pv, uint64_t rb, uint32_t w0,
@@ -137,16 +205,11 @@ __device__ __forceinline__ uint32_t tile_kmers_short(const PackedView& pv, uint6
                                                      uint64_t* buf, int lane) {
   uint32_t count = 0;
   for (uint32_t i0 = 0; i0 < nw; i0 += 32) {
-    uint32_t i = i0 + lane;
-    bool keep = false;
-    uint64_t key = 0;
-    if (i < nw) {
-      uint64_t p = rb + w0 + i;
-      if (pv.valid(p, k)) {
-        key = canonical_at(pv, p, k);
-        keep = !modimizer || mixsplit(key, seed) % sampling == 0;
-      }
-    }
+    const uint64_t p0 = rb + w0 + i0;
+    const uint32_t n = min(32u, nw - i0);
+    bool keep = short_valid(pv, p0, n, k, lane);
+    const uint64_t key = short_canonical(pv, p0, n, k, lane);
+    if (modimizer) keep = keep && mixsplit(key, seed) % sampling == 0;
     count = warp_append(buf, count, keep, key, lane);
   }
   return count;

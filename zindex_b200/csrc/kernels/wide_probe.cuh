@@ -102,6 +102,10 @@ struct WideRound {
   // Unsegmented: a round of this many keys or more is left to the window
   // probe (window_probe.cuh).
   uint64_t max_keys = ~0ull;
+  // Keys that the unsegmented list holds; more (records that overlap because
+  // offsets decrease) are dropped and reported.
+  uint64_t key_cap = ~0ull;
+  uint32_t* err = nullptr;
 };
 
 // Smallest count c with c / total >= ratio in IEEE double division: the
@@ -151,6 +155,73 @@ __global__ void wide_rounds_kernel(const unsigned long long* __restrict__ cursor
   if (tid == T - 1) round_first[nseg] = part[T - 1];
 }
 
+// extract_dense_kernel for canonical k-mers of k <= 32: a warp takes several
+// tiles at a time, counts their valid windows, reserves their places with one
+// atomic (one per tile kept the cursor's cache line busy: 1.1 ms for 1e6 tiles
+// on a B200) and writes the keys straight from registers.
+__device__ __forceinline__ void extract_short(const BatchView& bv, const SeedParams& sp,
+                                              uint64_t* __restrict__ out,
+                                              unsigned long long* __restrict__ cursor,
+                                              uint32_t warp, uint32_t warps, int lane,
+                                              const WideRound& sg) {
+  constexpr uint32_t kFull = 0xFFFFFFFFu;
+  uint32_t ntiles = *bv.ntiles;
+  if (bv.tile_hi && bv.tile_hi < ntiles) ntiles = bv.tile_hi;
+  if (ntiles <= bv.tile_lo) return;
+  const uint32_t group =
+      sg.nseg ? 1u : min(8u, max(1u, (ntiles - bv.tile_lo) / (2u * warps)));  // tiles at a time
+  const uint64_t step = (uint64_t)warps * group;
+  for (uint64_t t0 = bv.tile_lo + (uint64_t)warp * group; t0 < ntiles; t0 += step) {
+    const uint32_t m = ntiles - t0 < group ? (uint32_t)(ntiles - t0) : group;
+    // Lane j holds tile j: its first base and windows.
+    uint64_t first = 0;
+    uint32_t nw = 0;
+    if ((uint32_t)lane < m) {
+      const Tile t = bv.tiles[t0 + lane];
+      first = bv.offsets[t.record] + t.w0;
+      nw = t.nw;
+    }
+    uint32_t total = 0;
+    for (uint32_t j = 0; j < m; ++j) {
+      const uint64_t p = __shfl_sync(kFull, first, j);
+      const uint32_t w = __shfl_sync(kFull, nw, j);
+      for (uint32_t i0 = 0; i0 < w; i0 += 32)
+        total += __popc(__ballot_sync(kFull, short_valid(bv.pv, p + i0, min(32u, w - i0), sp.klen, lane)));
+    }
+    uint64_t* dst = out;
+    unsigned long long* cur = cursor;
+    if (sg.nseg) {
+      const uint32_t seg = segment_of(sg.seg_tiles, sg.nseg, (uint32_t)t0);
+      dst = out + wide_seg_base(sg, seg);
+      cur = sg.cursor + seg;
+    }
+    unsigned long long at = 0;
+    if (lane == 0 && total) at = atomicAdd(cur, (unsigned long long)total);
+    at = __shfl_sync(kFull, at, 0);
+    if (at + total > sg.key_cap) {
+      if (lane == 0) {
+        atomicAdd(cur, 0ull - total);
+        atomicOr(sg.err, kErrOffsets);
+      }
+      continue;
+    }
+    dst += at;
+    for (uint32_t j = 0; j < m; ++j) {
+      const uint64_t p = __shfl_sync(kFull, first, j);
+      const uint32_t w = __shfl_sync(kFull, nw, j);
+      for (uint32_t i0 = 0; i0 < w; i0 += 32) {
+        const uint32_t n = min(32u, w - i0);
+        const bool keep = short_valid(bv.pv, p + i0, n, sp.klen, lane);
+        uint64_t key = short_canonical(bv.pv, p + i0, n, sp.klen, lane);
+        if (sp.spaced) key = spaced_canonical(sp.pattern, key);
+        const uint32_t ballot = __ballot_sync(kFull, keep);
+        if (keep) dst[__popc(ballot & ((1u << lane) - 1u))] = key;
+        dst += __popc(ballot);
+      }
+    }
+  }
+}
+
 // Appends the seeds of tiles [tile_lo, tile_hi) (tile_hi 0 = to the end) to
 // out[], one atomic cursor bump per warp and tile. out holds at least
 // (tile_hi - tile_lo) * kTileWindows keys. Segmented (sg.nseg > 0): each
@@ -163,6 +234,11 @@ __global__ void extract_dense_kernel(BatchView bv, SeedParams sp, uint64_t* __re
   uint64_t* inner = reinterpret_cast<uint64_t*>(smem);
   uint8_t* p = smem + 256 * 8;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (MODE == 0 && sp.klen <= 32) {
+    extract_short(bv, sp, out, cursor, blockIdx.x * warps_per_block + warp,
+                  gridDim.x * warps_per_block, lane, sg);
+    return;
+  }
   uint8_t* wbase = p + (size_t)warp * DenseSmem::warp_bytes(MODE, sp.k);
   uint64_t* keys = reinterpret_cast<uint64_t*>(wbase);
   uint8_t* ocm = wbase + FusedSmem::key_bytes(MODE, sp.k, false);
@@ -173,7 +249,7 @@ __global__ void extract_dense_kernel(BatchView bv, SeedParams sp, uint64_t* __re
   const uint32_t warps_total = gridDim.x * warps_per_block;
   for (uint32_t t = bv.tile_lo + blockIdx.x * warps_per_block + warp; t < ntiles;
        t += warps_total) {
-    const uint32_t n = extract_tile<MODE>(bv, sp, bv.tiles[t], keys, ocm, inner, lane);
+    uint32_t n = extract_tile<MODE>(bv, sp, bv.tiles[t], keys, ocm, inner, lane);
     __syncwarp();
     unsigned long long at = 0;
     uint64_t* dst = out;
@@ -185,6 +261,13 @@ __global__ void extract_dense_kernel(BatchView bv, SeedParams sp, uint64_t* __re
     }
     if (lane == 0 && n) at = atomicAdd(cur, (unsigned long long)n);
     at = __shfl_sync(0xFFFFFFFFu, at, 0);
+    if (at + n > sg.key_cap) {
+      if (lane == 0) {
+        atomicAdd(cur, 0ull - n);
+        atomicOr(sg.err, kErrOffsets);
+      }
+      n = 0;
+    }
     for (uint32_t i = lane; i < n; i += 32) dst[at + i] = keys[i];
     __syncwarp();
   }
@@ -211,7 +294,8 @@ __global__ void order_count_kernel(const uint64_t* __restrict__ keys,
     atomicAdd(hist + order_bucket(keys[i], o), 1u);
 }
 
-// Step 2 (one block of 1,024 threads): the buckets' first places, in place.
+// Step 2 (one block of 1,024 threads): the buckets' first places, in place,
+// and the number of keys in hist[buckets].
 // The table goes through in stretches of 16,384 buckets, 16 consecutive ones
 // per thread in four 16-byte loads: a thread-strided walk of the same table
 // waited on one load at a time (107 us for 65,536 buckets on a B200).
@@ -259,6 +343,7 @@ __global__ void __launch_bounds__(1024) order_scan_kernel(uint32_t* __restrict__
     }
     run += all;
   }
+  if (tid == 0) hist[buckets] = run;
 }
 
 // Step 3: every key to its bucket's next place in out[]; next[b] ends as the
@@ -329,6 +414,22 @@ __device__ __forceinline__ void count_recovered(const DevIndex& ix, const RecHit
     }
     if (!hit) cnt.add(c, 1);
   }
+}
+
+// The recovered origins of a key that its filters miss.
+__device__ __forceinline__ void recover_key(const DevIndex& ix, const ColorLoc* __restrict__ color_loc,
+                                            uint64_t key, const WideCounters& cnt) {
+  const RecHit rec = recovery_lookup(ix.rec, recovery_hash(key, ix.seed));
+  if (!rec.len) return;
+  const uint64_t first = mixsplit(key, ix.seed), step = splitmix64(first);
+  count_recovered(ix, rec, color_loc, (uint32_t)fingerprint(key, ix.seed, ix.bits), cnt,
+                  [&](uint32_t ci, int r) {
+                    const DevClass& C = ix.cls[ci];
+                    const uint64_t part = C.partitions > 1 ? partition_id(key, ix.seed, C.partitions) : 0;
+                    const uint64_t base = mulhi64(first, C.slots / C.seg - (uint64_t)ix.hashes + 1);
+                    const uint64_t h = first + (uint64_t)r * step;
+                    return part * C.slots + (base + (uint64_t)r) * C.seg + ((h ^ (h >> 33)) & (C.seg - 1));
+                  });
 }
 
 // Group of dense bit p of a chunk (chunk-local group 0 = first field): word

@@ -25,7 +25,8 @@
 //   time. The match flags are counted in eight bit planes per lane (a
 //   carry-save adder takes four seeds in 6 logic operations plus the carry)
 //   and reach the block's counters every 255 seeds.
-// * Recovered origins are counted by recover_kernel, once per seed.
+// * Recovered origins are counted once per seed, when the keys are sorted
+//   (block_count_kernel) or by recover_kernel.
 #pragma once
 #include <stdint.h>
 
@@ -352,10 +353,8 @@ __global__ void __launch_bounds__(kWinThreads, 2)
   }
 }
 
-// Recovered origins of a round probed by the window probe: each origin that
-// the filter did not hit, once per seed (count_recovered). A seed's directory
-// entry is an independent random read; the rows are read again only for the
-// few seeds with origins.
+// Recovered origins of a round probed by the window probe and sorted through
+// global counters (block_count_kernel does it for the others).
 __global__ void __launch_bounds__(256)
     recover_kernel(const DevIndex* __restrict__ gix, const ColorLoc* __restrict__ color_loc,
                    const uint64_t* __restrict__ keys, const unsigned long long* __restrict__ nkeys,
@@ -364,20 +363,8 @@ __global__ void __launch_bounds__(256)
   if (n < min_keys) return;
   const WideCounters cnt{nullptr, counts};
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t key = keys[i];
-    const RecHit rec = recovery_lookup(gix->rec, recovery_hash(key, gix->seed));
-    if (!rec.len) continue;
-    const uint64_t first = mixsplit(key, gix->seed), step = splitmix64(first);
-    count_recovered(*gix, rec, color_loc, (uint32_t)fingerprint(key, gix->seed, gix->bits), cnt,
-                    [&](uint32_t ci, int r) {
-                      const DevClass& C = gix->cls[ci];
-                      const uint64_t part = C.partitions > 1 ? partition_id(key, gix->seed, C.partitions) : 0;
-                      const uint64_t base = mulhi64(first, C.slots / C.seg - (uint64_t)gix->hashes + 1);
-                      const uint64_t h = first + (uint64_t)r * step;
-                      return part * C.slots + (base + (uint64_t)r) * C.seg + ((h ^ (h >> 33)) & (C.seg - 1));
-                    });
-  }
+       i += (uint64_t)gridDim.x * blockDim.x)
+    recover_key(*gix, color_loc, keys[i], cnt);
 }
 
 }  // namespace zx
