@@ -112,7 +112,7 @@ __global__ void extract_region_kernel(BatchView bv, SeedParams sp,
                                       unsigned long long* __restrict__ cursor,
                                       uint64_t* __restrict__ out, int warps_per_block) {
   extern __shared__ __align__(16) uint8_t smem[];
-  uint64_t* inner = reinterpret_cast<uint64_t*>(smem);
+  uint16_t* inner = reinterpret_cast<uint16_t*>(smem);
   uint8_t* p = smem + 256 * 8;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint8_t* wbase = p + (size_t)warp * FusedSmem::warp_bytes(MODE, sp.k, 0, 0, 0, 4, 0, 0, false);
@@ -410,7 +410,7 @@ class DeviceBuilder {
     sp_.m = fp.m;
     sp_.klen = fp.k;
     sp_.seed = fp.seed;
-    sp_.sampling = fp.sampling;
+    sp_.set_sampling(fp.sampling);
     sp_.ocm = fp.mode == 1 && fp.k != fp.m ? ocm_params(fp.k, fp.m) : OcmParams{1, fp.m, 1};
     if (sp_.klen > 32) sp_.lk = long_kmer_consts(sp_.klen);
     sp_.spaced = fp.spaced ? 1 : 0;

@@ -630,7 +630,7 @@ void Engine::load(const std::string& dir, const OpenOptions& options) {
   sp_.m = (int)m_.minimizer_size;
   sp_.klen = m_.index_mode == kFindere ? (int)(m_.k - m_.findere_z) : (int)m_.k;
   sp_.seed = m_.seed;
-  sp_.sampling = m_.modimizer_sampling;
+  sp_.set_sampling(m_.modimizer_sampling);
   if (m_.index_mode == kMinimizers && m_.k != m_.minimizer_size)
     sp_.ocm = ocm_params((int)m_.k, (int)m_.minimizer_size);
   else

@@ -219,12 +219,13 @@ struct FusedSmem {
 template <int MODE>
 __device__ __forceinline__ uint32_t extract_tile(const BatchView& bv, const SeedParams& sp,
                                                  const Tile& t, uint64_t* keys, uint8_t* ocm,
-                                                 const uint64_t* inner, int lane) {
+                                                 const uint16_t* inner, int lane,
+                                                 const uint64_t* quads = nullptr) {
   const uint64_t rb = bv.offsets[t.record];
   uint32_t n;
   if (MODE == 1) {
     if (sp.k == sp.m) {
-      n = tile_ocm_full(bv.pv, rb, t.w0, t.nw, sp.m, keys, lane);
+      n = tile_ocm_full(bv.pv, sp, rb, t.w0, t.nw, keys, lane);
     } else {
       Rank16* pre = reinterpret_cast<Rank16*>(ocm);
       Rank16* suf = pre + FusedSmem::ocm_entries(sp.k);
@@ -232,11 +233,10 @@ __device__ __forceinline__ uint32_t extract_tile(const BatchView& bv, const Seed
       n = tile_ocm(bv.pv, rb, t.w0, t.nw, sp, inner, pre, suf, pos, keys, lane);
     }
   } else if (sp.klen <= 32) {
-    n = tile_kmers_short(bv.pv, rb, t.w0, t.nw, sp.klen, MODE == 2, sp.seed, sp.sampling, keys,
-                         lane);
+    n = tile_kmers_short(bv.pv, sp, rb, t.w0, t.nw, sp.klen, MODE == 2, keys, lane);
   } else {
-    n = tile_kmers_long(bv.pv, rb, t.w0, t.nw, sp.klen, sp.lk, MODE == 2, sp.seed, sp.sampling,
-                        keys, keys + kTileWindows, lane);
+    n = tile_kmers_long(bv.pv, sp, rb, t.w0, t.nw, sp.klen, MODE == 2, keys, keys + kTileWindows,
+                        quads, lane);
   }
   // Spaced seeds (anchors.rs:265-281; k-mer and minimizer indexes, patterns of
   // width k or m <= 31): the plain canonical keys, selected first, are mapped
@@ -254,11 +254,32 @@ __device__ __forceinline__ void load_index_smem(const DevIndex* __restrict__ gix
   for (uint32_t i = threadIdx.x; i < sizeof(DevIndex) / 16; i += blockDim.x) dst[i] = src[i];
 }
 
-__device__ __forceinline__ void build_inner_table(const SeedParams& sp, uint64_t* inner) {
+// Ranks of the s-mers' inner hashes (equal hashes share a rank; only their
+// order matters to open-closed minimizers), 2 bytes each, in a 256 x 8 byte
+// table that holds the hashes meanwhile. All threads of the block (at least a
+// warp) take part.
+__device__ __forceinline__ void build_inner_table(const SeedParams& sp, uint16_t* inner) {
   if (sp.mode != 1) return;
+  uint64_t* hash = reinterpret_cast<uint64_t*>(inner);
   const int s = sp.ocm.s;
-  for (uint32_t v = threadIdx.x; v < (1u << (2 * s)); v += blockDim.x)
-    inner[v] = mixsplit(canonical_encoded(v, s), sp.seed ^ kInnerHashSeed);
+  const uint32_t n = 1u << (2 * s);
+  for (uint32_t v = threadIdx.x; v < n; v += blockDim.x)
+    hash[v] = mixsplit(canonical_encoded(v, s), sp.seed ^ kInnerHashSeed);
+  __syncthreads();
+  uint32_t rank[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const uint32_t v = threadIdx.x + u * blockDim.x;
+    rank[u] = 0;
+    if (v < n)
+      for (uint32_t i = 0; i < n; ++i) rank[u] += hash[i] < hash[v];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const uint32_t v = threadIdx.x + u * blockDim.x;
+    if (v < n) inner[v] = (uint16_t)rank[u];
+  }
 }
 
 // Fused extraction + probe over the tile list (one instantiation per seed
@@ -282,9 +303,9 @@ __global__ void __launch_bounds__(256, MINB) fused_query_kernel(const DevIndex* 
     scount = reinterpret_cast<uint32_t*>(p);
     p += FusedSmem::counter_bytes(colors, 1);
   }
-  uint64_t* inner = nullptr;
+  uint16_t* inner = nullptr;
   if (MODE == 1) {
-    inner = reinterpret_cast<uint64_t*>(p);
+    inner = reinterpret_cast<uint16_t*>(p);
     p += 256 * 8;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -460,7 +481,7 @@ template <int MODE>
 __global__ void extract_kernel(BatchView bv, SeedParams sp, uint64_t* __restrict__ out,
                                uint32_t* __restrict__ out_count, int warps_per_block) {
   extern __shared__ __align__(16) uint8_t smem[];
-  uint64_t* inner = reinterpret_cast<uint64_t*>(smem);
+  uint16_t* inner = reinterpret_cast<uint16_t*>(smem);
   uint8_t* p = smem + 256 * 8;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint8_t* wbase = p + (size_t)warp * FusedSmem::warp_bytes(MODE, sp.k, 0, 0, 0, 4, 0, 0,

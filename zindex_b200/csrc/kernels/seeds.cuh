@@ -153,6 +153,27 @@ __device__ __forceinline__ uint64_t canonical_at(const PackedView& pv, uint64_t 
   return f < r ? f : r;
 }
 
+// Whether a modimizer index samples the key of this hash (hash % sampling == 0).
+__device__ __forceinline__ bool sampled(const SeedParams& sp, uint64_t hash) {
+  const uint64_t x = hash * sp.sampling_inverse;
+  const int r = sp.sampling_shift;
+  return ((x >> r) | (r ? x << (64 - r) : 0)) <= sp.sampling_most;
+}
+
+// Whether the len bases at p are all A/C/G/T (the warp together).
+__device__ __forceinline__ bool warp_valid(const PackedView& pv, uint64_t p, uint32_t len, int lane) {
+  const uint64_t q = p >> 5;
+  const uint32_t off = (uint32_t)(p & 31), end = off + len, words = (end + 31) >> 5;
+  bool bad = false;
+  for (uint32_t w = lane; w < words; w += 32) {
+    uint32_t m = __ldg(pv.invalid + q + w);
+    if (w == 0) m &= ~0u << off;
+    if (w + 1 == words && (end & 31)) m &= (1u << (end & 31)) - 1u;
+    bad |= m != 0;
+  }
+  return !__any_sync(0xFFFFFFFFu, bad);
+}
+
 // Appends the keys selected by `keep` (one per lane, order = lane order) to
 // the warp buffer; returns the new count (warp-uniform).
 __device__ __forceinline__ uint32_t warp_append(uint64_t* buf, uint32_t count, bool keep,
@@ -197,32 +218,79 @@ __device__ __forceinline__ uint64_t short_canonical(const PackedView& pv, uint64
   return f < c ? f : c;
 }
 
+// Canonical k-mers (k <= 32) of the nw <= 256 windows from global base p, whose
+// bases are all A/C/G/T, in window order: lane l takes the windows l * per ..
+// of per = ceil(nw / 32) and rolls them (a window's value from its
+// neighbour's costs a third of cutting it out of the packed words). Window i
+// goes to buf[i + pad * (i / per)]; pad 1 spreads the lanes' runs over the
+// banks.
+__device__ __forceinline__ void tile_kmers_run(const PackedView& pv, uint64_t p, uint32_t nw, int k,
+                                               uint64_t* buf, uint32_t pad, int lane) {
+  const uint32_t per = (nw + 31) / 32, a = (uint32_t)lane * per;
+  if (a >= nw) return;
+  const uint32_t n = min(per, nw - a);
+  uint64_t* out = buf + a + pad * (uint32_t)lane;
+  const uint64_t mask = k == 32 ? ~0ull : (1ull << (2 * k)) - 1;
+  uint64_t f = pv.fwd(p + a, k), r = revcomp(f, k);
+  // The bases after the first window (at most 7 are used).
+  uint64_t next = n > 1 ? pv.bits32(p + a + k) : 0;
+  out[0] = f < r ? f : r;
+  for (uint32_t j = 1; j < n; ++j) {
+    const uint64_t c = next >> 62;
+    next <<= 2;
+    f = ((f << 2) | c) & mask;
+    r = (r >> 2) | ((3 - c) << (2 * k - 2));
+    out[j] = f < r ? f : r;
+  }
+}
+
 // Canonical k-mers (k <= 32) of windows [w0, w0+nw) of the record starting at
-// global base `rb`: one window per lane per round, in window order.
-__device__ __forceinline__ uint32_t tile_kmers_short(const PackedView& pv, uint64_t rb, uint32_t w0,
-                                                     uint32_t nw, int k, bool modimizer,
-                                                     uint64_t seed, uint64_t sampling,
-                                                     uint64_t* buf, int lane) {
+// global base `rb`, in window order (modimizers: the sampled ones).
+__device__ __forceinline__ uint32_t tile_kmers_short(const PackedView& pv, const SeedParams& sp,
+                                                     uint64_t rb, uint32_t w0, uint32_t nw, int k,
+                                                     bool modimizer, uint64_t* buf, int lane) {
+  const uint64_t p = rb + w0;
+  if (!modimizer && nw && warp_valid(pv, p, nw + (uint32_t)k - 1, lane)) {
+    tile_kmers_run(pv, p, nw, k, buf, 0, lane);
+    return nw;
+  }
   uint32_t count = 0;
   for (uint32_t i0 = 0; i0 < nw; i0 += 32) {
-    const uint64_t p0 = rb + w0 + i0;
     const uint32_t n = min(32u, nw - i0);
-    bool keep = short_valid(pv, p0, n, k, lane);
-    const uint64_t key = short_canonical(pv, p0, n, k, lane);
-    if (modimizer) keep = keep && mixsplit(key, seed) % sampling == 0;
+    bool keep = short_valid(pv, p + i0, n, k, lane);
+    const uint64_t key = short_canonical(pv, p + i0, n, k, lane);
+    if (modimizer) keep = keep && sampled(sp, mixsplit(key, sp.seed));
     count = warp_append(buf, count, keep, key, lane);
   }
   return count;
 }
 
+// quads[x] and quads[256 + x]: the terms of four bases (first in the top bits
+// of x) in the forward and in the reverse polynomial of a long k-mer.
+__device__ __forceinline__ void build_long_table(uint64_t* quads) {
+  for (uint32_t x = threadIdx.x; x < 256; x += blockDim.x) {
+    uint64_t f = 0, r = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      f = f * kLongKmerBase + ((x >> (6 - 2 * j)) & 3) + 1;
+      r = r * kLongKmerBase + 4 - ((x >> (2 * j)) & 3);
+    }
+    quads[x] = f;
+    quads[256 + x] = r;
+  }
+}
+
 // Polynomial hashes (k > 32): each lane rolls over a contiguous run of
 // windows, restarting with a direct evaluation after invalid bases. Lane runs
-// are staged in `tmp` (nw entries) and concatenated in lane order.
-__device__ __forceinline__ uint32_t tile_kmers_long(const PackedView& pv, uint64_t rb, uint32_t w0,
-                                                    uint32_t nw, int k, const LongKmerConsts& lk,
-                                                    bool modimizer, uint64_t seed,
-                                                    uint64_t sampling, uint64_t* buf,
-                                                    uint64_t* tmp, int lane) {
+// are staged in `tmp` (nw entries) and concatenated in lane order. quads: the
+// table of build_long_table (the evaluation then takes four bases at a time:
+// base by base it was two thirds of a 49-mer's cost), or null.
+__device__ __forceinline__ uint32_t tile_kmers_long(const PackedView& pv, const SeedParams& sp,
+                                                    uint64_t rb, uint32_t w0, uint32_t nw, int k,
+                                                    bool modimizer, uint64_t* buf, uint64_t* tmp,
+                                                    const uint64_t* quads, int lane) {
+  const LongKmerConsts& lk = sp.lk;
+  const uint64_t base4 = kLongKmerBase * kLongKmerBase * kLongKmerBase * kLongKmerBase;
   const uint32_t per = (nw + 31) / 32;
   const uint32_t a = min(nw, per * lane), e = min(nw, a + per);
   uint32_t n = 0;
@@ -244,7 +312,19 @@ __device__ __forceinline__ uint32_t tile_kmers_long(const PackedView& pv, uint64
       f = 0;
       r = 0;
       uint64_t wgt = 1;
-      for (int q = 0; q < k; ++q) {
+      int q = 0;
+      if (quads) {
+        uint64_t v = 0;
+        for (; q + 4 <= k; q += 4) {
+          if ((q & 31) == 0) v = pv.bits32(p + q);
+          const uint32_t x = (uint32_t)(v >> 56);
+          v <<= 8;
+          f = f * base4 + quads[x];
+          r += quads[256 + x] * wgt;
+          wgt *= base4;
+        }
+      }
+      for (; q < k; ++q) {
         uint64_t c = pv.code(p + q);
         f = f * kLongKmerBase + (c + 1);
         r += (4 - c) * wgt;
@@ -252,7 +332,7 @@ __device__ __forceinline__ uint32_t tile_kmers_long(const PackedView& pv, uint64
       }
     }
     uint64_t key = splitmix64((f < r ? f : r) ^ lk.domain);
-    if (!modimizer || mixsplit(key, seed) % sampling == 0) tmp[a + n++] = key;
+    if (!modimizer || sampled(sp, mixsplit(key, sp.seed))) tmp[a + n++] = key;
   }
   uint32_t incl = n;
 #pragma unroll
@@ -350,9 +430,10 @@ constexpr uint32_t kOcmTile = 256;  // windows per minimizer tile
 // kOcmTile): pos[i] is window w0 - 1 + i's selected m-mer, as an index j
 // into the tile's anchors (record position w0 - 1 + j), or ~0 for an invalid
 // window. pre/suf hold at least nw + W entries each; inner is the
-// 4^s-entry inner hash table; pos holds nw + 1 entries.
-__device__ void tile_ocm_select(const PackedView& pv, uint64_t rb, uint32_t w0, uint32_t nw,
-                                const SeedParams& sp, const uint64_t* inner, Rank16* pre,
+// 4^s-entry table of inner hash ranks; pos holds nw + 1 entries. This form
+// takes windows of any span; tile_ocm_select_wide the usual ones.
+__device__ void tile_ocm_select_any(const PackedView& pv, uint64_t rb, uint32_t w0, uint32_t nw,
+                                const SeedParams& sp, const uint16_t* inner, Rank16* pre,
                                 Rank16* suf, uint32_t* pos, int lane) {
   const int k = sp.k, t = sp.ocm.t, s = sp.ocm.s, w = sp.ocm.w;
   const uint32_t W = (uint32_t)(k - t + 1);
@@ -367,9 +448,9 @@ __device__ void tile_ocm_select(const PackedView& pv, uint64_t rb, uint32_t w0, 
     if (w0 + j >= 1) {
       uint64_t p = rb + w0 + j - 1;
       uint64_t tf = pv.fwd(p, t);
-      uint64_t lo = ~0ull, h0 = 0, hm = 0, hl = 0;
+      uint32_t lo = ~0u, h0 = 0, hm = 0, hl = 0;
       for (int q = 0; q <= t - s; ++q) {
-        uint64_t h = inner[(tf >> (2 * (t - s - q))) & smask];
+        const uint32_t h = inner[(tf >> (2 * (t - s - q))) & smask];
         lo = h < lo ? h : lo;
         if (q == 0) h0 = h;
         if (q == (t - s) / 2) hm = h;
@@ -410,32 +491,193 @@ __device__ void tile_ocm_select(const PackedView& pv, uint64_t rb, uint32_t w0, 
   __syncwarp();
 }
 
+// Rank of an anchor or of a run of them in 12 bytes: class and the hash's top
+// 62 bits, then the hash's low 2 bits, and the leftmost and rightmost anchors
+// (15 bits each) of that rank.
+struct OcmRank {
+  uint64_t k;
+  uint32_t p;
+};
+
+// a lies left of b; equal ranks keep the leftmost and rightmost positions.
+__device__ __forceinline__ OcmRank ocm_min(const OcmRank& a, const OcmRank& b) {
+  OcmRank r;
+  const bool less = b.k < a.k || (b.k == a.k && (b.p >> 30) < (a.p >> 30));
+  r.k = less ? b.k : a.k;
+  r.p = less ? b.p : a.p;
+  if (a.k == b.k && (a.p >> 30) == (b.p >> 30)) r.p = (a.p & ~0x7FFFu) | (b.p & 0x7FFFu);
+  return r;
+}
+
+// Anchors of a lane in tile_ocm_select_wide.
+__device__ __forceinline__ uint32_t ocm_per_lane(uint32_t nw, uint32_t W) {
+  return (nw + W + 31) / 32;
+}
+
+// tile_ocm_select for windows of more than per = ocm_per_lane(nw, W) anchors:
+// lane l holds the anchors l * per .. and keeps their running minima from the
+// left (P) and from the right (S); a window's minimum is the S of its first
+// anchor, the minima of the whole lanes between (shuffled) and the P of its
+// last anchor. Each lane then selects for the windows that start at its
+// anchors, rolling their G and T counts. `scratch` holds 24 bytes for each of
+// 32 * (per | 1) anchors. (One lane per block of W anchors, as
+// tile_ocm_select_any has it, left most of the warp idle: 3.6 ms for 2^18 tiles
+// of 2,048-colour minimizer windows on a B200.)
+__device__ void tile_ocm_select_wide(const PackedView& pv, uint64_t rb, uint32_t w0, uint32_t nw,
+                                     const SeedParams& sp, const uint16_t* inner, uint8_t* scratch,
+                                     uint32_t* pos, int lane) {
+  constexpr uint32_t kFull = 0xFFFFFFFFu;
+  const int k = sp.k, t = sp.ocm.t, s = sp.ocm.s, w = sp.ocm.w;
+  const uint32_t W = (uint32_t)(k - t + 1), anchors = nw + W;
+  const uint32_t per = ocm_per_lane(nw, W), pitch = per | 1;  // odd: no bank conflicts
+  uint64_t* sk = reinterpret_cast<uint64_t*>(scratch);
+  uint64_t* pk = sk + 32 * pitch;
+  uint32_t* sp_ = reinterpret_cast<uint32_t*>(pk + 32 * pitch);
+  uint32_t* pp = sp_ + 32 * pitch;
+  const uint32_t a0 = (uint32_t)lane * per, at = (uint32_t)lane * pitch;
+  const uint32_t n = a0 < anchors ? min(per, anchors - a0) : 0;
+  // Position w0 - 1 of a record's first tile does not exist.
+  const uint32_t skip = w0 + a0 == 0 ? 1u : 0u;
+  const uint64_t p = rb + w0 + a0 - 1 + skip;  // first existing anchor of the lane
+  const uint32_t smask = (1u << (2 * s)) - 1;
+  const int last = t - s;
+  OcmRank run{~0ull, 0};
+  uint64_t v = 0;
+  int have = 0;  // bases left in v
+  for (uint32_t j = 0; j < n; ++j) {
+    OcmRank rk{~0ull, 3u << 30};  // no anchor: above every rank of a window
+    if (j >= skip) {
+      if (have < t) {
+        v = pv.bits32(p + (j - skip));
+        have = 32;
+      }
+      const uint64_t tf = v >> (64 - 2 * t);
+      v <<= 2;
+      --have;
+      uint32_t lo = ~0u, h0 = 0, hm = 0, hl = 0;
+      if (t <= 16) {
+        const uint32_t x = (uint32_t)tf;
+        for (int q = 0; q <= last; ++q) {
+          const uint32_t h = inner[(x >> (2 * (last - q))) & smask];
+          lo = min(lo, h);
+          if (q == 0) h0 = h;
+          if (q == last / 2) hm = h;
+          hl = h;
+        }
+      } else {
+        for (int q = 0; q <= last; ++q) {
+          const uint32_t h = inner[(uint32_t)(tf >> (2 * (last - q))) & smask];
+          lo = min(lo, h);
+          if (q == 0) h0 = h;
+          if (q == last / 2) hm = h;
+          hl = h;
+        }
+      }
+      const uint64_t cls = hm == lo ? 0 : (h0 == lo || hl == lo ? 1 : 2);
+      const uint64_t tr = revcomp(tf, t);
+      const uint64_t hash = mixsplit(tf < tr ? tf : tr, sp.seed);
+      rk.k = (cls << 62) | (hash >> 2);
+      rk.p = (uint32_t)hash << 30;
+    }
+    rk.p |= (a0 + j) * 0x8001u;  // left and right
+    run = j ? ocm_min(run, rk) : rk;
+    sk[at + j] = rk.k;
+    sp_[at + j] = rk.p;
+    pk[at + j] = run.k;
+    pp[at + j] = run.p;
+  }
+  if (n) {
+    OcmRank r{sk[at + n - 1], sp_[at + n - 1]};
+    for (uint32_t j = n - 1; j-- > 0;) {
+      r = ocm_min(OcmRank{sk[at + j], sp_[at + j]}, r);
+      sk[at + j] = r.k;
+      sp_[at + j] = r.p;
+    }
+  }
+  // Minima of the mid and of the mid + 1 lanes after this one.
+  const uint32_t mid = (W - 1) / per - 1;
+  OcmRank m0{0, 0}, m1{0, 0};
+  for (uint32_t d = 1; d <= mid + 1; ++d) {
+    const OcmRank o{__shfl_down_sync(kFull, run.k, d), __shfl_down_sync(kFull, run.p, d)};
+    m0 = m1;
+    m1 = d == 1 ? o : ocm_min(m1, o);
+  }
+  const bool all = warp_valid(pv, rb + (w0 ? w0 - 1 : 0), nw + (uint32_t)k - (w0 ? 0u : 1u), lane);
+  __syncwarp();
+  const uint32_t inverse = ((1u << 20) + (uint32_t)w - 1) / (uint32_t)w;  // x / w for x < 2^9
+  if (a0 + skip <= nw) {
+    uint32_t gt = pv.gt_count(p, k);
+    const uint32_t m = min(per, nw + 1 - a0);
+    // G or T flags of the bases that leave and enter the windows.
+    uint64_t out = m > 1 ? pv.bits32(p) : 0, in = m > 1 ? pv.bits32(p + k) : 0;
+    if (skip) pos[0] = 0xFFFFFFFFu;
+    for (uint32_t j = skip; j < m; ++j) {
+      const uint32_t i = a0 + j;
+      uint32_t je = j + W - 1 - (mid + 1) * per, le = (uint32_t)lane + mid + 1;
+      OcmRank best{sk[at + j], sp_[at + j]};
+      if (je >= per) {
+        je -= per;
+        ++le;
+        best = ocm_min(best, m1);
+      } else if (mid) {
+        best = ocm_min(best, m0);
+      }
+      best = ocm_min(best, OcmRank{pk[le * pitch + je], pp[le * pitch + je]});
+      const uint32_t anchor = gt > (uint32_t)k / 2 ? best.p & 0x7FFFu : (best.p >> 15) & 0x7FFFu;
+      const uint32_t d = anchor - i;
+      const bool ok = all || pv.valid(p + (j - skip), k);
+      pos[i] = ok ? i + d - ((d * inverse) >> 20) * (uint32_t)w : 0xFFFFFFFFu;
+      gt += (uint32_t)(in >> 63) - (uint32_t)(out >> 63);
+      in <<= 2;
+      out <<= 2;
+    }
+  }
+  __syncwarp();
+}
+
+// Selected minimizer positions (see tile_ocm_select_any); pre and suf are one
+// buffer.
+__device__ __forceinline__ void tile_ocm_select(const PackedView& pv, uint64_t rb, uint32_t w0,
+                                                uint32_t nw, const SeedParams& sp,
+                                                const uint16_t* inner, Rank16* pre, Rank16* suf,
+                                                uint32_t* pos, int lane) {
+  const uint32_t W = (uint32_t)(sp.k - sp.ocm.t + 1);
+  if (W > ocm_per_lane(nw, W))
+    tile_ocm_select_wide(pv, rb, w0, nw, sp, inner, reinterpret_cast<uint8_t*>(pre), pos, lane);
+  else
+    tile_ocm_select_any(pv, rb, w0, nw, sp, inner, pre, suf, pos, lane);
+}
+
 // Minimizers of windows [w0, w0+nw) (nw <= kOcmTile), buffers as for
 // tile_ocm_select. Emits in window order, dropping repeats of the previous
 // window's selected position within a run.
 __device__ uint32_t tile_ocm(const PackedView& pv, uint64_t rb, uint32_t w0, uint32_t nw,
-                             const SeedParams& sp, const uint64_t* inner, Rank16* pre,
+                             const SeedParams& sp, const uint16_t* inner, Rank16* pre,
                              Rank16* suf, uint32_t* pos, uint64_t* buf, int lane) {
-  const int m = sp.m;
   tile_ocm_select(pv, rb, w0, nw, sp, inner, pre, suf, pos, lane);
+  // The positions to emit first (about one window in ten), then their keys.
+  uint32_t* list = reinterpret_cast<uint32_t*>(pre);
   uint32_t count = 0;
   for (uint32_t i0 = 1; i0 <= nw; i0 += 32) {
-    uint32_t i = i0 + lane;
-    bool keep = false;
-    uint64_t key = 0;
-    if (i <= nw && pos[i] != 0xFFFFFFFFu && pos[i] != pos[i - 1]) {
-      keep = true;
-      key = canonical_at(pv, rb + w0 - 1 + pos[i], m);
-    }
-    count = warp_append(buf, count, keep, key, lane);
+    const uint32_t i = i0 + lane;
+    const uint32_t at = i <= nw ? pos[i] : 0xFFFFFFFFu;
+    const bool keep = at != 0xFFFFFFFFu && at != pos[i - 1];
+    const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, keep);
+    if (keep) list[count + __popc(ballot & ((1u << lane) - 1u))] = at;
+    count += __popc(ballot);
   }
+  __syncwarp();
+  for (uint32_t i = lane; i < count; i += 32)
+    buf[i] = canonical_at(pv, rb + w0 - 1 + list[i], sp.m);
+  __syncwarp();
   return count;
 }
 
 // Full-m-mer special case (k == m): every canonical m-mer.
-__device__ __forceinline__ uint32_t tile_ocm_full(const PackedView& pv, uint64_t rb, uint32_t w0,
-                                                  uint32_t nw, int m, uint64_t* buf, int lane) {
-  return tile_kmers_short(pv, rb, w0, nw, m, false, 0, 1, buf, lane);
+__device__ __forceinline__ uint32_t tile_ocm_full(const PackedView& pv, const SeedParams& sp,
+                                                  uint64_t rb, uint32_t w0, uint32_t nw,
+                                                  uint64_t* buf, int lane) {
+  return tile_kmers_short(pv, sp, rb, w0, nw, sp.m, false, buf, lane);
 }
 
 }  // namespace zx

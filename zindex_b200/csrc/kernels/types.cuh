@@ -18,6 +18,22 @@ struct SeedParams {
   int klen;        // length of the hashed k-mer: k, or k - z for findere s-mers
   uint64_t seed;
   uint64_t sampling;
+  // d = sampling divides x when x times the inverse of d's odd part, rotated
+  // right by d's factors of two, is at most (2^64 - 1) / d (the divisibility
+  // test of Granlund and Montgomery, PLDI 1994).
+  uint64_t sampling_inverse, sampling_most;
+  int sampling_shift;
+  void set_sampling(uint64_t d) {
+    sampling = d;
+    sampling_shift = 0;
+    sampling_inverse = sampling_most = 0;
+    if (!d) return;
+    sampling_most = ~0ull / d;
+    for (; !(d & 1); d >>= 1) ++sampling_shift;
+    uint64_t inv = d;  // Newton's iteration: right in its low 3, 6, 12, ... bits
+    for (int i = 0; i < 5; ++i) inv *= 2 - d * inv;
+    sampling_inverse = inv;
+  }
   OcmParams ocm;
   LongKmerConsts lk;
   int spaced;       // 1: keys are mapped through `pattern` (k-mers and minimizers)

@@ -53,16 +53,20 @@ struct ColorLoc {
 
 // Shared memory of the dense extraction per warp: one tile's keys (and the
 // staging of long k-mer hashes) and, for minimizers, the open-closed
-// minimizer scratch; no probe descriptors. The block adds the 256-entry inner
-// hash table.
+// minimizer scratch; no probe descriptors. The block adds a table.
 struct DenseSmem {
   static __host__ __device__ size_t warp_bytes(int mode, int k) {
-    size_t b = FusedSmem::key_bytes(mode, k, false);
+    size_t b = FusedSmem::key_bytes(mode, k, false) + 32 * 8;  // (padded runs: extract_short)
     if (mode == 1) b += 2 * FusedSmem::ocm_entries(k) * sizeof(Rank16) + (kTileWindows + 1) * 4 + 16;
     return (b + 15) / 16 * 16;
   }
+  // The block's table: the ranks of inner hashes (minimizers), or the terms
+  // of four bases (k-mers of k > 32).
+  static __host__ __device__ size_t table_bytes(int mode, int k) {
+    return mode != 1 && k > 32 ? 512 * 8 : 256 * 8;
+  }
   static __host__ __device__ size_t total(int mode, int k, int warps) {
-    return 256 * 8 + (size_t)warps * warp_bytes(mode, k);
+    return table_bytes(mode, k) + (size_t)warps * warp_bytes(mode, k);
   }
 };
 
@@ -156,14 +160,14 @@ __global__ void wide_rounds_kernel(const unsigned long long* __restrict__ cursor
 }
 
 // extract_dense_kernel for canonical k-mers of k <= 32: a warp takes several
-// tiles at a time, counts their valid windows, reserves their places with one
-// atomic (one per tile kept the cursor's cache line busy: 1.1 ms for 1e6 tiles
-// on a B200) and writes the keys straight from registers.
+// tiles at a time, counts their valid windows and reserves their places with
+// one atomic; tiles without an invalid base roll their k-mers (tile_kmers_run)
+// through a padded stage.
 __device__ __forceinline__ void extract_short(const BatchView& bv, const SeedParams& sp,
                                               uint64_t* __restrict__ out,
                                               unsigned long long* __restrict__ cursor,
                                               uint32_t warp, uint32_t warps, int lane,
-                                              const WideRound& sg) {
+                                              uint64_t* stage, const WideRound& sg) {
   constexpr uint32_t kFull = 0xFFFFFFFFu;
   uint32_t ntiles = *bv.ntiles;
   if (bv.tile_hi && bv.tile_hi < ntiles) ntiles = bv.tile_hi;
@@ -181,10 +185,15 @@ __device__ __forceinline__ void extract_short(const BatchView& bv, const SeedPar
       first = bv.offsets[t.record] + t.w0;
       nw = t.nw;
     }
-    uint32_t total = 0;
+    uint32_t total = 0, whole = 0;  // whole: tiles without an invalid base
     for (uint32_t j = 0; j < m; ++j) {
       const uint64_t p = __shfl_sync(kFull, first, j);
       const uint32_t w = __shfl_sync(kFull, nw, j);
+      if (warp_valid(bv.pv, p, w + (uint32_t)sp.klen - 1, lane)) {
+        whole |= 1u << j;
+        total += w;
+        continue;
+      }
       for (uint32_t i0 = 0; i0 < w; i0 += 32)
         total += __popc(__ballot_sync(kFull, short_valid(bv.pv, p + i0, min(32u, w - i0), sp.klen, lane)));
     }
@@ -209,6 +218,19 @@ __device__ __forceinline__ void extract_short(const BatchView& bv, const SeedPar
     for (uint32_t j = 0; j < m; ++j) {
       const uint64_t p = __shfl_sync(kFull, first, j);
       const uint32_t w = __shfl_sync(kFull, nw, j);
+      if ((whole >> j) & 1u) {
+        const uint32_t per = (w + 31) / 32, pad = ~per & 1u, inverse = (0x10000u + per - 1) / per;
+        tile_kmers_run(bv.pv, p, w, sp.klen, stage, pad, lane);
+        __syncwarp();
+        for (uint32_t i = lane; i < w; i += 32) {
+          uint64_t key = stage[i + pad * ((i * inverse) >> 16)];
+          if (sp.spaced) key = spaced_canonical(sp.pattern, key);
+          dst[i] = key;
+        }
+        __syncwarp();
+        dst += w;
+        continue;
+      }
       for (uint32_t i0 = 0; i0 < w; i0 += 32) {
         const uint32_t n = min(32u, w - i0);
         const bool keep = short_valid(bv.pv, p + i0, n, sp.klen, lane);
@@ -231,17 +253,23 @@ __global__ void extract_dense_kernel(BatchView bv, SeedParams sp, uint64_t* __re
                                      unsigned long long* __restrict__ cursor, int warps_per_block,
                                      WideRound sg) {
   extern __shared__ __align__(16) uint8_t smem[];
-  uint64_t* inner = reinterpret_cast<uint64_t*>(smem);
-  uint8_t* p = smem + 256 * 8;
+  uint16_t* inner = reinterpret_cast<uint16_t*>(smem);
+  uint8_t* p = smem + DenseSmem::table_bytes(MODE, sp.k);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (MODE == 0 && sp.klen <= 32) {
     extract_short(bv, sp, out, cursor, blockIdx.x * warps_per_block + warp,
-                  gridDim.x * warps_per_block, lane, sg);
+                  gridDim.x * warps_per_block, lane,
+                  reinterpret_cast<uint64_t*>(p + (size_t)warp * DenseSmem::warp_bytes(0, sp.k)), sg);
     return;
   }
   uint8_t* wbase = p + (size_t)warp * DenseSmem::warp_bytes(MODE, sp.k);
   uint64_t* keys = reinterpret_cast<uint64_t*>(wbase);
   uint8_t* ocm = wbase + FusedSmem::key_bytes(MODE, sp.k, false);
+  const uint64_t* quads = nullptr;
+  if (MODE != 1 && sp.klen > 32) {
+    build_long_table(reinterpret_cast<uint64_t*>(smem));
+    quads = reinterpret_cast<const uint64_t*>(smem);
+  }
   build_inner_table(sp, inner);
   __syncthreads();
   uint32_t ntiles = *bv.ntiles;
@@ -249,7 +277,7 @@ __global__ void extract_dense_kernel(BatchView bv, SeedParams sp, uint64_t* __re
   const uint32_t warps_total = gridDim.x * warps_per_block;
   for (uint32_t t = bv.tile_lo + blockIdx.x * warps_per_block + warp; t < ntiles;
        t += warps_total) {
-    uint32_t n = extract_tile<MODE>(bv, sp, bv.tiles[t], keys, ocm, inner, lane);
+    uint32_t n = extract_tile<MODE>(bv, sp, bv.tiles[t], keys, ocm, inner, lane, quads);
     __syncwarp();
     unsigned long long at = 0;
     uint64_t* dst = out;
