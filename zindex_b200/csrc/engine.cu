@@ -491,7 +491,7 @@ Workspace::~Workspace() {
                  wide_seg_cursor, wide_round_first, wide_keys_alt[0], wide_keys_alt[1],
                  wide_hist[0], wide_hist[1], wide_next[0], wide_next[1], round_keys[0],
                  round_keys[1], strobe_anchors, strobe_hashes, strobe_slots,
-                 strobe_count};
+                 strobe_count, strand_bases, strand_counts, strand_totals};
   for (void* p : dev)
     if (p) cudaFree(p);
   void* host[] = {h_bases, h_offsets, h_counts, h_total, h_seg_blocks, h_seg_records};
@@ -1741,8 +1741,10 @@ void Engine::link_strobes(Workspace& ws, const BatchView& bv, uint64_t nbases, c
   cuda_check(cudaGetLastError(), "strobe_anchor_kernel");
   const int len = mode == 1 ? sp_.m : sp_.klen;
   const uint32_t extra = mode == 1 && sp_.k != sp_.m ? (uint32_t)sp_.ocm.w - 1 : 0u;
-  strobe_link_kernel<<<grid, 256, 0, s>>>(bv, sp_, ws.strobe_anchors, ws.strobe_hashes, len,
-                                          extra, ws.strobe_slots, ws.strobe_count);
+  const int dense = mode == 0 || sp_.k == sp_.m;
+  strobe_link_kernel<<<grid, kLinkThreads, 0, s>>>(bv, sp_, ws.strobe_anchors, ws.strobe_hashes,
+                                                   len, extra, dense, ws.strobe_slots,
+                                                   ws.strobe_count);
   cuda_check(cudaGetLastError(), "strobe_link_kernel");
 }
 
@@ -2026,6 +2028,23 @@ void Engine::record_groups(Workspace& ws, const uint8_t* bases, uint64_t nbases,
     if (mean < (uint64_t)launch_.warps) warps = mean <= 2 ? 2 : (mean <= 4 ? 4 : 8);
     query_segments(ws, ws.bases, nb, ws.offsets, n, seg.data(), est.data(), (uint32_t)n, recover,
                    ws.rec_counts, ws.rec_totals, s, warps, prune_ratio);
+    if (strobes) {
+      // The reverse-complement strand too, and per record and colour the
+      // larger count (PreparedRead::new, query_stream.rs:516-534;
+      // Scores::score, query_stream.rs:690-701).
+      ensure_strand_capacity(ws, nb, n);
+      const int bgrid = (int)std::max<uint64_t>(1, std::min<uint64_t>((nb / 16 + 256) / 256, sms_ * 16ull));
+      strobe_reverse_kernel<<<bgrid, 256, 0, s>>>(ws.bases, nb, ws.offsets, n, ws.strand_bases);
+      cuda_check(cudaGetLastError(), "strobe_reverse_kernel");
+      cuda_check(cudaMemsetAsync(ws.strand_counts, 0, n * colors * 8, s), "memset");
+      cuda_check(cudaMemsetAsync(ws.strand_totals, 0, n * 8, s), "memset");
+      query_segments(ws, ws.strand_bases, nb, ws.offsets, n, seg.data(), est.data(), (uint32_t)n,
+                     recover, ws.strand_counts, ws.strand_totals, s, warps, prune_ratio);
+      const int cgrid = (int)std::min<uint64_t>((n * colors + 255) / 256, sms_ * 16ull);
+      strobe_best_kernel<<<cgrid, 256, 0, s>>>(ws.rec_counts, ws.strand_counts, n * colors,
+                                               ws.rec_totals, ws.strand_totals, n, ws.error);
+      cuda_check(cudaGetLastError(), "strobe_best_kernel");
+    }
     on_group(r0, n);
     cuda_check(cudaStreamSynchronize(s), "per-record query");
     check_error_word(ws);
@@ -2038,45 +2057,32 @@ void Engine::query_per_record(Workspace& ws, const uint8_t* bases, uint64_t nbas
                               uint64_t* counts, uint64_t* totals) {
   const uint64_t colors = m_.colors.size();
   cudaStream_t s = ws.stream;
-  auto run = [&](const uint8_t* b, uint64_t* c, uint64_t* t) {
-    record_groups(ws, b, nbases, offsets, records, recover, 0.0, [&](uint64_t r0, uint64_t n) {
-      cuda_check(cudaMemcpyAsync(c + r0 * colors, ws.rec_counts, n * colors * 8,
-                                 cudaMemcpyDeviceToHost, s),
-                 "D2H");
-      cuda_check(cudaMemcpyAsync(t + r0, ws.rec_totals, n * 8, cudaMemcpyDeviceToHost, s), "D2H");
-    });
-  };
-  run(bases, counts, totals);
-  if (!sp_.strobe_max) return;
-  // Randstrobemers: the reverse-complement strand too, and per record and
-  // colour the larger count (PreparedRead::new, query_stream.rs:516-534;
-  // Scores::score, query_stream.rs:690-701).
-  std::vector<uint8_t> rc(nbases);
-  reverse_complement_records(bases, offsets, records, rc.data());
-  std::vector<uint64_t> rcounts(records * colors), rtotals(records);
-  run(rc.data(), rcounts.data(), rtotals.data());
-  for (uint64_t r = 0; r < records; ++r)
-    check(rtotals[r] == totals[r], kEFormat, "canonical anchor counts must agree across strands");
-  for (uint64_t i = 0; i < records * colors; ++i) counts[i] = std::max(counts[i], rcounts[i]);
+  record_groups(ws, bases, nbases, offsets, records, recover, 0.0, [&](uint64_t r0, uint64_t n) {
+    cuda_check(cudaMemcpyAsync(counts + r0 * colors, ws.rec_counts, n * colors * 8,
+                               cudaMemcpyDeviceToHost, s),
+               "D2H");
+    cuda_check(cudaMemcpyAsync(totals + r0, ws.rec_totals, n * 8, cudaMemcpyDeviceToHost, s), "D2H");
+  });
 }
 
-void reverse_complement_records(const uint8_t* bases, const uint64_t* offsets, uint64_t records,
-                                uint8_t* out) {
-  // reverse_complement (src/anchors.rs:257-263): ACGT of either case become
-  // the upper-case complement, every other byte stays a separator.
-  static const struct Table {
-    uint8_t t[256];
-    Table() {
-      for (int i = 0; i < 256; ++i) t[i] = (uint8_t)i;
-      t['A'] = t['a'] = 'T';
-      t['C'] = t['c'] = 'G';
-      t['G'] = t['g'] = 'C';
-      t['T'] = t['t'] = 'A';
-    }
-  } table;
-  for (uint64_t r = 0; r < records; ++r) {
-    const uint64_t a = offsets[r], b = offsets[r + 1];
-    for (uint64_t i = a; i < b; ++i) out[a + (b - 1 - i)] = table.t[bases[i]];
+void Engine::ensure_strand_capacity(Workspace& ws, uint64_t nbases, uint64_t records) {
+  const uint64_t counts = records * std::max<uint64_t>(m_.colors.size(), 1);
+  if (nbases > ws.cap_strand_bases || !ws.strand_bases) {
+    if (ws.strand_bases) cudaFree(ws.strand_bases);
+    ws.strand_bases = nullptr;
+    const uint64_t cap = std::max<uint64_t>({nbases, ws.cap_strand_bases * 3 / 2, 4096});
+    dev_alloc(&ws.strand_bases, cap + 64, "reverse strands");
+    ws.cap_strand_bases = cap;
+  }
+  if (counts > ws.cap_strand_counts || records > ws.cap_strand_records || !ws.strand_counts) {
+    for (void* p : {(void*)ws.strand_counts, (void*)ws.strand_totals})
+      if (p) cudaFree(p);
+    ws.strand_counts = nullptr;
+    ws.strand_totals = nullptr;
+    ws.cap_strand_counts = std::max(counts, ws.cap_strand_counts);
+    ws.cap_strand_records = std::max(records, ws.cap_strand_records);
+    dev_alloc(&ws.strand_counts, ws.cap_strand_counts, "reverse strand counters");
+    dev_alloc(&ws.strand_totals, ws.cap_strand_records, "reverse strand totals");
   }
 }
 
@@ -2084,24 +2090,22 @@ void Engine::query_strobes_host(Workspace& ws, const uint8_t* bases, uint64_t nb
                                 const uint64_t* offsets, uint64_t records, bool recover,
                                 uint64_t* counts, uint64_t* total) {
   check(offsets[0] == 0 && offsets[records] == nbases, kEInval, "offsets must span the bases");
-  const uint64_t colors = std::max<uint64_t>(m_.colors.size(), 1);
-  const uint64_t step = std::max<uint64_t>(1, (32ull << 20) / colors);
-  std::vector<uint64_t> c, t, rel;
-  std::fill(counts, counts + m_.colors.size(), 0);
-  *total = 0;
-  for (uint64_t r0 = 0; r0 < records; r0 += step) {
-    const uint64_t n = std::min(step, records - r0), b0 = offsets[r0];
-    rel.resize(n + 1);
-    for (uint64_t r = 0; r <= n; ++r) rel[r] = offsets[r0 + r] - b0;
-    check(rel[n] <= nbases - b0, kEInval, "offsets must be non-decreasing");
-    c.resize(n * m_.colors.size());
-    t.resize(n);
-    query_per_record(ws, bases + b0, rel[n], rel.data(), n, recover, c.data(), t.data());
-    for (uint64_t r = 0; r < n; ++r) {
-      *total += t[r];
-      for (uint64_t i = 0; i < m_.colors.size(); ++i) counts[i] += c[r * m_.colors.size() + i];
-    }
-  }
+  const uint32_t colors = (uint32_t)m_.colors.size();
+  ensure_capacity(ws, 0, 0, true);
+  ensure_host_capacity(ws, 0, 0);
+  cudaStream_t s = ws.stream;
+  cuda_check(cudaMemsetAsync(ws.counts, 0, colors * 8ull, s), "memset");
+  cuda_check(cudaMemsetAsync(ws.total, 0, 8, s), "memset");
+  record_groups(ws, bases, nbases, offsets, records, recover, 0.0, [&](uint64_t, uint64_t n) {
+    sum_records_kernel<<<(int)((n + kSumRecords - 1) / kSumRecords), 256, 0, s>>>(
+        ws.rec_counts, ws.rec_totals, n, colors, ws.counts, ws.total);
+    cuda_check(cudaGetLastError(), "sum_records_kernel");
+  });
+  cuda_check(cudaMemcpyAsync(ws.h_counts, ws.counts, colors * 8ull, cudaMemcpyDeviceToHost, s), "D2H");
+  cuda_check(cudaMemcpyAsync(ws.h_total, ws.total, 8, cudaMemcpyDeviceToHost, s), "D2H");
+  cuda_check(cudaStreamSynchronize(s), "query");
+  memcpy(counts, ws.h_counts, colors * 8ull);
+  *total = *ws.h_total;
 }
 
 void Engine::query_record_hits(Workspace& ws, const uint8_t* bases, uint64_t nbases,
@@ -2171,6 +2175,7 @@ static void raise_error_word(uint32_t err) {
   if (err & kErrOffsets)
     raise(kEInval, "record offsets must be non-decreasing, end within the bases and span fewer "
                    "than 2^31 bases (offending records were skipped; counts are incomplete)");
+  if (err & kErrStrands) raise(kEFormat, "canonical anchor counts must agree across strands");
   if (err) raise(kETimeout, "a bounded device wait expired during the query");
 }
 

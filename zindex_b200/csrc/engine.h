@@ -92,6 +92,11 @@ struct Workspace {
   uint64_t* strobe_slots = nullptr;
   uint32_t* strobe_count = nullptr;
   uint64_t cap_strobe_bases = 0, cap_strobe_tiles = 0;
+  // Their reverse strands: a record group's bases and counters.
+  uint8_t* strand_bases = nullptr;
+  uint64_t* strand_counts = nullptr;
+  unsigned long long* strand_totals = nullptr;
+  uint64_t cap_strand_bases = 0, cap_strand_counts = 0, cap_strand_records = 0;
   uint64_t* wide_keys2 = nullptr;  // second dense key list (rounds alternate)
   cudaStream_t aux_stream = nullptr;  // wide-row queries: extraction beside the probe
   cudaEvent_t wide_fork = nullptr, wide_ext[2] = {}, wide_probe[2] = {};
@@ -124,10 +129,6 @@ struct Workspace {
   ~Workspace();
   void release_graphs();
 };
-
-// Reverse complement of every record of a host batch, records in place.
-void reverse_complement_records(const uint8_t* bases, const uint64_t* offsets, uint64_t records,
-                                uint8_t* out);
 
 class Engine {
  public:
@@ -307,6 +308,7 @@ class Engine {
   // each tile's linked seeds into ws.strobe_slots / strobe_count.
   void ensure_strobe_capacity(Workspace& ws, uint64_t nbases, uint64_t tiles);
   void link_strobes(Workspace& ws, const BatchView& bv, uint64_t nbases, cudaStream_t s);
+  void ensure_strand_capacity(Workspace& ws, uint64_t nbases, uint64_t records);
   // Runs host records in device groups (one segment per record): after each
   // group's launch, on_group(r0, n) enqueues its read-back on ws.stream; the
   // stream is then synchronised and the error word checked.

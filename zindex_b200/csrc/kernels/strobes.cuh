@@ -18,8 +18,14 @@
 //   the record's last tile also the positions past its last window start,
 //   which only minimizer windows select): a forward scan of the table that
 //   stops at strobe_max, at the record's end and at the first invalid base
-//   (a run break), for any strobe_max. A tile's seeds go to its slot of
-//   kStrobeSlot keys, in position order.
+//   (a run break), for any strobe_max. Only the low 8 bits of a candidate's
+//   hash decide, so a warp stages those of the next positions in shared
+//   memory and each lane scans its own stretch (five instructions a
+//   candidate). A tile's seeds go to its slot of kStrobeSlot keys, in position
+//   order.
+//
+// Both strands of a record are scored on the device: strobe_reverse_kernel
+// makes the reverse complements, strobe_best_kernel keeps the larger count.
 #pragma once
 #include <stdint.h>
 
@@ -91,17 +97,24 @@ __global__ void strobe_anchor_kernel(BatchView bv, SeedParams sp, uint32_t* __re
   }
 }
 
+constexpr uint32_t kStrobeStage = 1024;  // positions whose hash bytes a warp holds
+constexpr int kLinkThreads = 256;
+
 // Seeds of every tile into slots[t * kStrobeSlot ...], their number in
 // slot_count[t]. len: candidate length (k, or m); extra: positions past a
 // record's last window start that can hold candidates (w - 1 for open-closed
-// minimizers with k > m, else 0; at most kStrobeExtra).
-__global__ void strobe_link_kernel(BatchView bv, SeedParams sp, const uint32_t* __restrict__ anchors,
-                                   const uint64_t* __restrict__ hashes, int len, uint32_t extra,
-                                   uint64_t* __restrict__ slots, uint32_t* __restrict__ slot_count) {
+// minimizers with k > m, else 0; at most kStrobeExtra); dense: every position
+// of a run up to its last len bases is a candidate.
+__global__ void __launch_bounds__(kLinkThreads)
+    strobe_link_kernel(BatchView bv, SeedParams sp, const uint32_t* __restrict__ anchors,
+                       const uint64_t* __restrict__ hashes, int len, uint32_t extra, int dense,
+                       uint64_t* __restrict__ slots, uint32_t* __restrict__ slot_count) {
+  __shared__ uint8_t stage_bytes[kLinkThreads / 32][kStrobeStage];
   const int lane = threadIdx.x & 31;
+  uint8_t* stage = stage_bytes[threadIdx.x >> 5];
   const uint32_t ntiles = *bv.ntiles;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const uint64_t dmin = sp.strobe_min, dmax = sp.strobe_max;
+  const uint64_t dmin = max(1u, sp.strobe_min), dmax = sp.strobe_max;
   auto is_anchor = [&](uint64_t p) { return (__ldg(anchors + (p >> 5)) >> (p & 31)) & 1u; };
   for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntiles; t += warps) {
     const Tile tile = bv.tiles[t];
@@ -112,35 +125,130 @@ __global__ void strobe_link_kernel(BatchView bv, SeedParams sp, const uint32_t* 
     // last tile the candidate positions past them.
     uint64_t end = tile.w0 + tile.nw;
     if (end == windows && extra) end = min(end + extra, rlen >= (uint64_t)len ? rlen - len + 1 : 0);
+    const uint64_t starts = rlen - (uint64_t)len + 1;  // (a tile's record has rlen >= len)
     uint64_t* out = slots + (uint64_t)t * kStrobeSlot;
     uint32_t count = 0;
     for (uint64_t q0 = tile.w0; q0 < end; q0 += 32) {
       const uint64_t q = q0 + lane;
-      bool keep = false;
-      uint64_t key = 0;
-      if (q < end && is_anchor(rb + q)) {
-        const uint64_t h = __ldg(hashes + rb + q);
-        uint64_t partner = h;
-        int fewest = 9;
-        for (uint64_t d = 1; d <= dmax; ++d) {
-          const uint64_t c = q + d;
-          // The record ends, or a base of the run does: no more partners.
-          if (c + len > rlen || (bv.pv.inv32(rb + c + len - 1) & 1u)) break;
-          if (d < dmin || !is_anchor(rb + c)) continue;
-          const uint64_t hc = __ldg(hashes + rb + c);
-          const int x = __popcll((h ^ hc) & 0xFFull);
-          if (x < fewest) {
-            fewest = x;
-            partner = hc;
-            if (!fewest) break;
+      const bool keep = q < end && is_anchor(rb + q);
+      uint64_t h = 0, partner = 0;
+      uint64_t reach = 0;  // partners are at most this far
+      if (keep) {
+        h = partner = __ldg(hashes + rb + q);
+        // The valid bases from q + len on, as far as a partner could use them.
+        const uint64_t most = min(dmax, starts - 1 - q);
+        while (reach < most) {
+          const uint32_t bad = bv.pv.inv32(rb + q + len + reach);
+          if (bad) {
+            reach += __ffs(bad) - 1;
+            break;
+          }
+          reach += 32;
+        }
+        reach = min(reach, most);
+      }
+      int fewest = 9;
+      const uint64_t far = min(q0 + 31 + dmax, starts - 1);  // last position any lane may use
+      for (uint64_t c0 = q0 + dmin; c0 <= far; c0 += kStrobeStage) {
+        const uint32_t m = (uint32_t)min((uint64_t)kStrobeStage, far - c0 + 1);
+        if (!__any_sync(0xFFFFFFFFu, keep && q + reach >= c0)) break;
+        __syncwarp();
+        for (uint32_t i = lane; i < m; i += 32) stage[i] = (uint8_t)__ldg(hashes + rb + c0 + i);
+        __syncwarp();
+        if (keep && reach >= dmin && q + reach >= c0) {
+          const uint32_t lo = q + dmin > c0 ? (uint32_t)(q + dmin - c0) : 0u;
+          const uint32_t hi = (uint32_t)min((uint64_t)m - 1, q + reach - c0);
+          const uint32_t mine = (uint32_t)h & 0xFFu;
+          uint32_t best = ~0u;  // differing bits << 16 | place in the stage: the first of the fewest
+          if (dense) {
+#pragma unroll 4
+            for (uint32_t i = lo; i <= hi; ++i) best = min(best, (__popc(mine ^ stage[i]) << 16) | i);
+          } else {
+            for (uint32_t i0 = lo; i0 <= hi; i0 += 32) {
+              // Candidates among positions i0 .. i0 + 31 (bits past hi cleared).
+              const uint64_t p = rb + c0 + i0;
+              const uint64_t two = (uint64_t)__ldg(anchors + (p >> 5)) |
+                                   ((uint64_t)((p & 31) ? __ldg(anchors + (p >> 5) + 1) : 0u) << 32);
+              uint32_t x = (uint32_t)(two >> (p & 31));
+              if (hi - i0 < 31) x &= (2u << (hi - i0)) - 1u;
+              for (; x; x &= x - 1) {
+                const uint32_t i = i0 + __ffs(x) - 1;
+                best = min(best, (__popc(mine ^ stage[i]) << 16) | i);
+              }
+            }
+          }
+          if (best != ~0u && (int)(best >> 16) < fewest) {
+            fewest = (int)(best >> 16);
+            partner = __ldg(hashes + rb + c0 + (best & 0xFFFFu));
           }
         }
-        key = (h >> 1) + (partner >> 1);
-        keep = true;
       }
-      count = warp_append(out, count, keep, key, lane);
+      count = warp_append(out, count, keep, (h >> 1) + (partner >> 1), lane);
     }
     if (lane == 0) slot_count[t] = count;
+  }
+}
+
+// Reverse complement of every record into out, records in place (src/
+// anchors.rs:257-263): A, C, G and T of either case become the upper-case
+// complement, every other byte stays. A thread takes 16 bases; offsets that
+// the tile planner reports are not followed (bases outside every record stay
+// unwritten).
+__global__ void strobe_reverse_kernel(const uint8_t* __restrict__ bases, uint64_t nbases,
+                                      const uint64_t* __restrict__ offsets, uint64_t records,
+                                      uint8_t* __restrict__ out) {
+  const uint64_t pieces = (nbases + 15) / 16;
+  for (uint64_t x = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; x < pieces;
+       x += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t i0 = x * 16, i1 = min(nbases, i0 + 16);
+    uint64_t lo = 0, hi = records;  // last record that starts at or before i0
+    while (hi - lo > 1) {
+      const uint64_t mid = (lo + hi) >> 1;
+      if (__ldg(offsets + mid) <= i0) lo = mid;
+      else hi = mid;
+    }
+    for (uint64_t i = i0, r = lo; i < i1; ++i) {
+      while (r + 1 < records && __ldg(offsets + r + 1) <= i) ++r;
+      const uint64_t a = __ldg(offsets + r), b = __ldg(offsets + r + 1);
+      if (i < a || i >= b || b > nbases) continue;
+      const uint8_t c = bases[i];
+      const uint32_t code = encode_base(c);
+      out[a + (b - 1 - i)] = code > 3 ? c : (uint8_t)(0x41434754u >> (8 * code));
+    }
+  }
+}
+
+// counts = the larger of the two strands' counts (records x colours); the
+// strands' totals must agree.
+__global__ void strobe_best_kernel(uint64_t* __restrict__ counts, const uint64_t* __restrict__ other,
+                                   uint64_t n, const unsigned long long* __restrict__ totals,
+                                   const unsigned long long* __restrict__ other_totals,
+                                   uint64_t records, uint32_t* __restrict__ err) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
+       i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t c = other[i];
+    if (c > counts[i]) counts[i] = c;
+    if (i < records && totals[i] != other_totals[i]) atomicOr(err, kErrStrands);
+  }
+}
+
+// sums[c] += the counts of colour c over the records, *total += their totals:
+// kSumRecords records per block.
+constexpr uint32_t kSumRecords = 32;
+__global__ void sum_records_kernel(const uint64_t* __restrict__ counts,
+                                   const unsigned long long* __restrict__ totals, uint64_t records,
+                                   uint32_t colors, uint64_t* __restrict__ sums,
+                                   unsigned long long* __restrict__ total) {
+  const uint64_t r0 = (uint64_t)blockIdx.x * kSumRecords, r1 = min(records, r0 + kSumRecords);
+  for (uint32_t c = threadIdx.x; c < colors; c += blockDim.x) {
+    unsigned long long s = 0;
+    for (uint64_t r = r0; r < r1; ++r) s += counts[r * colors + c];
+    if (s) atomicAdd(reinterpret_cast<unsigned long long*>(sums + c), s);
+  }
+  if (threadIdx.x == 0) {
+    unsigned long long s = 0;
+    for (uint64_t r = r0; r < r1; ++r) s += totals[r];
+    if (s) atomicAdd(total, s);
   }
 }
 

@@ -9,6 +9,7 @@ namespace zx {
 
 // Bits of a query's device error word.
 constexpr uint32_t kErrWait = 1u;     // a bounded wait expired (staged gather)
+constexpr uint32_t kErrStrands = 4u;  // a record's two strands have different anchor counts
 constexpr uint32_t kErrOffsets = 2u;  // a record's offsets decrease, leave the bases, or span 2^31
 
 struct SeedParams {
