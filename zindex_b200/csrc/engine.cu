@@ -1106,6 +1106,25 @@ bool Engine::wide_eligible(int warps) const {
 
 bool Engine::wide_form(const QueryLaunch& l) const { return l.wide && wide_eligible(l.warps); }
 
+bool Engine::dense_batch(uint64_t nbases) const {
+  if (!launch_default_ || launch_.wide || !win_slices_ || nbases <= kSmallBases ||
+      nbases > kRoundKeys)
+    return false;
+  uint64_t seeds = nbases;
+  if (sp_.mode == kMinimizers) seeds = 2 * nbases / (uint64_t)(sp_.ocm.w + 1);
+  if (sp_.mode == kModimizers) seeds = nbases / std::max<uint64_t>(sp_.sampling, 1);
+  return seeds >= 2 * win_min_keys_;
+}
+
+QueryLaunch Engine::dense_launch() const {
+  QueryLaunch l = default_fused_launch();
+  l.wide = 1;
+  l.order = 1;
+  l.warps = 4;
+  l.smem_counters = 1;
+  return l;
+}
+
 void Engine::wide_shape(const QueryLaunch& l, int& J, int& HQ, uint32_t* team) const {
   const uint32_t T = (uint32_t)l.warps * 32u, nc = wide_chunks();
   // Rows of at most half a block of chunks: teams of the next power of two of
@@ -1213,6 +1232,11 @@ void Engine::set_launch(const QueryLaunch& l) {
   check(fused_smem_bytes(l) <= 227 * 1024, kEInval, "launch needs too much shared memory");
   std::lock_guard<std::mutex> lock(mu_);
   launch_ = l;
+  const QueryLaunch d = default_launch();
+  launch_default_ = l.team == d.team && l.warps == d.warps && l.blocks == d.blocks &&
+                    l.smem_counters == d.smem_counters && l.stage_bytes == d.stage_bytes &&
+                    l.min_blocks == d.min_blocks && l.planes == d.planes && l.split == d.split &&
+                    l.wide == d.wide && l.order == d.order;
   ws_->release_graphs();
 }
 
@@ -1228,14 +1252,16 @@ void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, b
                              uint64_t round_bases) {
   const uint64_t colors = m_.colors.size();
   // Split minimizer and wide-row queries: key slots allocated before any graph capture.
-  const bool wide = wide_form(launch_);
-  const bool whole = wide && !segmented && ensure_round_capacity(ws, std::min(nbases, round_bases));
-  if (kernel_mode(launch_) == 4 || (wide && !whole)) ensure_split_capacity(ws);
+  const uint64_t at_once = std::min(nbases, round_bases);
+  const bool dense = !segmented && dense_batch(at_once);
+  const bool wide = wide_form(launch_) || dense;
+  const bool whole = wide && !segmented && ensure_round_capacity(ws, at_once);
+  if (kernel_mode(launch_) == 4 || (wide_form(launch_) && !whole)) ensure_split_capacity(ws);
   const bool rounds =
-      !whole && nbases / kTileWindows + records + nbases / kFindereTask + 1 > kSplitTiles;
+      !whole && wide_form(launch_) && nbases / kTileWindows + records + nbases / kFindereTask + 1 > kSplitTiles;
   if (wide) ensure_cursors(ws);
-  if (wide && rounds) ensure_wide_pipeline(ws);
-  if (wide && launch_.order && !segmented) {
+  if (rounds) ensure_wide_pipeline(ws);
+  if (((wide_form(launch_) && launch_.order) || (dense && whole)) && !segmented) {
     ensure_order_capacity(ws, 0, whole);
     if (rounds) ensure_order_capacity(ws, 1, whole);
   }
@@ -1401,6 +1427,7 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   // Small batches: one block packs and plans (one launch for pack, count,
   // scan and fill), and with few colours the fused kernel adds into the
   // caller's counters (no reduction launch).
+  const bool dense = dense_batch(nbases) && ensure_round_capacity(ws, nbases);
   const bool small = records <= kSmallRecords && nbases <= kSmallBases && !wide_form(l) &&
                      kernel_mode(l) != 4;
   if (small) {
@@ -1415,10 +1442,24 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
     cuda_check(cudaGetLastError(), "pack_kernel");
     plan_tiles(ws, offsets, records, nbases, s);
   }
+  const uint64_t tiles_bound = nbases / kTileWindows + records + nbases / kFindereTask + 1;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  cuda_check(cudaStreamIsCapturing(s, &capturing), "cudaStreamIsCapturing");
+  const bool timed = timing_ && capturing == cudaStreamCaptureStatusNone;
+  if (wide_form(l) || dense) {
+    // Indexes of narrow rows take the window probe for batches of many more
+    // seeds than rows, and the fused kernel for the others.
+    const BatchView bv{PackedView{ws.packed, ws.invalid}, offsets, ws.tiles, ws.tile_first + records,
+                       ws.fstate};
+    if (timed) cuda_check(cudaEventRecord(ev_begin_, s), "cudaEventRecord");
+    run_wide(ws, wide_form(l) ? l : dense_launch(), bv, tiles_bound, nbases, recover, counts, total,
+             0, s);
+    if (timed) cuda_check(cudaEventRecord(ev_end_, s), "cudaEventRecord");
+    return;
+  }
   const int kmode = kernel_mode(l);
   const size_t smem = fused_smem_bytes(l);
   const int blocks_cap = max_blocks(l);
-  uint64_t tiles_bound = nbases / kTileWindows + records + nbases / kFindereTask + 1;
   uint64_t want = (tiles_bound + l.warps - 1) / l.warps;
   int blocks = l.blocks > 0 ? std::min(l.blocks, blocks_cap)
                             : (int)std::min<uint64_t>((uint64_t)blocks_cap, std::max<uint64_t>(want, 1));
@@ -1431,9 +1472,6 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
     cuda_check(cudaMemsetAsync(ws.fstate, 0,
                                (uint64_t)blocks * l.warps * 2 * m_.colors.size() * 4, s),
                "memset");
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  cuda_check(cudaStreamIsCapturing(s, &capturing), "cudaStreamIsCapturing");
-  const bool timed = timing_ && capturing == cudaStreamCaptureStatusNone;
   if (timed) cuda_check(cudaEventRecord(ev_begin_, s), "cudaEventRecord");
   FusedFn fn = fused_for(kmode, l);
   // The dynamic shared-memory limit is a property of the kernel function, shared by
@@ -1447,11 +1485,6 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
                                                                                colors, counts);
     cuda_check(cudaGetLastError(), "reduce_counters_kernel");
   };
-  if (wide_form(l)) {
-    run_wide(ws, bv, tiles_bound, nbases, recover, counts, total, 0, s);
-    if (timed) cuda_check(cudaEventRecord(ev_end_, s), "cudaEventRecord");
-    return;
-  }
   if (kmode != 4) {
     fn<<<blocks, l.warps * 32, smem, s>>>(recover ? d_ix_rec_ : d_ix_norec_, bv, sp_, l, ws.partial,
                                           counts, total, ws.error);
@@ -1489,15 +1522,14 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   if (timed) cuda_check(cudaEventRecord(ev_end_, s), "cudaEventRecord");
 }
 
-void Engine::run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, uint64_t max_keys,
-                      bool recover, uint64_t* counts, unsigned long long* total, uint32_t segments,
+void Engine::run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv,
+                      uint64_t tiles_bound, uint64_t max_keys, bool recover, uint64_t* counts, unsigned long long* total, uint32_t segments,
                       cudaStream_t s, double prune_ratio) {
   // Rounds of up to kSplitTiles tiles; per round the extraction kernel
   // appends the tiles' seeds to one dense list (segmented: each segment's
   // seeds to its own part of it), the wide probe counts them, and the block
   // counters are added up (segmented: each block adds its counters to the
   // segment it leaves).
-  const QueryLaunch& l = launch_;
   const size_t smem = fused_smem_bytes(l);
   const int blocks_cap = max_blocks(l);
   int J, HQ;
@@ -1677,8 +1709,8 @@ void Engine::ensure_order_capacity(Workspace& ws, int b, bool whole) {
 }
 
 bool Engine::ensure_round_capacity(Workspace& ws, uint64_t keys) {
-  if (keys > kRoundKeys) return false;
-  const int lists = launch_.order ? 2 : 1;
+  if (keys > kRoundKeys || keys >= ws.round_refused) return false;
+  const int lists = launch_.wide && !launch_.order ? 1 : 2;
   bool have = true;
   for (int i = 0; i < lists; ++i) have &= ws.round_keys[i] && ws.cap_round_keys >= keys;
   if (have) return true;
@@ -1697,6 +1729,7 @@ bool Engine::ensure_round_capacity(Workspace& ws, uint64_t keys) {
         if (ws.round_keys[j]) cudaFree(ws.round_keys[j]);
         ws.round_keys[j] = nullptr;
       }
+      ws.round_refused = keys;  // (not tried again: the call may be under capture)
       return false;
     }
   ws.cap_round_keys = cap;
@@ -1841,7 +1874,8 @@ void Engine::query_segments(Workspace& ws, const uint8_t* bases, uint64_t nbases
     BatchView bv{PackedView{ws.packed, ws.invalid}, offsets, ws.tiles, ws.tile_first + records,
                  ws.fstate};
     const uint64_t tiles_bound = nbases / kTileWindows + records + nbases / kFindereTask + 1;
-    run_wide(ws, bv, tiles_bound, nbases, recover, counts, totals, segments, s, prune_ratio);
+    run_wide(ws, launch_, bv, tiles_bound, nbases, recover, counts, totals, segments, s,
+             prune_ratio);
     return;
   }
   QueryLaunch l = fused_launch(launch_);
@@ -1863,12 +1897,16 @@ void Engine::query_segments(Workspace& ws, const uint8_t* bases, uint64_t nbases
   const uint32_t wpb = (uint32_t)l.warps;
   // Grid shares: proportional to the estimated tiles, at least one block,
   // at most one warp per tile.
+  // With more segments than blocks fit, a long one still gets enough blocks
+  // that its warps take no more tiles than the average warp (at least 4).
   uint64_t est_total = 0;
   for (uint32_t i = 0; i < segments; ++i) est_total += est_tiles[i];
+  const uint64_t warp_tiles = std::max<uint64_t>(4, est_total / ((uint64_t)cap * wpb));
   uint32_t blocks = 0;
   for (uint32_t i = 0; i < segments; ++i) {
     ws.h_seg_blocks[i] = blocks;
     uint64_t share = est_total ? est_tiles[i] * (uint64_t)cap / est_total : 1;
+    share = std::max<uint64_t>(share, est_tiles[i] / (wpb * warp_tiles));
     share = std::min<uint64_t>(share, (est_tiles[i] + wpb - 1) / wpb);
     blocks += (uint32_t)std::max<uint64_t>(share, 1);
     ws.h_seg_records[i] = seg_records[i];
@@ -2026,6 +2064,7 @@ void Engine::record_groups(Workspace& ws, const uint8_t* bases, uint64_t nbases,
     int warps = 0;
     const uint64_t mean = (tiles + n - 1) / n;
     if (mean < (uint64_t)launch_.warps) warps = mean <= 2 ? 2 : (mean <= 4 ? 4 : 8);
+    if (2 * tiles <= 3 * n) warps = 1;
     query_segments(ws, ws.bases, nb, ws.offsets, n, seg.data(), est.data(), (uint32_t)n, recover,
                    ws.rec_counts, ws.rec_totals, s, warps, prune_ratio);
     if (strobes) {

@@ -84,7 +84,7 @@ struct Workspace {
   uint32_t* wide_next[2] = {};
   // Wide-row queries of one round: the whole batch's keys, and in order.
   uint64_t* round_keys[2] = {};
-  uint64_t cap_round_keys = 0;
+  uint64_t cap_round_keys = 0, round_refused = ~0ull;
   // Randstrobemer queries: candidate bits and strobe hashes per base, each
   // tile's linked seeds (kStrobeSlot per tile) and their numbers.
   uint32_t* strobe_anchors = nullptr;
@@ -160,6 +160,12 @@ class Engine {
   uint32_t wide_chunks() const;
   bool wide_eligible(int warps) const;
   bool wide_form(const QueryLaunch& l) const;
+  // Whether an unsegmented batch of an index that defaults to the fused kernel
+  // (rows of fewer than 16 chunks; the launch not changed) has so many more
+  // seeds than rows that sorting it for the window probe pays, and the launch
+  // it then runs with.
+  bool dense_batch(uint64_t nbases) const;
+  QueryLaunch dense_launch() const;
   void wide_shape(const QueryLaunch& l, int& J, int& HQ, uint32_t* team = nullptr) const;
   size_t fused_smem_bytes(const QueryLaunch& l) const;
   int max_blocks(const QueryLaunch& l) const;
@@ -296,8 +302,8 @@ class Engine {
   // prune_ratio > 0 (segmented per-record reports): threshold pruning of the
   // colours that cannot reach count / total >= prune_ratio.
   // max_keys: no more seeds than this in the batch (its bases).
-  void run_wide(Workspace& ws, const BatchView& bv, uint64_t tiles_bound, uint64_t max_keys,
-                bool recover, uint64_t* counts, unsigned long long* total, uint32_t segments,
+  void run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv, uint64_t tiles_bound,
+                uint64_t max_keys, bool recover, uint64_t* counts, unsigned long long* total, uint32_t segments,
                 cudaStream_t s, double prune_ratio = 0.0);
   // Buckets of the ordered rounds and the window probe's slices of the rows
   // (kernels/window_probe.cuh).
@@ -323,6 +329,7 @@ class Engine {
   int sms_ = 0;
   SeedParams sp_{};
   QueryLaunch launch_{};
+  bool launch_default_ = true;
   DevIndex host_ix_{};
   DevIndex* d_ix_rec_ = nullptr;    // with recovery
   DevIndex* d_ix_norec_ = nullptr;  // recovery disabled
