@@ -25,17 +25,17 @@ CASES = [
 ]
 
 
-def _index(d, colors, **opts):
+def _index(base, colors, **opts):
     lengths = [2000 if c % 3 == 0 else (4000 if c % 3 == 1 else 9000) for c in range(colors)]
-    (d / "g").mkdir()
+    (base / "g").mkdir()
     lines = []
     for c, n in enumerate(lengths):
-        p = d / "g" / f"g{c}.fa"
+        p = base / "g" / f"g{c}.fa"
         helpers.write_fasta(p, [dna(n, 31 + c)])
         lines.append(f"g{c}\t{p}")
-    (d / "fof.tsv").write_text("\n".join(lines) + "\n")
-    build_index(d / "fof.tsv", d / "index", min_docs=1, **opts)
-    return d / "index", [dna(n, 31 + c) for c, n in enumerate(lengths)]
+    (base / "fof.tsv").write_text("\n".join(lines) + "\n")
+    build_index(base / "fof.tsv", base / "index", min_docs=1, **opts)
+    return base / "index", [dna(n, 31 + c) for c, n in enumerate(lengths)]
 
 
 @pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(f"{k}{v}" for k, v in c.items()))
@@ -71,3 +71,32 @@ def test_window_probe_around_its_threshold(gpu, oracle, tmp_path):
             got, total = index.query_records(bases, offsets)
             assert total == want_total
             np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("case", [dict(colors=64, H=4, b=8, k=31), dict(colors=9, H=3, b=16, k=25),
+                                  dict(colors=30, H=2, b=4, k=45, groups="0,1;5,6"),
+                                  dict(colors=100, H=8, b=8, mode="modimizers", k=31, d=4),
+                                  dict(colors=100, H=4, b=8, mode="minimizers", k=31, m=21)],
+                         ids=lambda c: "-".join(f"{k}{v}" for k, v in c.items()))
+def test_dense_batches_of_narrow_rows(gpu, oracle, tmp_path, case):
+    """Batches past 1 MiB of an index that defaults to the fused kernel: the
+    window probe, and the fused kernel itself once a launch names it."""
+    import zindex_b200 as zx
+
+    ix, genomes = _index(tmp_path, **case)
+    reads = sample_reads(genomes, np.random.default_rng(8), 8000, 151, n_runs=0.05)
+    bases, offsets = zx.pack_records(reads)
+    assert len(bases) > 1 << 20
+    with zx.Index(ix) as index:
+        assert not index.launch()["wide"]
+        for recover in (True, False):
+            want, want_total = oracle.query_records(ix, bases, offsets, recover=recover)
+            for cut in (1, 4):  # chunks past and below 1 MiB
+                index.set_launch(cut=cut)
+                got, total = index.query_records(bases, offsets, recover=recover)
+                assert total == want_total
+                np.testing.assert_array_equal(got, want)
+        index.set_launch(planes=0)
+        got, total = index.query_records(bases, offsets, recover=False)
+        assert total == want_total
+        np.testing.assert_array_equal(got, want)

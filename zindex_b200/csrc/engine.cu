@@ -12,6 +12,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
+#include "kernels/findere.cuh"
 #include "kernels/key_order.cuh"
 #include "kernels/query_kernels.cuh"
 #include "kernels/record_hits.cuh"
@@ -124,7 +125,9 @@ FusedFn fused_mode(int mode) {
 // blocks per SM) x gather (register teams with per-hit counter updates,
 // staged ring, or register teams with bit-plane counters).
 FusedFn fused_for(int mode, const QueryLaunch& l) {
-  // Findere has one form: the row-index probe with per-colour position masks.
+  // Findere: position masks and bit-sliced runs (mode 5), else the row-index
+  // probe with per-colour round masks.
+  if (mode == 5) return l.min_blocks == 3 ? findere_query_kernel<3> : findere_query_kernel<2>;
   if (mode == 3) return l.min_blocks == 3 ? fused_query_kernel<3, 3, 2> : fused_query_kernel<3, 2, 2>;
   // Probe of seeds extracted beforehand (split minimizer queries): row-index form only.
   if (mode == 4)
@@ -416,8 +419,9 @@ void Engine::query_device_noalloc(const uint8_t* bases, uint64_t nbases, const u
   l.stage_bytes = 0;
   l.blocks = 0;
   l.split = 0;
-  const size_t smem = fused_smem_bytes(l);
-  FusedFn fn = fused_for(sp_.mode, l);
+  l = run_launch(l);
+  const size_t smem = launch_smem_bytes(l);
+  FusedFn fn = fused_for(kernel_mode(l), l);
   cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
              "cudaFuncSetAttribute");
   int per_sm = 0;
@@ -427,7 +431,7 @@ void Engine::query_device_noalloc(const uint8_t* bases, uint64_t nbases, const u
   int blocks = (int)std::min<uint64_t>((uint64_t)std::max(1, per_sm) * sms_, std::max<uint64_t>(want, 1));
   l.blocks = blocks;
   const uint64_t fstate_bytes =
-      m_.index_mode == kFindere && m_.colors.size() > kFindereSmemColors
+      m_.index_mode == kFindere && !findere_dense_ && m_.colors.size() > kFindereSmemColors
           ? (uint64_t)blocks * l.warps * 2 * m_.colors.size() * 4
           : 0;
   // Scratch layout, every region 256-byte aligned.
@@ -475,6 +479,7 @@ void Engine::query_device_noalloc(const uint8_t* bases, uint64_t nbases, const u
     cuda_check(cudaGetLastError(), "fill_tiles_kernel");
   }
   BatchView bv{PackedView{packed, invalid}, offsets, tile_list, tile_first + records, fstate};
+  bv.color_loc = d_color_loc_;
   fn<<<blocks, l.warps * 32, smem, s>>>(recover ? d_ix_rec_ : d_ix_norec_, bv, sp_, l, nullptr,
                                         counts, total, err);
   cuda_check(cudaGetLastError(), "fused_query_kernel");
@@ -904,6 +909,20 @@ void Engine::load(const std::string& dir, const OpenOptions& options) {
   norec.rec = DevRecovery{nullptr, nullptr, nullptr, 0, nullptr};
   cuda_check(cudaMemcpy(d_ix_norec_, &norec, sizeof(DevIndex), cudaMemcpyHostToDevice), "upload");
   plan_windows();
+  if (m_.index_mode == kFindere && m_.fingerprint_bits >= 4 && wide_chunks() <= kFindereChunks) {
+    std::vector<bool> banked(m_.colors.size(), false);
+    bool single = true;
+    for (const auto& cls : m_.classes)
+      for (const GroupMeta& g : m_.banks[cls[0]].groups) {
+        single &= g.members.size() == 1;
+        for (auto c : g.members)
+          if (c < banked.size()) banked[c] = true;
+      }
+    QueryLaunch one = default_fused_launch();
+    one.warps = 1;
+    findere_dense_ = single && findere_smem_bytes(one) <= kFindereBlockBytes &&
+                     std::find(banked.begin(), banked.end(), false) == banked.end();
+  }
   launch_ = default_launch();
   ws_ = make_workspace();
   load_s_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
@@ -1147,6 +1166,7 @@ void Engine::check_not_strobes() const {
 }
 
 int Engine::kernel_mode(const QueryLaunch& l) const {
+  if (m_.index_mode == kFindere) return findere_dense_ ? 5 : 3;
   return l.split && sp_.mode == kMinimizers && l.planes == 1 && l.stage_bytes == 0 ? 4 : sp_.mode;
 }
 
@@ -1154,9 +1174,25 @@ size_t Engine::fused_smem_bytes(const QueryLaunch& l) const {
   if (wide_form(l))
     return WideSmem::total((uint32_t)m_.colors.size(), host_ix_.classes, m_.hashes,
                            l.smem_counters);
-  const int mode = kernel_mode(l);
+  const int mode = m_.index_mode == kFindere ? 3 : kernel_mode(l);
   return FusedSmem::total(mode, sp_.k, (uint32_t)m_.colors.size(), host_ix_.classes, m_.hashes, l,
                           FusedSmem::shared_words(mode, host_ix_, l), sp_.strobe_max != 0);
+}
+
+size_t Engine::findere_smem_bytes(const QueryLaunch& l) const {
+  return FindereSmem::total(sp_.k, (uint32_t)m_.colors.size(), wide_chunks(), host_ix_.classes,
+                            m_.hashes, sp_.k - sp_.klen, l);
+}
+
+QueryLaunch Engine::run_launch(const QueryLaunch& l) const {
+  QueryLaunch r = l;
+  if (findere_dense_)
+    while (r.warps > 1 && findere_smem_bytes(r) > kFindereBlockBytes) r.warps /= 2;
+  return r;
+}
+
+size_t Engine::launch_smem_bytes(const QueryLaunch& l) const {
+  return findere_dense_ ? findere_smem_bytes(l) : fused_smem_bytes(l);
 }
 
 int Engine::max_blocks(const QueryLaunch& l) const {
@@ -1167,7 +1203,7 @@ int Engine::max_blocks(const QueryLaunch& l) const {
       cached_for_.cut == l.cut && cached_for_.split == l.split && cached_for_.wide == l.wide)
     return cached_blocks_;
   int per_sm = 0;
-  size_t smem = fused_smem_bytes(l);
+  size_t smem = launch_smem_bytes(l);
   if (wide_form(l)) {
     int J, HQ;
     wide_shape(l, J, HQ);
@@ -1302,7 +1338,7 @@ void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, b
     ws.cap_tiles = tiles;
     ws.release_graphs();
   }
-  if (m_.index_mode == kFindere) {
+  if (m_.index_mode == kFindere && !findere_dense_) {
     const uint64_t need = (uint64_t)max_blocks(launch_) * launch_.warps * 2 * std::max<uint64_t>(colors, 1);
     if (need > ws.cap_fstate) {
       if (ws.fstate) cudaFree(ws.fstate);
@@ -1311,7 +1347,7 @@ void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, b
       ws.release_graphs();
     }
   }
-  uint64_t partial = (uint64_t)max_blocks(launch_) * colors;
+  uint64_t partial = (uint64_t)max_blocks(run_launch(launch_)) * colors;
   if (partial > ws.cap_partial) {
     if (ws.partial) cudaFree(ws.partial);
     dev_alloc(&ws.partial, partial, "block counters");
@@ -1457,8 +1493,9 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
     if (timed) cuda_check(cudaEventRecord(ev_end_, s), "cudaEventRecord");
     return;
   }
+  l = run_launch(l);
   const int kmode = kernel_mode(l);
-  const size_t smem = fused_smem_bytes(l);
+  const size_t smem = launch_smem_bytes(l);
   const int blocks_cap = max_blocks(l);
   uint64_t want = (tiles_bound + l.warps - 1) / l.warps;
   int blocks = l.blocks > 0 ? std::min(l.blocks, blocks_cap)
@@ -1466,9 +1503,10 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   l.blocks = blocks;
   BatchView bv{PackedView{ws.packed, ws.invalid}, offsets, ws.tiles, ws.tile_first + records,
                ws.fstate};
+  bv.color_loc = d_color_loc_;
   // Findere round state: in shared memory for up to kFindereSmemColors
   // colours, else in this zeroed scratch.
-  if (m_.index_mode == kFindere && m_.colors.size() > kFindereSmemColors)
+  if (m_.index_mode == kFindere && !findere_dense_ && m_.colors.size() > kFindereSmemColors)
     cuda_check(cudaMemsetAsync(ws.fstate, 0,
                                (uint64_t)blocks * l.warps * 2 * m_.colors.size() * 4, s),
                "memset");
@@ -1893,6 +1931,7 @@ void Engine::query_segments(Workspace& ws, const uint8_t* bases, uint64_t nbases
           "a randstrobemer query holds at most 262,144 tiles (about 64 Mbases) per launch");
     ensure_strobe_capacity(ws, nbases, std::max<uint64_t>(tiles, 1));
   }
+  l = run_launch(l);
   const int cap = max_blocks(l);
   const uint32_t wpb = (uint32_t)l.warps;
   // Grid shares: proportional to the estimated tiles, at least one block,
@@ -1920,7 +1959,8 @@ void Engine::query_segments(Workspace& ws, const uint8_t* bases, uint64_t nbases
     ws.cap_partial = (uint64_t)blocks * colors;
     ws.release_graphs();
   }
-  if (m_.index_mode == kFindere && (uint64_t)blocks * wpb * 2 * colors > ws.cap_fstate) {
+  if (m_.index_mode == kFindere && !findere_dense_ &&
+      (uint64_t)blocks * wpb * 2 * colors > ws.cap_fstate) {
     if (ws.fstate) cudaFree(ws.fstate);
     dev_alloc(&ws.fstate, (uint64_t)blocks * wpb * 2 * colors, "findere colour state");
     ws.cap_fstate = (uint64_t)blocks * wpb * 2 * colors;
@@ -1945,20 +1985,21 @@ void Engine::query_segments(Workspace& ws, const uint8_t* bases, uint64_t nbases
                                                               segments, ws.seg_tiles);
   cuda_check(cudaGetLastError(), "segment_tiles_kernel");
   l.blocks = (int)blocks;
-  const int kmode = strobes ? 4 : sp_.mode;
+  const int kmode = strobes ? 4 : kernel_mode(l);
   const size_t smem = strobes ? FusedSmem::total(4, sp_.k, (uint32_t)colors, host_ix_.classes,
                                                  m_.hashes, l,
                                                  FusedSmem::shared_words(4, host_ix_, l), true)
-                              : fused_smem_bytes(l);
+                              : launch_smem_bytes(l);
   BatchView bv{PackedView{ws.packed, ws.invalid}, offsets, ws.tiles, ws.tile_first + records,
                ws.fstate, segments, ws.seg_blocks, ws.seg_tiles};
+  bv.color_loc = d_color_loc_;
   if (strobes) {
     link_strobes(ws, bv, nbases, s);
     bv.prekeys = ws.strobe_slots;
     bv.prekey_count = ws.strobe_count;
     bv.prekey_stride = kStrobeSlot;
   }
-  if (m_.index_mode == kFindere && colors > kFindereSmemColors)
+  if (m_.index_mode == kFindere && !findere_dense_ && colors > kFindereSmemColors)
     cuda_check(cudaMemsetAsync(ws.fstate, 0, (uint64_t)blocks * wpb * 2 * colors * 4, s), "memset");
   FusedFn fn = fused_for(kmode, l);
   cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
@@ -1989,7 +2030,7 @@ void Engine::record_groups(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   // for findere, the extra per-warp colour state stay within 256 MiB each.
   const uint64_t budget = 256ull << 20;
   uint64_t gmax = budget / (colors * 8);
-  if (m_.index_mode == kFindere) gmax = std::min<uint64_t>(gmax, budget / (colors * 8 * launch_.warps));
+  if (m_.index_mode == kFindere && !findere_dense_) gmax = std::min<uint64_t>(gmax, budget / (colors * 8 * launch_.warps));
   gmax = std::max<uint64_t>(1, std::min<uint64_t>(gmax, 1ull << 20));
   // Randstrobemer groups: one launch's tile slots and a candidate table of
   // 8 bytes per base (64 Mi bases).

@@ -168,6 +168,12 @@ class Engine {
   QueryLaunch dense_launch() const;
   void wide_shape(const QueryLaunch& l, int& J, int& HQ, uint32_t* team = nullptr) const;
   size_t fused_smem_bytes(const QueryLaunch& l) const;
+  // Findere by position masks (findere_dense_): its shared memory, and the
+  // launch with as many warps as leave room for two blocks per SM (any other
+  // index: the launch itself); the shared memory of the kernel that runs.
+  size_t findere_smem_bytes(const QueryLaunch& l) const;
+  QueryLaunch run_launch(const QueryLaunch& l) const;
+  size_t launch_smem_bytes(const QueryLaunch& l) const;
   int max_blocks(const QueryLaunch& l) const;
   // Bytes of fingerprint planes gathered per seed, summed over classes.
   uint64_t gather_bytes_per_seed() const;
@@ -335,6 +341,7 @@ class Engine {
   DevIndex* d_ix_norec_ = nullptr;  // recovery disabled
   ColorLoc* d_color_loc_ = nullptr;  // colour -> class, member, group (wide probe)
   OrderKey order_;
+  bool findere_dense_ = false;  // kernels/findere.cuh runs this index's queries
   bool block_order_ = false;  // buckets fit a block's shared memory (kernels/key_order.cuh)
   WinSlice* d_win_slices_ = nullptr;  // none: no window probe for this index
   uint32_t win_slices_ = 0, win_weights_ = 0;

@@ -143,6 +143,7 @@ struct BatchView {
   const uint64_t* prekeys;
   const uint32_t* prekey_count;
   uint32_t prekey_stride;
+  const struct ColorLoc* color_loc;  // findere: colour -> class, group (findere.cuh)
 };
 
 // Shared memory of the fused kernel, in order: DevIndex copy, counters,

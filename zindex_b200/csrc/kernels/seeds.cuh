@@ -218,7 +218,7 @@ __device__ __forceinline__ uint64_t short_canonical(const PackedView& pv, uint64
   return f < c ? f : c;
 }
 
-// Canonical k-mers (k <= 32) of the nw <= 256 windows from global base p, whose
+// Canonical k-mers (k <= 32) of the nw <= 512 windows from global base p, whose
 // bases are all A/C/G/T, in window order: lane l takes the windows l * per ..
 // of per = ceil(nw / 32) and rolls them (a window's value from its
 // neighbour's costs a third of cutting it out of the packed words). Window i
@@ -232,7 +232,7 @@ __device__ __forceinline__ void tile_kmers_run(const PackedView& pv, uint64_t p,
   uint64_t* out = buf + a + pad * (uint32_t)lane;
   const uint64_t mask = k == 32 ? ~0ull : (1ull << (2 * k)) - 1;
   uint64_t f = pv.fwd(p + a, k), r = revcomp(f, k);
-  // The bases after the first window (at most 7 are used).
+  // The bases after the first window (at most 15 are used).
   uint64_t next = n > 1 ? pv.bits32(p + a + k) : 0;
   out[0] = f < r ? f : r;
   for (uint32_t j = 1; j < n; ++j) {
@@ -352,23 +352,29 @@ __device__ __forceinline__ uint32_t tile_kmers_long(const PackedView& pv, const 
 // of valid[i / 32] set when its s bases are all A/C/G/T (scan_canonical_kmers
 // per ACGT run, lib.rs:645-731, as findere scans them, findere.rs:178-233).
 // k > 32 uses the polynomial hash, each lane rolling over a contiguous range.
-__device__ __forceinline__ void tile_smers(const PackedView& pv, uint64_t rb, uint32_t w0,
+// True when it found every position valid without testing each.
+__device__ __forceinline__ bool tile_smers(const PackedView& pv, uint64_t rb, uint32_t w0,
                                            uint32_t npos, int s, const LongKmerConsts& lk,
                                            uint64_t* keys, uint32_t* valid, int lane) {
   if (s <= 32) {
+    const uint64_t p = rb + w0;
+    if (warp_valid(pv, p, npos + (uint32_t)s - 1, lane)) {
+      tile_kmers_run(pv, p, npos, s, keys, 0, lane);
+      for (uint32_t w = lane; w < (npos + 31) / 32; w += 32)
+        valid[w] = npos - w * 32 >= 32 ? ~0u : (1u << (npos - w * 32)) - 1u;
+      __syncwarp();
+      return true;
+    }
     for (uint32_t i0 = 0; i0 < npos; i0 += 32) {
-      const uint32_t i = i0 + lane;
-      bool ok = false;
-      if (i < npos) {
-        const uint64_t p = rb + w0 + i;
-        ok = pv.valid(p, s);
-        if (ok) keys[i] = canonical_at(pv, p, s);
-      }
+      const uint32_t n = min(32u, npos - i0);
+      const bool ok = short_valid(pv, p + i0, n, s, lane);
+      const uint64_t key = short_canonical(pv, p + i0, n, s, lane);
+      if (ok) keys[i0 + lane] = key;
       const uint32_t bits = __ballot_sync(0xFFFFFFFFu, ok);
       if (lane == 0) valid[i0 >> 5] = bits;
     }
     __syncwarp();
-    return;
+    return false;
   }
   for (uint32_t w = lane; w < (npos + 31) / 32; w += 32) valid[w] = 0;
   __syncwarp();
@@ -403,6 +409,7 @@ __device__ __forceinline__ void tile_smers(const PackedView& pv, uint64_t rb, ui
     atomicOr(valid + (i >> 5), 1u << (i & 31));
   }
   __syncwarp();
+  return false;
 }
 
 // ---- open-closed mod-minimizers -------------------------------------------

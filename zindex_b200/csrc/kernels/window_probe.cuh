@@ -84,6 +84,22 @@ __device__ __forceinline__ uint32_t maj(uint32_t a, uint32_t b, uint32_t c) {
   return (a & b) | (c & (a | b));
 }
 
+// Adds four flags words to the planes: a carry-save adder for the first two
+// planes, half adders for the carry.
+__device__ __forceinline__ void plane_add4(uint32_t (&planes)[kWinPlanes], const uint32_t (&d)[4]) {
+  const uint32_t t = planes[0] ^ d[0] ^ d[1], c0 = maj(planes[0], d[0], d[1]);
+  const uint32_t c1 = maj(t, d[2], d[3]);
+  planes[0] = t ^ d[2] ^ d[3];
+  uint32_t m = maj(planes[1], c0, c1);
+  planes[1] ^= c0 ^ c1;
+#pragma unroll
+  for (int k = 2; k < kWinPlanes; ++k) {
+    const uint32_t x = planes[k] & m;
+    planes[k] ^= m;
+    m = x;
+  }
+}
+
 // One block's run [pos, stop) of a slice's sorted seeds. HT: the hash count (0:
 // any, rows folded four at a time); LW: log2 of the slice's width, so that a
 // team's strides are constants.
@@ -273,18 +289,7 @@ __device__ __forceinline__ void window_slice(const DevIndex* __restrict__ ix, co
             d[s] &= ~multi;
           }
         }
-        // Carry-save: four flags words into the planes.
-        const uint32_t t = planes[0] ^ d[0] ^ d[1], c0 = maj(planes[0], d[0], d[1]);
-        const uint32_t c1 = maj(t, d[2], d[3]);
-        planes[0] = t ^ d[2] ^ d[3];
-        uint32_t m = maj(planes[1], c0, c1);
-        planes[1] ^= c0 ^ c1;
-#pragma unroll
-        for (int k = 2; k < kWinPlanes; ++k) {
-          const uint32_t x = planes[k] & m;
-          planes[k] ^= m;
-          m = x;
-        }
+        plane_add4(planes, d);
       }
       __syncwarp();
     }
