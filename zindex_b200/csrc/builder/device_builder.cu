@@ -112,7 +112,7 @@ __global__ void extract_region_kernel(BatchView bv, SeedParams sp,
                                       unsigned long long* __restrict__ cursor,
                                       uint64_t* __restrict__ out, int warps_per_block) {
   extern __shared__ __align__(16) uint8_t smem[];
-  uint16_t* inner = reinterpret_cast<uint16_t*>(smem);
+  uint8_t* inner = smem;
   uint8_t* p = smem + 256 * 8;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint8_t* wbase = p + (size_t)warp * FusedSmem::warp_bytes(MODE, sp.k, 0, 0, 0, 4, 0, 0, false);

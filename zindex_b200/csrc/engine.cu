@@ -174,13 +174,14 @@ WideFn wide_fn(int J, int HQ, int T) {
 }
 
 // Window probe by hash count: exact unrolls of the common ones.
+template <bool B16>
 WindowFn window_fn(int hashes) {
   switch (hashes) {
-    case 2: return window_probe_kernel<2>;
-    case 3: return window_probe_kernel<3>;
-    case 4: return window_probe_kernel<4>;
-    case 8: return window_probe_kernel<8>;
-    default: return window_probe_kernel<0>;
+    case 2: return window_probe_kernel<2, B16>;
+    case 3: return window_probe_kernel<3, B16>;
+    case 4: return window_probe_kernel<4, B16>;
+    case 8: return window_probe_kernel<8, B16>;
+    default: return window_probe_kernel<0, B16>;
   }
 }
 
@@ -1005,6 +1006,9 @@ void Engine::plan_windows() {
   cuda_check(cudaMemcpy(d_win_slices_, slices.data(), slices.size() * sizeof(WinSlice),
                         cudaMemcpyHostToDevice),
              "upload");
+  win_b16_ = m_.fingerprint_bits == 16;
+  for (const auto& cls : m_.classes)
+    for (const GroupMeta& g : m_.banks[cls[0]].groups) win_b16_ &= g.members.size() == 1;
   win_slices_ = (uint32_t)slices.size();
   win_weights_ = weights;
   // Windows pay once a round's row reads are a few times the rows copied.
@@ -1577,12 +1581,19 @@ void Engine::run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv,
   cuda_check(cudaFuncSetAttribute(wfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
              "cudaFuncSetAttribute");
   const int ewarps = 4;
-  const size_t esmem = DenseSmem::total(sp_.mode, sp_.k, ewarps);
+  const size_t esmem = DenseSmem::total(sp_.mode, sp_, ewarps);
   DenseExtractFn efn = dense_extract_for(sp_.mode);
   cuda_check(cudaFuncSetAttribute(efn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)esmem),
              "cudaFuncSetAttribute");
-  const int egrid = (int)std::min<uint64_t>((kSplitTiles + ewarps - 1) / ewarps,
-                                            (uint64_t)sms_ * 8);
+  // As many blocks as are resident at once: the tiles are dealt out in equal
+  // shares, and a second wave of a third of the blocks doubled the time.
+  if (!extract_per_sm_) {
+    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&extract_per_sm_, efn, ewarps * 32, esmem),
+               "occupancy");
+    extract_per_sm_ = std::max(1, extract_per_sm_);
+  }
+  const int egrid = (int)std::min<uint64_t>(std::max<uint64_t>((tiles_bound + ewarps - 1) / ewarps, 1),
+                                            (uint64_t)sms_ * extract_per_sm_);
   // A tile holds at most 256 seeds: one probe round.
   const int wblocks = l.blocks > 0 ? std::min(l.blocks, blocks_cap)
                                    : (int)std::min<uint64_t>(blocks_cap, std::max<uint64_t>(tiles_bound, 1));
@@ -1713,7 +1724,7 @@ void Engine::run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv,
                                             segments ? nullptr : total, sg);
     cuda_check(cudaGetLastError(), "wide_probe_kernel");
     if (windows) {
-      WindowFn winfn = window_fn(m_.hashes);
+      WindowFn winfn = win_b16_ ? window_fn<true>(m_.hashes) : window_fn<false>(m_.hashes);
       cuda_check(cudaFuncSetAttribute(winfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)kWinBlockBytes),
                  "cudaFuncSetAttribute");

@@ -345,6 +345,7 @@ class Engine {
   bool block_order_ = false;  // buckets fit a block's shared memory (kernels/key_order.cuh)
   WinSlice* d_win_slices_ = nullptr;  // none: no window probe for this index
   uint32_t win_slices_ = 0, win_weights_ = 0;
+  bool win_b16_ = false;  // 16-bit fields of single-member groups
   uint64_t win_min_keys_ = ~0ull;
   std::vector<void*> allocations_;
   uint64_t resident_bytes_ = 0;
@@ -353,6 +354,7 @@ class Engine {
   bool timing_ = false;
   cudaEvent_t ev_begin_ = nullptr, ev_end_ = nullptr;
   int cached_blocks_ = 0;
+  int extract_per_sm_ = 0;  // resident blocks of the dense extraction
   int noalloc_slot_ = -1;  // error word of the allocation-free query, once used
   double load_s_ = 0, banks_load_s_ = 0, recovery_load_s_ = 0;
   QueryLaunch cached_for_{};

@@ -220,7 +220,7 @@ struct FusedSmem {
 template <int MODE>
 __device__ __forceinline__ uint32_t extract_tile(const BatchView& bv, const SeedParams& sp,
                                                  const Tile& t, uint64_t* keys, uint8_t* ocm,
-                                                 const uint16_t* inner, int lane,
+                                                 const uint8_t* inner, int lane,
                                                  const uint64_t* quads = nullptr) {
   const uint64_t rb = bv.offsets[t.record];
   uint32_t n;
@@ -256,10 +256,10 @@ __device__ __forceinline__ void load_index_smem(const DevIndex* __restrict__ gix
 }
 
 // Ranks of the s-mers' inner hashes (equal hashes share a rank; only their
-// order matters to open-closed minimizers), 2 bytes each, in a 256 x 8 byte
+// order matters to open-closed minimizers), a byte each, in a 256 x 8 byte
 // table that holds the hashes meanwhile. All threads of the block (at least a
 // warp) take part.
-__device__ __forceinline__ void build_inner_table(const SeedParams& sp, uint16_t* inner) {
+__device__ __forceinline__ void build_inner_table(const SeedParams& sp, uint8_t* inner) {
   if (sp.mode != 1) return;
   uint64_t* hash = reinterpret_cast<uint64_t*>(inner);
   const int s = sp.ocm.s;
@@ -279,7 +279,7 @@ __device__ __forceinline__ void build_inner_table(const SeedParams& sp, uint16_t
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
     const uint32_t v = threadIdx.x + u * blockDim.x;
-    if (v < n) inner[v] = (uint16_t)rank[u];
+    if (v < n) inner[v] = (uint8_t)rank[u];
   }
 }
 
@@ -304,9 +304,9 @@ __global__ void __launch_bounds__(256, MINB) fused_query_kernel(const DevIndex* 
     scount = reinterpret_cast<uint32_t*>(p);
     p += FusedSmem::counter_bytes(colors, 1);
   }
-  uint16_t* inner = nullptr;
+  uint8_t* inner = nullptr;
   if (MODE == 1) {
-    inner = reinterpret_cast<uint16_t*>(p);
+    inner = p;
     p += 256 * 8;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -482,7 +482,7 @@ template <int MODE>
 __global__ void extract_kernel(BatchView bv, SeedParams sp, uint64_t* __restrict__ out,
                                uint32_t* __restrict__ out_count, int warps_per_block) {
   extern __shared__ __align__(16) uint8_t smem[];
-  uint16_t* inner = reinterpret_cast<uint16_t*>(smem);
+  uint8_t* inner = smem;
   uint8_t* p = smem + 256 * 8;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint8_t* wbase = p + (size_t)warp * FusedSmem::warp_bytes(MODE, sp.k, 0, 0, 0, 4, 0, 0,

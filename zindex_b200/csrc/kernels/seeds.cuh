@@ -440,7 +440,7 @@ constexpr uint32_t kOcmTile = 256;  // windows per minimizer tile
 // 4^s-entry table of inner hash ranks; pos holds nw + 1 entries. This form
 // takes windows of any span; tile_ocm_select_wide the usual ones.
 __device__ void tile_ocm_select_any(const PackedView& pv, uint64_t rb, uint32_t w0, uint32_t nw,
-                                const SeedParams& sp, const uint16_t* inner, Rank16* pre,
+                                const SeedParams& sp, const uint8_t* inner, Rank16* pre,
                                 Rank16* suf, uint32_t* pos, int lane) {
   const int k = sp.k, t = sp.ocm.t, s = sp.ocm.s, w = sp.ocm.w;
   const uint32_t W = (uint32_t)(k - t + 1);
@@ -508,17 +508,77 @@ struct OcmRank {
 
 // a lies left of b; equal ranks keep the leftmost and rightmost positions.
 __device__ __forceinline__ OcmRank ocm_min(const OcmRank& a, const OcmRank& b) {
-  OcmRank r;
-  const bool less = b.k < a.k || (b.k == a.k && (b.p >> 30) < (a.p >> 30));
-  r.k = less ? b.k : a.k;
-  r.p = less ? b.p : a.p;
-  if (a.k == b.k && (a.p >> 30) == (b.p >> 30)) r.p = (a.p & ~0x7FFFu) | (b.p & 0x7FFFu);
+  const bool less = b.k < a.k;
+  OcmRank r{less ? b.k : a.k, less ? b.p : a.p};
+  if (a.k == b.k) {  // (seldom: the same t-mer twice)
+    const uint32_t x = a.p >> 30, y = b.p >> 30;
+    r.p = y < x ? b.p : (x < y ? a.p : (a.p & ~0x7FFFu) | (b.p & 0x7FFFu));
+  }
   return r;
 }
 
 // Anchors of a lane in tile_ocm_select_wide.
 __device__ __forceinline__ uint32_t ocm_per_lane(uint32_t nw, uint32_t W) {
   return (nw + W + 31) / 32;
+}
+
+// The ranks of a lane's anchors skip .. n - 1 (the first at base p) and their
+// running minima for t <= 16 and LAST = t - s in 4 .. 8, by rolling: the t-mer
+// and its reverse complement, and the inner ranks' sliding minimum from
+// minima of 2 and 4 that byte registers hold back (last eight ranks in `old`,
+// two and four minima in `two` and `four`). Returns the minimum of all.
+template <int LAST>
+__device__ __forceinline__ OcmRank ocm_ranks(const PackedView& pv, uint64_t p, uint32_t skip,
+                                             uint32_t n, uint32_t a0, const SeedParams& sp,
+                                             const uint8_t* inner, uint64_t* sk, uint32_t* sp_,
+                                             uint64_t* pk, uint32_t* pp) {
+  static_assert(LAST >= 4 && LAST <= 8 && LAST % 2 == 0, "inner positions of an anchor");
+  constexpr int kBack = LAST - 3 < 4 ? LAST - 3 : 4;  // the second minimum of four, so far back
+  const int t = sp.ocm.t, s = sp.ocm.s;
+  const uint32_t tmask = t == 16 ? ~0u : (1u << (2 * t)) - 1u, smask = (1u << (2 * s)) - 1u;
+  uint64_t v = pv.bits32(p);  // (an anchor's bases: at most 17 + 15)
+  uint32_t f = 0, r = 0, two = 0, four = 0;
+  uint64_t old = 0;
+  auto base = [&]() {
+    const uint32_t c = (uint32_t)(v >> 62);
+    v <<= 2;
+    f = ((f << 2) | c) & tmask;
+    r = (r >> 2) | ((3u - c) << (2 * t - 2));
+  };
+  for (int i = 0; i < s - 1; ++i) base();
+  uint32_t h0 = 0, hm = 0, hl = 0, lo = 0;
+  auto slide = [&]() {
+    base();
+    hl = inner[f & smask];
+    const uint32_t m2 = min(hl, (uint32_t)old & 0xFFu);
+    const uint32_t m4 = min(m2, (two >> 8) & 0xFFu);
+    h0 = (uint32_t)(old >> (8 * (LAST - 1))) & 0xFFu;
+    hm = (uint32_t)(old >> (8 * (LAST / 2 - 1))) & 0xFFu;
+    lo = min(min(m4, (four >> (8 * (kBack - 1))) & 0xFFu), h0);
+    old = (old << 8) | hl;
+    two = (two << 8) | m2;
+    four = (four << 8) | m4;
+  };
+#pragma unroll
+  for (int i = 0; i < LAST; ++i) slide();
+  OcmRank run{~0ull, 0};
+  for (uint32_t j = 0; j < n; ++j) {
+    OcmRank rk{~0ull, 3u << 30};
+    if (j >= skip) {
+      slide();
+      const uint32_t cls = hm == lo ? 0u : (h0 == lo || hl == lo ? 1u : 2u);
+      const uint64_t hash = mixsplit((uint64_t)min(f, r), sp.seed);
+      rk.k = ((uint64_t)cls << 62) | (hash >> 2);
+      rk.p = (uint32_t)hash << 30;
+    }
+    rk.p |= (a0 + j) * 0x8001u;
+    run = j ? ocm_min(run, rk) : rk;
+    sk[j] = rk.k;
+    sp_[j] = rk.p;
+    pk[j] = run.k;
+    pp[j] = run.p;
+  }
+  return run;
 }
 
 // tile_ocm_select for windows of more than per = ocm_per_lane(nw, W) anchors:
@@ -531,7 +591,7 @@ __device__ __forceinline__ uint32_t ocm_per_lane(uint32_t nw, uint32_t W) {
 // tile_ocm_select_any has it, left most of the warp idle: 3.6 ms for 2^18 tiles
 // of 2,048-colour minimizer windows on a B200.)
 __device__ void tile_ocm_select_wide(const PackedView& pv, uint64_t rb, uint32_t w0, uint32_t nw,
-                                     const SeedParams& sp, const uint16_t* inner, uint8_t* scratch,
+                                     const SeedParams& sp, const uint8_t* inner, uint8_t* scratch,
                                      uint32_t* pos, int lane) {
   constexpr uint32_t kFull = 0xFFFFFFFFu;
   const int k = sp.k, t = sp.ocm.t, s = sp.ocm.s, w = sp.ocm.w;
@@ -549,9 +609,15 @@ __device__ void tile_ocm_select_wide(const PackedView& pv, uint64_t rb, uint32_t
   const uint32_t smask = (1u << (2 * s)) - 1;
   const int last = t - s;
   OcmRank run{~0ull, 0};
+  const bool fast = t <= 16 && last >= 4 && last <= 8;
+  if (fast && n > skip) {
+    if (last == 8) run = ocm_ranks<8>(pv, p, skip, n, a0, sp, inner, sk + at, sp_ + at, pk + at, pp + at);
+    else if (last == 6) run = ocm_ranks<6>(pv, p, skip, n, a0, sp, inner, sk + at, sp_ + at, pk + at, pp + at);
+    else run = ocm_ranks<4>(pv, p, skip, n, a0, sp, inner, sk + at, sp_ + at, pk + at, pp + at);
+  }
   uint64_t v = 0;
   int have = 0;  // bases left in v
-  for (uint32_t j = 0; j < n; ++j) {
+  for (uint32_t j = fast && n > skip ? n : 0; j < n; ++j) {
     OcmRank rk{~0ull, 3u << 30};  // no anchor: above every rank of a window
     if (j >= skip) {
       if (have < t) {
@@ -562,23 +628,12 @@ __device__ void tile_ocm_select_wide(const PackedView& pv, uint64_t rb, uint32_t
       v <<= 2;
       --have;
       uint32_t lo = ~0u, h0 = 0, hm = 0, hl = 0;
-      if (t <= 16) {
-        const uint32_t x = (uint32_t)tf;
-        for (int q = 0; q <= last; ++q) {
-          const uint32_t h = inner[(x >> (2 * (last - q))) & smask];
-          lo = min(lo, h);
-          if (q == 0) h0 = h;
-          if (q == last / 2) hm = h;
-          hl = h;
-        }
-      } else {
-        for (int q = 0; q <= last; ++q) {
-          const uint32_t h = inner[(uint32_t)(tf >> (2 * (last - q))) & smask];
-          lo = min(lo, h);
-          if (q == 0) h0 = h;
-          if (q == last / 2) hm = h;
-          hl = h;
-        }
+      for (int q = 0; q <= last; ++q) {
+        const uint32_t h = inner[(uint32_t)(tf >> (2 * (last - q))) & smask];
+        lo = min(lo, h);
+        if (q == 0) h0 = h;
+        if (q == last / 2) hm = h;
+        hl = h;
       }
       const uint64_t cls = hm == lo ? 0 : (h0 == lo || hl == lo ? 1 : 2);
       const uint64_t tr = revcomp(tf, t);
@@ -646,7 +701,7 @@ __device__ void tile_ocm_select_wide(const PackedView& pv, uint64_t rb, uint32_t
 // buffer.
 __device__ __forceinline__ void tile_ocm_select(const PackedView& pv, uint64_t rb, uint32_t w0,
                                                 uint32_t nw, const SeedParams& sp,
-                                                const uint16_t* inner, Rank16* pre, Rank16* suf,
+                                                const uint8_t* inner, Rank16* pre, Rank16* suf,
                                                 uint32_t* pos, int lane) {
   const uint32_t W = (uint32_t)(sp.k - sp.ocm.t + 1);
   if (W > ocm_per_lane(nw, W))
@@ -655,14 +710,13 @@ __device__ __forceinline__ void tile_ocm_select(const PackedView& pv, uint64_t r
     tile_ocm_select_any(pv, rb, w0, nw, sp, inner, pre, suf, pos, lane);
 }
 
-// Minimizers of windows [w0, w0+nw) (nw <= kOcmTile), buffers as for
-// tile_ocm_select. Emits in window order, dropping repeats of the previous
-// window's selected position within a run.
-__device__ uint32_t tile_ocm(const PackedView& pv, uint64_t rb, uint32_t w0, uint32_t nw,
-                             const SeedParams& sp, const uint16_t* inner, Rank16* pre,
-                             Rank16* suf, uint32_t* pos, uint64_t* buf, int lane) {
+// The positions (as pos[]) that the windows [w0, w0+nw) emit, in window order,
+// into the uint32 list at pre; returns their number.
+__device__ __forceinline__ uint32_t tile_ocm_list(const PackedView& pv, uint64_t rb, uint32_t w0,
+                                                  uint32_t nw, const SeedParams& sp,
+                                                  const uint8_t* inner, Rank16* pre, Rank16* suf,
+                                                  uint32_t* pos, int lane) {
   tile_ocm_select(pv, rb, w0, nw, sp, inner, pre, suf, pos, lane);
-  // The positions to emit first (about one window in ten), then their keys.
   uint32_t* list = reinterpret_cast<uint32_t*>(pre);
   uint32_t count = 0;
   for (uint32_t i0 = 1; i0 <= nw; i0 += 32) {
@@ -674,6 +728,17 @@ __device__ uint32_t tile_ocm(const PackedView& pv, uint64_t rb, uint32_t w0, uin
     count += __popc(ballot);
   }
   __syncwarp();
+  return count;
+}
+
+// Minimizers of windows [w0, w0+nw) (nw <= kOcmTile), buffers as for
+// tile_ocm_select. Emits in window order, dropping repeats of the previous
+// window's selected position within a run.
+__device__ uint32_t tile_ocm(const PackedView& pv, uint64_t rb, uint32_t w0, uint32_t nw,
+                             const SeedParams& sp, const uint8_t* inner, Rank16* pre,
+                             Rank16* suf, uint32_t* pos, uint64_t* buf, int lane) {
+  const uint32_t count = tile_ocm_list(pv, rb, w0, nw, sp, inner, pre, suf, pos, lane);
+  const uint32_t* list = reinterpret_cast<const uint32_t*>(pre);
   for (uint32_t i = lane; i < count; i += 32)
     buf[i] = canonical_at(pv, rb + w0 - 1 + list[i], sp.m);
   __syncwarp();

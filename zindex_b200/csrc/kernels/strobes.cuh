@@ -63,10 +63,10 @@ __global__ void strobe_anchor_kernel(BatchView bv, SeedParams sp, uint32_t* __re
                                      uint64_t* __restrict__ hashes, int warps_per_block) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint16_t* inner = nullptr;
+  uint8_t* inner = nullptr;
   uint8_t* wbase = smem;
   if (MODE == 1) {
-    inner = reinterpret_cast<uint16_t*>(smem);
+    inner = smem;
     wbase = smem + 256 * 8 + (size_t)warp * StrobeSmem::warp_bytes(1, sp.k);
     build_inner_table(sp, inner);
     __syncthreads();

@@ -55,9 +55,18 @@ struct ColorLoc {
 // staging of long k-mer hashes) and, for minimizers, the open-closed
 // minimizer scratch; no probe descriptors. The block adds a table.
 struct DenseSmem {
-  static __host__ __device__ size_t warp_bytes(int mode, int k) {
-    size_t b = FusedSmem::key_bytes(mode, k, false) + 32 * 8;  // (padded runs: extract_short)
-    if (mode == 1) b += 2 * FusedSmem::ocm_entries(k) * sizeof(Rank16) + (kTileWindows + 1) * 4 + 16;
+  // k-mers of k <= 32, and minimizers that are every m-mer (extract_short).
+  static __host__ __device__ bool is_short(int mode, const SeedParams& sp) {
+    return (mode == 0 && sp.klen <= 32) || (mode == 1 && sp.k == sp.m);
+  }
+  static __host__ __device__ size_t ocm_scratch(const SeedParams& sp) {
+    const uint32_t W = (uint32_t)(sp.k - sp.ocm.t + 1), per = (kTileWindows + W + 31) / 32;
+    return W > per ? (size_t)24 * 32 * (per | 1) : (size_t)2 * sizeof(Rank16) * (kTileWindows + W);
+  }
+  static __host__ __device__ size_t warp_bytes(int mode, const SeedParams& sp) {
+    size_t b;
+    if (mode == 1 && !is_short(mode, sp)) b = ocm_scratch(sp) + (kTileWindows + 1) * 4;
+    else b = FusedSmem::key_bytes(mode, sp.k, false) + (is_short(mode, sp) ? 32 * 8 : 0);  // (padded runs)
     return (b + 15) / 16 * 16;
   }
   // The block's table: the ranks of inner hashes (minimizers), or the terms
@@ -65,8 +74,8 @@ struct DenseSmem {
   static __host__ __device__ size_t table_bytes(int mode, int k) {
     return mode != 1 && k > 32 ? 512 * 8 : 256 * 8;
   }
-  static __host__ __device__ size_t total(int mode, int k, int warps) {
-    return table_bytes(mode, k) + (size_t)warps * warp_bytes(mode, k);
+  static __host__ __device__ size_t total(int mode, const SeedParams& sp, int warps) {
+    return table_bytes(mode, sp.k) + (size_t)warps * warp_bytes(mode, sp);
   }
 };
 
@@ -253,18 +262,17 @@ __global__ void extract_dense_kernel(BatchView bv, SeedParams sp, uint64_t* __re
                                      unsigned long long* __restrict__ cursor, int warps_per_block,
                                      WideRound sg) {
   extern __shared__ __align__(16) uint8_t smem[];
-  uint16_t* inner = reinterpret_cast<uint16_t*>(smem);
+  uint8_t* inner = smem;
   uint8_t* p = smem + DenseSmem::table_bytes(MODE, sp.k);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (MODE == 0 && sp.klen <= 32) {
+  if (DenseSmem::is_short(MODE, sp)) {
     extract_short(bv, sp, out, cursor, blockIdx.x * warps_per_block + warp,
                   gridDim.x * warps_per_block, lane,
-                  reinterpret_cast<uint64_t*>(p + (size_t)warp * DenseSmem::warp_bytes(0, sp.k)), sg);
+                  reinterpret_cast<uint64_t*>(p + (size_t)warp * DenseSmem::warp_bytes(MODE, sp)), sg);
     return;
   }
-  uint8_t* wbase = p + (size_t)warp * DenseSmem::warp_bytes(MODE, sp.k);
+  uint8_t* wbase = p + (size_t)warp * DenseSmem::warp_bytes(MODE, sp);
   uint64_t* keys = reinterpret_cast<uint64_t*>(wbase);
-  uint8_t* ocm = wbase + FusedSmem::key_bytes(MODE, sp.k, false);
   const uint64_t* quads = nullptr;
   if (MODE != 1 && sp.klen > 32) {
     build_long_table(reinterpret_cast<uint64_t*>(smem));
@@ -277,7 +285,18 @@ __global__ void extract_dense_kernel(BatchView bv, SeedParams sp, uint64_t* __re
   const uint32_t warps_total = gridDim.x * warps_per_block;
   for (uint32_t t = bv.tile_lo + blockIdx.x * warps_per_block + warp; t < ntiles;
        t += warps_total) {
-    uint32_t n = extract_tile<MODE>(bv, sp, bv.tiles[t], keys, ocm, inner, lane, quads);
+    uint32_t n;
+    uint64_t first = 0;  // minimizers: the base that the listed positions count from
+    if constexpr (MODE == 1) {
+      const Tile tile = bv.tiles[t];
+      const uint64_t rb = bv.offsets[tile.record];
+      Rank16* pre = reinterpret_cast<Rank16*>(wbase);
+      first = rb + tile.w0 - 1;
+      n = tile_ocm_list(bv.pv, rb, tile.w0, tile.nw, sp, inner, pre, pre + (kTileWindows + sp.k - sp.ocm.t + 1),
+                        reinterpret_cast<uint32_t*>(wbase + DenseSmem::ocm_scratch(sp)), lane);
+    } else {
+      n = extract_tile<MODE>(bv, sp, bv.tiles[t], keys, nullptr, inner, lane, quads);
+    }
     __syncwarp();
     unsigned long long at = 0;
     uint64_t* dst = out;
@@ -296,7 +315,15 @@ __global__ void extract_dense_kernel(BatchView bv, SeedParams sp, uint64_t* __re
       }
       n = 0;
     }
-    for (uint32_t i = lane; i < n; i += 32) dst[at + i] = keys[i];
+    if constexpr (MODE == 1) {
+      const uint32_t* list = reinterpret_cast<const uint32_t*>(wbase);
+      for (uint32_t i = lane; i < n; i += 32) {
+        const uint64_t key = canonical_at(bv.pv, first + list[i], sp.m);
+        dst[at + i] = sp.spaced ? spaced_canonical(sp.pattern, key) : key;
+      }
+    } else {
+      for (uint32_t i = lane; i < n; i += 32) dst[at + i] = keys[i];
+    }
     __syncwarp();
   }
 }

@@ -102,8 +102,11 @@ __device__ __forceinline__ void plane_add4(uint32_t (&planes)[kWinPlanes], const
 
 // One block's run [pos, stop) of a slice's sorted seeds. HT: the hash count (0:
 // any, rows folded four at a time); LW: log2 of the slice's width, so that a
-// team's strides are constants.
-template <int HT, int LW>
+// team's strides are constants. B16: 16-bit fields and no multi-member group;
+// the fields that differ are then counted as they are, two to a register (a
+// two-way minimum with 1 and an add per word instead of the 5.5 logic
+// operations of flags and planes).
+template <int HT, int LW, bool B16>
 __device__ __forceinline__ void window_slice(const DevIndex* __restrict__ ix, const WinSlice& S,
                                              const OrderKey& order, uint64_t pos, uint64_t stop,
                                              const uint64_t* __restrict__ keys,
@@ -111,7 +114,7 @@ __device__ __forceinline__ void window_slice(const DevIndex* __restrict__ ix, co
                                              uint8_t* smem, uint64_t* __restrict__ counts) {
   constexpr uint32_t w = 1u << LW, nteams = 32u >> LW, row_bytes = w * 16u;
   constexpr int kStep = w < 4 ? (int)w : 4;  // seeds of a team at a time
-  const int H = HT ? HT : ix->hashes, b = ix->bits, lb = log2_bits(b);
+  const int H = HT ? HT : ix->hashes, b = B16 ? 16 : ix->bits, lb = log2_bits(b);
   const uint32_t Hp = WinSmem::rows_per_seed(H), tile_bytes = WinSmem::tile_bytes(H);
   const int warp = threadIdx.x >> 5;
   const uint32_t lane = threadIdx.x & 31u, tl = lane & (w - 1), team = lane >> LW;
@@ -148,8 +151,23 @@ __device__ __forceinline__ void window_slice(const DevIndex* __restrict__ ix, co
   uint32_t planes[kWinPlanes];
 #pragma unroll
   for (int k = 0; k < kWinPlanes; ++k) planes[k] = 0;
-  uint32_t counted = 0;  // seeds in the planes (the warp's bound)
+  uint32_t differ[4] = {0, 0, 0, 0};  // B16: per word, the seeds that each half differed from
+  uint32_t counted = 0;               // seeds in the planes (the warp's bound)
+  constexpr uint32_t kCounts = B16 ? 65535u : 255u;
   auto flush = [&]() {
+    if constexpr (B16) {
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) {
+#pragma unroll
+        for (uint32_t f = 0; f < 2; ++f) {
+          const uint32_t same = counted - ((differ[q] >> (16 * f)) & 0xFFFFu);
+          if (same && ((valid >> (16 * f + q)) & 1u)) atomicAdd(scount + (2 * q + f) * 32u + lane, same);
+        }
+        differ[q] = 0;
+      }
+      counted = 0;
+      return;
+    }
     uint32_t any = 0;
 #pragma unroll
     for (int k = 0; k < kWinPlanes; ++k) any |= planes[k];
@@ -230,7 +248,7 @@ __device__ __forceinline__ void window_slice(const DevIndex* __restrict__ ix, co
       }
       g = take();
       key = g + lane < nseeds ? __ldg(keys + pos + g + lane) : 0;
-      if (counted + w > 255u) flush();
+      if (counted + w > kCounts) flush();
       counted += w;
       __syncwarp();
 #pragma unroll 1
@@ -257,11 +275,18 @@ __device__ __forceinline__ void window_slice(const DevIndex* __restrict__ ix, co
             }
           }
           const uint32_t x[4] = {acc.x, acc.y, acc.z, acc.w};
+          if constexpr (B16) {
+            const uint32_t dead = n < 32 && sd >= n ? ~0u : 0u;  // past the last seed: all differ
+#pragma unroll
+            for (int q = 0; q < 4; ++q) differ[q] += __vminu2(x[q] | dead, 0x00010001u);
+            continue;
+          }
           uint32_t m = 0;
 #pragma unroll
           for (int q = 0; q < 4; ++q) m |= (~(((x[q] & lo) + lo) | x[q]) & hi) >> (uint32_t)(b - 1 - q);
           d[s] = m & valid;
         }
+        if constexpr (B16) continue;
         if (n < 32) {
 #pragma unroll
           for (int s = 0; s < kStep; ++s)
@@ -310,7 +335,7 @@ __device__ __forceinline__ void window_slice(const DevIndex* __restrict__ ix, co
   __syncthreads();
 }
 
-template <int HT>
+template <int HT, bool B16>
 __global__ void __launch_bounds__(kWinThreads, 2)
     window_probe_kernel(const DevIndex* __restrict__ ix, WinPlan plan,
                         const uint64_t* __restrict__ keys,
@@ -348,11 +373,11 @@ __global__ void __launch_bounds__(kWinThreads, 2)
       const uint64_t stop = u1 >= s_end ? nk : (u1 - s_first + S.weight - 1) / S.weight;
       if (pos >= stop) continue;
       switch (S.lw) {
-        case 4: window_slice<HT, 4>(ix, S, plan.order, pos, stop, keys, bucket_end, smem, counts); break;
-        case 3: window_slice<HT, 3>(ix, S, plan.order, pos, stop, keys, bucket_end, smem, counts); break;
-        case 2: window_slice<HT, 2>(ix, S, plan.order, pos, stop, keys, bucket_end, smem, counts); break;
-        case 1: window_slice<HT, 1>(ix, S, plan.order, pos, stop, keys, bucket_end, smem, counts); break;
-        default: window_slice<HT, 0>(ix, S, plan.order, pos, stop, keys, bucket_end, smem, counts); break;
+        case 4: window_slice<HT, 4, B16>(ix, S, plan.order, pos, stop, keys, bucket_end, smem, counts); break;
+        case 3: window_slice<HT, 3, B16>(ix, S, plan.order, pos, stop, keys, bucket_end, smem, counts); break;
+        case 2: window_slice<HT, 2, B16>(ix, S, plan.order, pos, stop, keys, bucket_end, smem, counts); break;
+        case 1: window_slice<HT, 1, B16>(ix, S, plan.order, pos, stop, keys, bucket_end, smem, counts); break;
+        default: window_slice<HT, 0, B16>(ix, S, plan.order, pos, stop, keys, bucket_end, smem, counts); break;
       }
     }
   }
