@@ -1335,7 +1335,8 @@ void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, b
     ws.cap_tiles = 0;
     ws.release_graphs();
   }
-  uint64_t tiles = ws.cap_bases / kTileWindows + ws.cap_bases / kFindereTask + ws.cap_records + 16;
+  uint64_t tiles = ws.cap_bases / kTileWindows + ws.cap_bases / kFindereTask + ws.cap_records +
+                   kSmallTiles + 16;
   if (tiles > ws.cap_tiles) {
     if (ws.tiles) cudaFree(ws.tiles);
     dev_alloc(&ws.tiles, tiles, "tiles");
@@ -1468,21 +1469,26 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   // scan and fill), and with few colours the fused kernel adds into the
   // caller's counters (no reduction launch).
   const bool dense = dense_batch(nbases) && ensure_round_capacity(ws, nbases);
-  const bool small = records <= kSmallRecords && nbases <= kSmallBases && !wide_form(l) &&
-                     kernel_mode(l) != 4;
+  const bool fused = !wide_form(l) && kernel_mode(l) != 4;
+  const bool small = records <= kSmallRecords &&
+                     nbases <= (fused ? kSmallBases : wide_form(l) ? kSmallWideBases : 0);
+  uint32_t tw = kTileWindows;
   if (small) {
+    if (fused && m_.index_mode != kFindere)
+      for (tw = 32; tw < kTileWindows && nbases / tw > kSmallTiles;) tw *= 2;
     small_plan_kernel<<<1, 1024, 0, s>>>(bases, nbases, ws.packed, ws.invalid, words, offsets,
-                                         (uint32_t)records, span(), m_.index_mode == kFindere,
-                                         ws.tile_first, ws.tiles, ws.error);
+                                         (uint32_t)records, span(), m_.index_mode == kFindere, tw,
+                                         ws.tile_first, ws.tiles, fused ? nullptr : ws.wide_cursor,
+                                         ws.error);
     cuda_check(cudaGetLastError(), "small_plan_kernel");
-    if (m_.colors.size() <= kSmallColors) l.smem_counters = 0;
+    if (fused && m_.colors.size() <= kSmallColors) l.smem_counters = 0;
   } else {
     int grid = (int)std::min<uint64_t>((words + 255) / 256, (uint64_t)sms_ * 16);
     pack_kernel<<<std::max(grid, 1), 256, 0, s>>>(bases, nbases, ws.packed, ws.invalid, words);
     cuda_check(cudaGetLastError(), "pack_kernel");
     plan_tiles(ws, offsets, records, nbases, s);
   }
-  const uint64_t tiles_bound = nbases / kTileWindows + records + nbases / kFindereTask + 1;
+  const uint64_t tiles_bound = nbases / tw + records + nbases / kFindereTask + 1;
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   cuda_check(cudaStreamIsCapturing(s, &capturing), "cudaStreamIsCapturing");
   const bool timed = timing_ && capturing == cudaStreamCaptureStatusNone;
@@ -1493,7 +1499,7 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
                        ws.fstate};
     if (timed) cuda_check(cudaEventRecord(ev_begin_, s), "cudaEventRecord");
     run_wide(ws, wide_form(l) ? l : dense_launch(), bv, tiles_bound, nbases, recover, counts, total,
-             0, s);
+             0, s, 0.0, small);
     if (timed) cuda_check(cudaEventRecord(ev_end_, s), "cudaEventRecord");
     return;
   }
@@ -1566,7 +1572,7 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
 
 void Engine::run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv,
                       uint64_t tiles_bound, uint64_t max_keys, bool recover, uint64_t* counts, unsigned long long* total, uint32_t segments,
-                      cudaStream_t s, double prune_ratio) {
+                      cudaStream_t s, double prune_ratio, bool cleared) {
   // Rounds of up to kSplitTiles tiles; per round the extraction kernel
   // appends the tiles' seeds to one dense list (segmented: each segment's
   // seeds to its own part of it), the wide probe counts them, and the block
@@ -1595,8 +1601,15 @@ void Engine::run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv,
   const int egrid = (int)std::min<uint64_t>(std::max<uint64_t>((tiles_bound + ewarps - 1) / ewarps, 1),
                                             (uint64_t)sms_ * extract_per_sm_);
   // A tile holds at most 256 seeds: one probe round.
+  // Unsegmented batches of fewer seeds than a round per block: rounds of 32
+  // seeds and more.
+  uint64_t round_seeds = kWideSeeds, probe_rounds = tiles_bound;
+  if (!segments && max_keys < (uint64_t)blocks_cap * kWideSeeds) {
+    round_seeds = std::max<uint64_t>(32, round_up((max_keys + blocks_cap - 1) / blocks_cap, 32));
+    probe_rounds = (max_keys + round_seeds - 1) / round_seeds;
+  }
   const int wblocks = l.blocks > 0 ? std::min(l.blocks, blocks_cap)
-                                   : (int)std::min<uint64_t>(blocks_cap, std::max<uint64_t>(tiles_bound, 1));
+                                   : (int)std::min<uint64_t>(blocks_cap, std::max<uint64_t>(probe_rounds, 1));
   // One round when its key lists hold every base of the batch; else rounds of
   // kSplitTiles tiles.
   const bool whole = !segments && ensure_round_capacity(ws, max_keys);
@@ -1639,13 +1652,14 @@ void Engine::run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv,
         !segments && (l.order == 2 || (l.order == 1 && (!win_slices_ || max_keys >= win_min_keys_ / 8)));
     if (ordered) ensure_order_capacity(ws, b, whole);
     sg.interleave = !segments && l.order == 2 ? 1u : 0u;
+    sg.round_seeds = (uint32_t)round_seeds;
     const bool windows = ordered && l.order == 1 && win_slices_ && max_keys >= win_min_keys_;
     if (windows) sg.max_keys = win_min_keys_;
     if (overlap && r >= 2)
       cuda_check(cudaStreamWaitEvent(xs, ws.wide_probe[b], 0), "cudaStreamWaitEvent");
     if (segments)
       cuda_check(cudaMemsetAsync(sg.cursor, 0, segments * 8ull, xs), "memset");
-    else
+    else if (!cleared || rounds > 1)
       cuda_check(cudaMemsetAsync(ws.wide_cursor + 2 * b, 0, 16, xs), "memset");
     efn<<<egrid, ewarps * 32, esmem, xs>>>(rb, sp_, keys, ws.wide_cursor + 2 * b, ewarps, sg);
     cuda_check(cudaGetLastError(), "extract_dense_kernel");

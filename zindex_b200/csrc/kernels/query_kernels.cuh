@@ -47,9 +47,11 @@ __device__ __forceinline__ uint32_t record_windows(const uint64_t* offsets, uint
   return len >= (uint64_t)span ? (uint32_t)(len - span + 1) : 0u;
 }
 
-// Tiles per record. Findere tiles never cross a 16,384-window task.
-__device__ __forceinline__ uint32_t record_tiles(uint32_t w, int findere) {
-  if (!findere) return (w + kTileWindows - 1) / kTileWindows;
+// Tiles of tw windows per record. Findere tiles (tw = kTileWindows) never
+// cross a 16,384-window task.
+__device__ __forceinline__ uint32_t record_tiles(uint32_t w, int findere,
+                                                 uint32_t tw = kTileWindows) {
+  if (!findere) return (w + tw - 1) / tw;
   const uint32_t full = w / kFindereTask, rest = w % kFindereTask;
   return full * (kFindereTask / kTileWindows) + (rest + kTileWindows - 1) / kTileWindows;
 }
@@ -79,20 +81,29 @@ __global__ void fill_tiles_kernel(const uint64_t* __restrict__ offsets, uint64_t
   }
 }
 
-// Small batches (a few thousand records, up to 1 MiB of bases): one block
-// packs the bases and plans the tiles (count, scan and fill), so the query is
-// two launches instead of six.
+// Small batches (a few thousand records, up to 1 MiB of bases; 256 KiB for the
+// wide-row form, whose kernels follow more launches anyway): one block packs
+// the bases, plans the tiles (count, scan and fill) and clears the wide-row
+// cursors, so the query is two or three launches instead of six and more.
+// The fused kernel takes the 32 seeds of a step from one tile at a time, and
+// a warp waits for memory in every step, so a small batch is cut into about
+// kSmallTiles tiles of 32 to 256 windows: 100 records of 1,000 bases took 45
+// us in 256-window tiles (eight steps a warp, most of the GPU idle).
 constexpr uint32_t kSmallRecords = 4096;
 constexpr uint64_t kSmallBases = 1ull << 20;
+constexpr uint64_t kSmallWideBases = 1ull << 18;
+constexpr uint64_t kSmallTiles = 4096;
 
 __global__ void __launch_bounds__(1024)
     small_plan_kernel(const uint8_t* __restrict__ bases, uint64_t nbases,
                       uint64_t* __restrict__ packed, uint32_t* __restrict__ invalid,
                       uint64_t words, const uint64_t* __restrict__ offsets, uint32_t records,
-                      int span, int findere, uint32_t* __restrict__ tile_first,
-                      Tile* __restrict__ tiles, uint32_t* __restrict__ err) {
+                      int span, int findere, uint32_t tw, uint32_t* __restrict__ tile_first,
+                      Tile* __restrict__ tiles, unsigned long long* __restrict__ cursor,
+                      uint32_t* __restrict__ err) {
   __shared__ uint32_t sums[1024];
   const uint32_t T = blockDim.x, tid = threadIdx.x;
+  if (cursor && tid < 2) cursor[tid] = 0;
   for (uint64_t w = tid; w < words; w += T) pack_word(bases, nbases, packed, invalid, w);
   // Each thread plans a contiguous run of records: their tile counts, a
   // block scan of the runs' sums, then the tiles.
@@ -100,7 +111,7 @@ __global__ void __launch_bounds__(1024)
   const uint32_t lo = min(records, tid * per), hi = min(records, lo + per);
   uint32_t mine = 0;
   for (uint32_t r = lo; r < hi; ++r)
-    mine += record_tiles(record_windows(offsets, r, span, nbases, err), findere);
+    mine += record_tiles(record_windows(offsets, r, span, nbases, err), findere, tw);
   sums[tid] = mine;
   __syncthreads();
   for (uint32_t off = 1; off < T; off <<= 1) {
@@ -115,7 +126,7 @@ __global__ void __launch_bounds__(1024)
     const uint32_t w = record_windows(offsets, r, span, nbases, nullptr);
     for (uint32_t w0 = 0; w0 < w;) {
       const uint32_t task = (w0 / kFindereTask) * kFindereTask;
-      const uint32_t end = min(w, min(w0 + kTileWindows, task + kFindereTask));
+      const uint32_t end = min(w, min(w0 + tw, task + kFindereTask));
       tiles[t++] = Tile{r, w0, end - w0, task};
       w0 = end;
     }

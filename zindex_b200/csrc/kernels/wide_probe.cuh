@@ -106,8 +106,11 @@ struct WideRound {
   unsigned long long* totals = nullptr;   // seeds of each segment
   uint32_t nseg = 0;
   uint32_t tile_lo = 0;                   // first tile of the extraction round
-  // Unsegmented: 1 = blocks take interleaved seeds (see the probe loop).
+  // Unsegmented: 1 = blocks take interleaved seeds (see the probe loop); seeds
+  // of a probe round (at most kWideSeeds; fewer in a small batch, so that more
+  // blocks share it).
   uint32_t interleave = 0;
+  uint32_t round_seeds = kWideSeeds;
   // Segmented per-record reports: colours reported when count / total >=
   // min_ratio (> 0 turns on threshold pruning); tile_hi ends the round.
   double min_ratio = 0.0;
@@ -660,7 +663,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
   const uint64_t mine = !inter || nk <= blockIdx.x ? 0 : (nk - blockIdx.x + G - 1) / G;
   const uint64_t nrounds = sg.nseg ? (uint64_t)__ldg(sg.round_first + sg.nseg)
                            : inter ? (mine + kWideSeeds - 1) / kWideSeeds
-                                   : (nk + kWideSeeds - 1) / kWideSeeds;
+                                   : (nk + sg.round_seeds - 1) / sg.round_seeds;
   for (uint64_t r = inter ? 0 : blockIdx.x; r < nrounds; r += inter ? 1 : G) {
     uint64_t base, kstride = 1;  // seed i of the round: keys[base + i * kstride]
     uint32_t n;
@@ -694,8 +697,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
       const uint64_t left = mine - r * kWideSeeds;
       n = left < (uint64_t)kWideSeeds ? (uint32_t)left : (uint32_t)kWideSeeds;
     } else {
-      base = r * kWideSeeds;
-      n = nk - base < (uint64_t)kWideSeeds ? (uint32_t)(nk - base) : (uint32_t)kWideSeeds;
+      base = r * sg.round_seeds;
+      n = nk - base < sg.round_seeds ? (uint32_t)(nk - base) : sg.round_seeds;
     }
     // Descriptors: pattern and row indices of each seed; recovered origins
     // the filter misses are counted by the seed's owner.
