@@ -100,3 +100,33 @@ def test_dense_batches_of_narrow_rows(gpu, oracle, tmp_path, case):
         got, total = index.query_records(bases, offsets, recover=False)
         assert total == want_total
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("colors", [300, 40])
+def test_page_locked_chunks_join_one_list(gpu, oracle, tmp_path, colors):
+    """Host batches in page-locked memory: the chunks' seeds are probed
+    together, and a record whose offsets decrease is still reported."""
+    import torch
+
+    import zindex_b200 as zx
+
+    ix, genomes = _index(tmp_path, colors=colors, H=4, b=8, k=31)
+    reads = sample_reads(genomes, np.random.default_rng(9), 24000, 150, n_runs=0.05)
+    reads += sample_reads(genomes, np.random.default_rng(10), 40, 3000)
+    bases, offsets = zx.pack_records(reads)
+    want, want_total = oracle.query_records(ix, bases, offsets)
+    locked = torch.from_numpy(bases).pin_memory().numpy()
+    with zx.Index(ix) as index:
+        for cut in (1, 2, 3, 4):
+            index.set_launch(cut=cut)
+            got, total = index.query_records(locked, offsets)
+            assert total == want_total
+            np.testing.assert_array_equal(got, want)
+        bad = offsets.copy()
+        bad[1001] = bad[1003]  # record 1001 ends before it starts
+        with pytest.raises(zx.ZxError) as err:
+            index.query_records(locked, bad)
+        assert err.value.code == 1
+        got, total = index.query_records(locked, offsets)
+        assert total == want_total
+        np.testing.assert_array_equal(got, want)

@@ -308,10 +308,14 @@ class Engine {
   // prune_ratio > 0 (segmented per-record reports): threshold pruning of the
   // colours that cannot reach count / total >= prune_ratio.
   // max_keys: no more seeds than this in the batch (its bases). cleared: the
-  // key cursors are zero already (small_plan_kernel).
+  // key cursors are not to be cleared (small_plan_kernel did, or an earlier
+  // chunk's keys are in the list). parts: of a batch in one round, the
+  // extraction alone (its keys join the list) or with the probe.
+  static constexpr int kWideExtract = 1, kWideProbe = 2;
   void run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv, uint64_t tiles_bound,
                 uint64_t max_keys, bool recover, uint64_t* counts, unsigned long long* total, uint32_t segments,
-                cudaStream_t s, double prune_ratio = 0.0, bool cleared = false);
+                cudaStream_t s, double prune_ratio = 0.0, bool cleared = false,
+                int parts = kWideExtract | kWideProbe);
   // Buckets of the ordered rounds and the window probe's slices of the rows
   // (kernels/window_probe.cuh).
   void plan_windows();
