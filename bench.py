@@ -207,29 +207,28 @@ def long_pool(cache: Path, rank: int, name: str = "c2"):
 
 def launches_per_step(ix, nbases: int, records: int) -> int:
     """Kernels one batched query launches (all compiled into libzindex_b200.so):
-    pack, count_tiles, the two kernels of the CUB tile scan and fill_tiles;
-    then the fused query kernel and, with shared counters, the counter
-    reduction, once or once per round of a split minimizer query or of the
-    wide-row form (plus the extraction kernel each round, and for ordered
-    wide rounds the counting sort's bucket count, scan and scatter). Small
-    batches take two or three."""
+    pack, count_tiles, the two kernels of the CUB tile scan and fill_tiles (one
+    kernel for small batches); then the fused query kernel and, with shared
+    counters, the counter reduction, once or once per round of a split
+    minimizer query; or, for the wide-row form, per round the extraction, the
+    sort of ordered rounds (bucket count, scan and twice bin places and tile
+    scatter), the wide probe and, with ordered rounds, the window probe (of
+    the two probes the one that the round's key count does not select returns
+    at once). Batches of up to 2^28 bases are one round."""
     lc, info = ix.launch(), ix.info
-    plan = 5
     probe = 1 + (1 if lc["smem_counters"] else 0)
     tiles_bound = nbases // 256 + records + nbases // 16384 + 1
     split = lc.get("split") and info.index_mode == 1 and lc["planes"] == 1 and lc["stage_bytes"] == 0
-    if records <= 4096 and nbases <= (1 << 20) and not lc.get("wide") and not split:
+    if lc.get("wide"):
+        plan = 1 if records <= 4096 and nbases <= (1 << 18) else 5
+        rounds = 1 if nbases <= (1 << 28) else -(-tiles_bound // 262144)
+        return plan + rounds * (2 + (6 if lc.get("order") else 0) + (1 if lc.get("order") == 1 else 0))
+    if records <= 4096 and nbases <= (1 << 20) and not split:
         # Small batches: one block packs and plans, then the fused kernel
         # (adding into the caller's counters for up to 1,024 colours).
         return 1 + 1 + (1 if lc["smem_counters"] and ix.colors > 1024 else 0)
-    if lc.get("wide"):
-        # Wide-row form: per round the dense extraction, the probe and (with
-        # shared counters) the reduction.
-        rounds = -(-tiles_bound // 262144)
-        sort = 3 if lc.get("order") else 0
-        return plan + rounds * (1 + sort + probe)
-    if lc.get("split") and info.index_mode == 1 and lc["planes"] == 1 and lc["stage_bytes"] == 0:
-        tiles_bound = nbases // 256 + records + nbases // 16384 + 1
+    plan = 5
+    if split:
         rounds = -(-tiles_bound // 262144)
         return plan + rounds * (1 + probe)
     return plan + probe

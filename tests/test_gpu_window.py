@@ -130,3 +130,27 @@ def test_page_locked_chunks_join_one_list(gpu, oracle, tmp_path, colors):
         got, total = index.query_records(locked, offsets)
         assert total == want_total
         np.testing.assert_array_equal(got, want)
+
+
+def test_more_buckets_than_a_block_counts(gpu, oracle, tmp_path):
+    """A class of 2^17 segments: 2^18 buckets, counted in L2."""
+    import subprocess
+
+    import zindex_b200 as zx
+
+    subprocess.run([str(helpers.ZX_BUILD), "--synth", "uniform:2:6000000:6000000:5", "-o",
+                    str(tmp_path / "index"), "-q", "-k", "31", "-H", "4", "-b", "8", "--device"],
+                   check=True)
+    genomes = [np.frombuffer(dna(6_000_000, 5 + c), dtype=np.uint8) for c in range(2)]
+    rng = np.random.default_rng(4)
+    reads = [genomes[i % 2][at: at + 10_000] for i, at in enumerate(rng.integers(0, 5_990_000, 1900))]
+    bases = np.concatenate(reads)
+    offsets = np.arange(len(reads) + 1, dtype=np.uint64) * 10_000
+    with zx.Index(tmp_path / "index") as index:
+        got, total = index.query_records(bases, offsets)
+        index.set_launch(cut=1)
+        once, total_once = index.query_records(bases, offsets)
+    want, want_total = oracle.query_records(tmp_path / "index", bases, offsets)
+    assert total == total_once == want_total
+    np.testing.assert_array_equal(got, want)
+    np.testing.assert_array_equal(once, want)

@@ -953,20 +953,18 @@ void Engine::plan_windows() {
   };
   // Buckets of the ordered rounds: about two per segment of the largest
   // class, at least 2^10 and at most 2^18 over the partitions; 2^13, which a
-  // block sorts in shared memory, where that leaves every class slices of
+  // block counts in shared memory, where that leaves every class slices of
   // eight chunks or what finer buckets would leave it (half the slice width
-  // costs the probe about a tenth, the sort through global counters more
-  // than half of the probe).
+  // costs the probe a tenth; counting 1.2e8 keys in L2 takes 1.1 ms more).
   order_.fbits = 10;
   while (order_.fbits + pbits < kMaxOrderBits && (1ull << order_.fbits) < 2 * most) ++order_.fbits;
-  if (order_.fbits + pbits > kBlockOrderBits && pbits < kBlockOrderBits) {
-    const int coarse = kBlockOrderBits - pbits;
+  if (order_.fbits + pbits > kLocalOrderBits && pbits < kLocalOrderBits) {
+    const int coarse = kLocalOrderBits - pbits;
     bool keep = true;
     for (uint32_t c = 0; c < host_ix_.classes; ++c)
       keep &= widest(host_ix_.cls[c], coarse) >= std::min(3, widest(host_ix_.cls[c], order_.fbits));
     if (keep) order_.fbits = coarse;
   }
-  block_order_ = order_.fbits + pbits <= kBlockOrderBits;
   if (order_.fbits + pbits > kMaxOrderBits || !wide_eligible(8)) return;
 
   // Slices of every class: as wide as fits, the remainder cut where the sum
@@ -1675,56 +1673,45 @@ void Engine::run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv,
       // read on the device.
       uint64_t* sorted = whole ? ws.round_keys[1] : ws.wide_keys_alt[b];
       cuda_check(cudaMemsetAsync(ws.wide_hist[b], 0, order_.buckets() * 4ull, xs), "memset");
-      if (block_order_) {
-        const uint32_t buckets = order_.buckets();
-        const int ogrid = sms_ * 2;
-        unsigned long long* n = ws.wide_cursor + 2 * b;
-        const bool look = windows && recover && host_ix_.rec.bits;
-        const size_t csmem = 
-            buckets * 4ull + (look ? kRecQueueBytes : 0) + (look && host_ix_.rec.filter ? kRecFilterBytes : 0);
-        cuda_check(cudaFuncSetAttribute(block_count_kernel,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem),
-                   "cudaFuncSetAttribute");
-        block_count_kernel<<<ogrid, kOrderThreads, csmem, xs>>>(
-            dix, d_color_loc_, keys, n, order_, look ? win_min_keys_ : ~0ull, ws.wide_hist[b],
-            counts);
-        cuda_check(cudaGetLastError(), "block_count_kernel");
-        order_scan_kernel<<<1, 1024, 0, xs>>>(ws.wide_hist[b], buckets);
-        cuda_check(cudaGetLastError(), "order_scan_kernel");
-        cuda_check(cudaFuncSetAttribute(tile_scatter_kernel,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)sizeof(TileSmem)),
-                   "cudaFuncSetAttribute");
-        // By the upper half of the bucket bits into the other list, then by
-        // all of them back into this one.
-        int half = 0;
-        while ((1u << (2 * half)) < buckets) ++half;
-        const uint64_t* from = keys;
-        uint64_t* to = sorted;
-        for (int shift : {half, 0}) {
-          const uint32_t bins = buckets >> shift;
-          order_bins_kernel<<<(bins + 255) / 256, 256, 0, xs>>>(ws.wide_hist[b], bins, shift,
-                                                                ws.wide_next[b]);
-          cuda_check(cudaGetLastError(), "order_bins_kernel");
-          tile_scatter_kernel<<<ogrid, kTileThreads, sizeof(TileSmem), xs>>>(
-              from, n, order_, shift, ws.wide_next[b], to);
-          cuda_check(cudaGetLastError(), "tile_scatter_kernel");
-          from = sorted;
-          to = keys;
-        }
-        sorted = keys;
-        bucket_end = ws.wide_hist[b] + 1;
-      } else {
-        const int ogrid = sms_ * 8;
-        order_count_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + 2 * b, order_,
-                                                  ws.wide_hist[b]);
-        cuda_check(cudaGetLastError(), "order_count_kernel");
-        order_scan_kernel<<<1, 1024, 0, xs>>>(ws.wide_hist[b], order_.buckets());
-        cuda_check(cudaGetLastError(), "order_scan_kernel");
-        order_scatter_kernel<<<ogrid, 256, 0, xs>>>(keys, ws.wide_cursor + 2 * b, order_,
-                                                    ws.wide_hist[b], sorted);
-        cuda_check(cudaGetLastError(), "order_scatter_kernel");
+      const uint32_t buckets = order_.buckets();
+      const int ogrid = sms_ * 2;
+      unsigned long long* n = ws.wide_cursor + 2 * b;
+      const bool look = windows && recover && host_ix_.rec.bits;
+      const size_t csmem = (buckets <= kLocalBuckets ? buckets * 4ull : 0) +
+                           (look ? kRecQueueBytes : 0) +
+                           (look && host_ix_.rec.filter ? kRecFilterBytes : 0);
+      cuda_check(cudaFuncSetAttribute(block_count_kernel,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem),
+                 "cudaFuncSetAttribute");
+      block_count_kernel<<<ogrid, kOrderThreads, csmem, xs>>>(
+          dix, d_color_loc_, keys, n, order_, look ? win_min_keys_ : ~0ull, ws.wide_hist[b],
+          counts);
+      cuda_check(cudaGetLastError(), "block_count_kernel");
+      order_scan_kernel<<<1, 1024, 0, xs>>>(ws.wide_hist[b], buckets);
+      cuda_check(cudaGetLastError(), "order_scan_kernel");
+      cuda_check(cudaFuncSetAttribute(tile_scatter_kernel,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(TileSmem)),
+                 "cudaFuncSetAttribute");
+      // By the upper half of the bucket bits into the other list, then by
+      // all of them back into this one.
+      int half = 0;
+      while ((1u << (2 * half)) < buckets) ++half;
+      const uint64_t* from = keys;
+      uint64_t* to = sorted;
+      for (int shift : {half, 0}) {
+        const uint32_t bins = buckets >> shift;
+        order_bins_kernel<<<(bins + 255) / 256, 256, 0, xs>>>(ws.wide_hist[b], bins, shift,
+                                                              ws.wide_next[b]);
+        cuda_check(cudaGetLastError(), "order_bins_kernel");
+        tile_scatter_kernel<<<ogrid, kTileThreads, sizeof(TileSmem), xs>>>(
+            from, n, order_, shift, ws.wide_next[b], to);
+        cuda_check(cudaGetLastError(), "tile_scatter_kernel");
+        from = sorted;
+        to = keys;
       }
+      sorted = keys;
+      bucket_end = ws.wide_hist[b] + 1;
       probe_keys = sorted;
     }
     if (segments) {
@@ -1751,11 +1738,6 @@ void Engine::run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv,
                                                        bucket_end, ws.wide_cursor + 2 * b + 1,
                                                        counts, total);
       cuda_check(cudaGetLastError(), "window_probe_kernel");
-      if (!block_order_ && recover && host_ix_.rec.bits) {
-        recover_kernel<<<sms_ * 8, 256, 0, s>>>(dix, d_color_loc_, probe_keys, ws.wide_cursor + 2 * b,
-                                                win_min_keys_, counts);
-        cuda_check(cudaGetLastError(), "recover_kernel");
-      }
     }
     if (overlap) cuda_check(cudaEventRecord(ws.wide_probe[b], s), "cudaEventRecord");
   }
@@ -1764,8 +1746,7 @@ void Engine::run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv,
 void Engine::ensure_order_capacity(Workspace& ws, int b, bool whole) {
   if (!ws.wide_hist[b]) {
     dev_alloc(&ws.wide_hist[b], order_.buckets() + 4ull, "round order buckets");
-    if (block_order_)
-      dev_alloc(&ws.wide_next[b], order_.buckets(), "round order places");
+    dev_alloc(&ws.wide_next[b], order_.buckets(), "round order places");
     ws.release_graphs();
   }
   if (!whole && !ws.wide_keys_alt[b]) {

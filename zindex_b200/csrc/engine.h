@@ -347,7 +347,6 @@ class Engine {
   ColorLoc* d_color_loc_ = nullptr;  // colour -> class, member, group (wide probe)
   OrderKey order_;
   bool findere_dense_ = false;  // kernels/findere.cuh runs this index's queries
-  bool block_order_ = false;  // buckets fit a block's shared memory (kernels/key_order.cuh)
   WinSlice* d_win_slices_ = nullptr;  // none: no window probe for this index
   uint32_t win_slices_ = 0, win_weights_ = 0;
   bool win_b16_ = false;  // 16-bit fields of single-member groups

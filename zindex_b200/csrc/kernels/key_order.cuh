@@ -1,16 +1,19 @@
-// Block order: the counting sort of a round's keys when its buckets fit a
-// block's shared memory (at most 2^13).
+// Ordered rounds: the counting sort of a round's keys by bucket (order_bucket).
 //
-// The sort through global counters (order_count / scan / scatter_kernel) does
-// two L2 atomics and one lone 8-byte write per key. Here block_count_kernel
-// counts in shared memory (and looks up each key's recovered origins for the
-// window probe, since it has the key in hand), and two passes of
-// tile_scatter_kernel place the keys: by the buckets' upper bits, then by the
-// lower ones. A pass sorts a tile of 8,192 keys in shared memory and writes
-// each bin's keys as one run at a place reserved with one atomic; about 2^7
-// bins a pass keep the runs at some 64 keys. (One pass over all 2^13 buckets
-// with a block's own runs left millions of partly written sectors open and
-// took 4.5 ms for 1.2e8 keys.)
+// block_count_kernel counts the buckets - in shared memory up to 2^13 of them,
+// else with one L2 atomic per key - and looks up each key's recovered origins
+// for the window probe, since it has the key in hand; order_scan_kernel makes
+// the buckets' places; two passes of tile_scatter_kernel place the keys, by the
+// buckets' upper half of the bits, then by all of them. A pass sorts a tile of
+// 8,192 keys in shared memory and writes each bin's keys as one run at a place
+// reserved with one atomic; 2^5 to 2^9 bins a pass keep the runs long.
+//
+// B200, 1.2e8 keys, 2^13 buckets: count with recovered origins 0.86 ms, the
+// passes 0.72 ms each. (A scatter through global counters, two atomics and a
+// lone 8-byte write per key, took 2.0 ms, its count 1.2 ms and the recovered
+// origins apart 2.4 ms; one pass over 2^13 buckets with a block's own runs
+// left millions of partly written sectors open and took 4.5 ms; tiles of 4,096
+// keys at three blocks per SM 0.80 ms a pass.)
 #pragma once
 #include <stdint.h>
 
@@ -18,7 +21,8 @@
 
 namespace zx {
 
-constexpr int kBlockOrderBits = 13;
+constexpr int kLocalOrderBits = 13;  // buckets that a block counts in shared memory
+constexpr uint32_t kLocalBuckets = 1u << kLocalOrderBits;
 constexpr int kOrderThreads = 1024;
 constexpr int kOrderUnroll = 4;  // keys of a thread in flight
 
@@ -50,11 +54,13 @@ __global__ void __launch_bounds__(kOrderThreads)
   order_run(n, lo, hi);
   if (lo >= hi) return;
   const uint32_t buckets = o.buckets();
-  uint32_t* filter = bins + buckets;
+  const bool local = buckets <= kLocalBuckets;
+  uint32_t* filter = bins + (local ? buckets : 0);
   const DevRecovery rec = gix->rec;
   const bool recover = n >= min_keys;
   const bool filtered = recover && rec.filter;
-  for (uint32_t b = threadIdx.x; b < buckets; b += kOrderThreads) bins[b] = 0;
+  if (local)
+    for (uint32_t b = threadIdx.x; b < buckets; b += kOrderThreads) bins[b] = 0;
   if (filtered)
     for (uint32_t i = threadIdx.x; i < (uint32_t)(kRecFilterBytes / 16); i += kOrderThreads)
       reinterpret_cast<uint4*>(filter)[i] = __ldg(reinterpret_cast<const uint4*>(rec.filter) + i);
@@ -76,7 +82,10 @@ __global__ void __launch_bounds__(kOrderThreads)
     }
 #pragma unroll
     for (int u = 0; u < kOrderUnroll; ++u)
-      if (live[u]) atomicAdd(bins + order_bucket(key[u], o), 1u);
+      if (live[u]) {
+        if (local) atomicAdd(bins + order_bucket(key[u], o), 1u);
+        else atomicAdd(hist + order_bucket(key[u], o), 1u);
+      }
     if (!recover) continue;
 #pragma unroll
     for (int u = 0; u < kOrderUnroll; ++u) {
@@ -95,6 +104,7 @@ __global__ void __launch_bounds__(kOrderThreads)
   }
   if (recover && lane < queued)
     recover_key(*gix, color_loc, queue[lane], WideCounters{nullptr, counts});
+  if (!local) return;
   __syncthreads();
   for (uint32_t b = threadIdx.x; b < buckets; b += kOrderThreads)
     if (bins[b]) atomicAdd(hist + b, bins[b]);

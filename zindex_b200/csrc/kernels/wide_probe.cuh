@@ -342,17 +342,7 @@ __device__ __forceinline__ uint32_t order_bucket(uint64_t key, const OrderKey& o
          (uint32_t)(mixsplit(key, o.seed) >> (64 - o.fbits));
 }
 
-// Ordered rounds, step 1: keys per bucket (hist zeroed before).
-__global__ void order_count_kernel(const uint64_t* __restrict__ keys,
-                                   const unsigned long long* __restrict__ nkeys, OrderKey o,
-                                   uint32_t* __restrict__ hist) {
-  const uint64_t n = *nkeys;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    atomicAdd(hist + order_bucket(keys[i], o), 1u);
-}
-
-// Step 2 (one block of 1,024 threads): the buckets' first places, in place,
+// The buckets' first places from their counts (one block of 1,024 threads), in place,
 // and the number of keys in hist[buckets].
 // The table goes through in stretches of 16,384 buckets, 16 consecutive ones
 // per thread in four 16-byte loads: a thread-strided walk of the same table
@@ -402,19 +392,6 @@ __global__ void __launch_bounds__(1024) order_scan_kernel(uint32_t* __restrict__
     run += all;
   }
   if (tid == 0) hist[buckets] = run;
-}
-
-// Step 3: every key to its bucket's next place in out[]; next[b] ends as the
-// end of bucket b.
-__global__ void order_scatter_kernel(const uint64_t* __restrict__ keys,
-                                     const unsigned long long* __restrict__ nkeys, OrderKey o,
-                                     uint32_t* __restrict__ next, uint64_t* __restrict__ out) {
-  const uint64_t n = *nkeys;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = keys[i];
-    out[atomicAdd(next + order_bucket(k, o), 1u)] = k;
-  }
 }
 
 // Shared memory of the wide probe: DevIndex copy, colour counters (optional),

@@ -26,7 +26,7 @@
 //   carry-save adder takes four seeds in 6 logic operations plus the carry)
 //   and reach the block's counters every 255 seeds.
 // * Recovered origins are counted once per seed, when the keys are sorted
-//   (block_count_kernel) or by recover_kernel.
+//   (block_count_kernel).
 #pragma once
 #include <stdint.h>
 
@@ -381,20 +381,6 @@ __global__ void __launch_bounds__(kWinThreads, 2)
       }
     }
   }
-}
-
-// Recovered origins of a round probed by the window probe and sorted through
-// global counters (block_count_kernel does it for the others).
-__global__ void __launch_bounds__(256)
-    recover_kernel(const DevIndex* __restrict__ gix, const ColorLoc* __restrict__ color_loc,
-                   const uint64_t* __restrict__ keys, const unsigned long long* __restrict__ nkeys,
-                   uint64_t min_keys, uint64_t* __restrict__ counts) {
-  const uint64_t n = *nkeys;
-  if (n < min_keys) return;
-  const WideCounters cnt{nullptr, counts};
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    recover_key(*gix, color_loc, keys[i], cnt);
 }
 
 }  // namespace zx
