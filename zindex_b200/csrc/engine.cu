@@ -1681,7 +1681,8 @@ void Engine::run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv,
                            (look ? kRecQueueBytes : 0) +
                            (look && host_ix_.rec.filter ? kRecFilterBytes : 0);
       cuda_check(cudaFuncSetAttribute(block_count_kernel,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem),
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(kLocalBuckets * 4 + kRecQueueBytes + kRecFilterBytes)),
                  "cudaFuncSetAttribute");
       block_count_kernel<<<ogrid, kOrderThreads, csmem, xs>>>(
           dix, d_color_loc_, keys, n, order_, look ? win_min_keys_ : ~0ull, ws.wide_hist[b],
