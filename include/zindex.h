@@ -207,6 +207,13 @@ int zx_default_launch(const zx_index* index, zx_launch* out);
  * for indexes whose default is not the wide-row form. */
 int zx_default_fused_launch(const zx_index* index, zx_launch* out);
 
+/* Most bases of an unsegmented batch whose seeds are sorted and probed as one
+ * list (0: the default and the most, 2^28). The lists hold 16 to 20 bytes per
+ * base of the largest such batch until the index is closed; this call gives
+ * them back. A larger batch takes several rounds of 2^18 tiles (the wide-row
+ * form) or the fused kernel. Never changes results. */
+int zx_set_round_bases(zx_index* index, uint64_t bases);
+
 /* Status of the asynchronous zx_query_device / zx_query_device_noalloc calls
  * of this index since the last status call: ZX_OK; ZX_EINVAL when record
  * offsets of any of them were invalid

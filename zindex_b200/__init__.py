@@ -253,6 +253,12 @@ class Index:
                      int(d["order"] if order is None else order))
         _lib.check(_lib.load().zx_set_launch(self._h, byref(l)))
 
+    def set_round_bases(self, bases: int = 0) -> None:
+        """Most bases of an unsegmented batch that is sorted and probed as one
+        list (0: 2^28, the most); gives the lists' memory back. Larger batches
+        take several rounds, or the fused kernel. Never changes results."""
+        _lib.check(_lib.load().zx_set_round_bases(self._h, int(bases)))
+
     def query_status(self) -> None:
         """Raise if a bounded device wait expired in an asynchronous query."""
         _lib.check(_lib.load().zx_query_status(self._h))

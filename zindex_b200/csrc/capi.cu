@@ -346,6 +346,14 @@ int zx_set_launch(zx_index* index, const zx_launch* l) {
   });
 }
 
+int zx_set_round_bases(zx_index* index, uint64_t bases) {
+  return guarded([&] {
+    zx::check(index, zx::kEInval, "null argument");
+    std::lock_guard<std::mutex> lock(index->mu);
+    index->engine->set_round_bases(bases);
+  });
+}
+
 int zx_query_status(zx_index* index) {
   return guarded([&] {
     zx::check(index, zx::kEInval, "null argument");

@@ -925,6 +925,7 @@ void Engine::load(const std::string& dir, const OpenOptions& options) {
                      std::find(banked.begin(), banked.end(), false) == banked.end();
   }
   launch_ = default_launch();
+  round_bases_ = kRoundKeys;
   ws_ = make_workspace();
   load_s_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
 }
@@ -1129,7 +1130,7 @@ bool Engine::wide_form(const QueryLaunch& l) const { return l.wide && wide_eligi
 
 bool Engine::dense_batch(uint64_t nbases) const {
   if (!launch_default_ || launch_.wide || !win_slices_ || nbases <= kSmallBases ||
-      nbases > kRoundKeys)
+      nbases > round_bases_)
     return false;
   uint64_t seeds = nbases;
   if (sp_.mode == kMinimizers) seeds = 2 * nbases / (uint64_t)(sp_.ocm.w + 1);
@@ -1283,7 +1284,22 @@ std::unique_ptr<Workspace> Engine::make_workspace() {
   auto ws = std::make_unique<Workspace>();
   ws->device = device_;
   cuda_check(cudaStreamCreateWithFlags(&ws->stream, cudaStreamNonBlocking), "cudaStreamCreate");
+  // Always: which batches of a host query take the wide form depends on each
+  // chunk's size (dense_batch), not on the largest one alone.
+  dev_alloc(&ws->wide_cursor, 4, "dense key cursors");
   return ws;
+}
+
+void Engine::set_round_bases(uint64_t bases) {
+  cuda_check(cudaSetDevice(device_), "cudaSetDevice");
+  round_bases_ = bases ? std::min(bases, kRoundKeys) : kRoundKeys;
+  ws_->release_graphs();
+  for (uint64_t*& p : ws_->round_keys) {
+    if (p) cudaFree(p);
+    p = nullptr;
+  }
+  ws_->cap_round_keys = 0;
+  ws_->round_refused = ~0ull;
 }
 
 void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, bool segmented,
@@ -1363,7 +1379,6 @@ void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, b
   if (kernel_mode(launch_) == 4 || (wide_form(launch_) && !whole)) ensure_split_capacity(ws);
   const bool rounds =
       !whole && wide_form(launch_) && nbases / kTileWindows + records + nbases / kFindereTask + 1 > kSplitTiles;
-  if (wide) ensure_cursors(ws);
   if (rounds) ensure_wide_pipeline(ws);
   if (((wide_form(launch_) && launch_.order) || (dense && whole)) && !segmented) {
     ensure_order_capacity(ws, 0, whole);
@@ -1757,7 +1772,7 @@ void Engine::ensure_order_capacity(Workspace& ws, int b, bool whole) {
 }
 
 bool Engine::ensure_round_capacity(Workspace& ws, uint64_t keys) {
-  if (keys > kRoundKeys || keys >= ws.round_refused) return false;
+  if (keys > round_bases_ || keys >= ws.round_refused) return false;
   const int lists = launch_.wide && !launch_.order ? 1 : 2;
   bool have = true;
   for (int i = 0; i < lists; ++i) have &= ws.round_keys[i] && ws.cap_round_keys >= keys;
@@ -1872,12 +1887,6 @@ void Engine::ensure_split_capacity(Workspace& ws) {
   if (ws.split_keys) return;
   dev_alloc(&ws.split_keys, kSplitTiles * kTileWindows, "split key slots");
   dev_alloc(&ws.split_counts, kSplitTiles, "split key counts");
-  ws.release_graphs();
-}
-
-void Engine::ensure_cursors(Workspace& ws) {
-  if (ws.wide_cursor) return;
-  dev_alloc(&ws.wide_cursor, 4, "dense key cursors");
   ws.release_graphs();
 }
 
@@ -2386,7 +2395,7 @@ void Engine::query_host(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   // 250,000 reads of 256 colours in four chunks took 3.66 ms, joined 2.96 ms).
   // Staging pageable memory takes longer than the probes, which then hide
   // behind it chunk by chunk.
-  const bool joined = direct && chunks > 1 && nbases <= kRoundKeys && (wide_form(launch_) || dense_batch(nbases));
+  const bool joined = direct && chunks > 1 && nbases <= round_bases_ && (wide_form(launch_) || dense_batch(nbases));
   ensure_capacity(ws, nbases, records + chunks, false, joined ? nbases : most);
   ensure_host_capacity(ws, nbases, records + chunks);
   const uint64_t colors = m_.colors.size();

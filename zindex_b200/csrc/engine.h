@@ -151,6 +151,9 @@ class Engine {
   QueryLaunch launch() const { return launch_; }
   void set_launch(const QueryLaunch& l);
   QueryLaunch default_launch() const;
+  // Most bases of an unsegmented batch that is sorted and probed as one list
+  // (0: kRoundKeys, also the most); the lists held are given back.
+  void set_round_bases(uint64_t bases);
   // The fused kernel's default launch (segmented and allocation-free queries
   // run the fused kernel; a wide-row launch maps to it, keeping its cut).
   QueryLaunch default_fused_launch() const;
@@ -296,10 +299,9 @@ class Engine {
   // Ordered wide-row rounds: sort buffers of key list b (0 or 1); whole: the
   // sorted keys go to the round lists.
   void ensure_order_capacity(Workspace& ws, int b, bool whole);
-  // Key lists of a batch in one round (up to kRoundKeys keys); false: too many
+  // Key lists of a batch in one round (up to round_bases_ keys); false: too many
   // keys or no memory, and the batch runs in rounds of kSplitTiles tiles.
   bool ensure_round_capacity(Workspace& ws, uint64_t keys);
-  void ensure_cursors(Workspace& ws);
   // Wide-row form over the planned tiles of a packed batch: rounds of up to
   // kSplitTiles tiles, each a dense extraction and a wide probe. segments = 0:
   // one query into counts / *total; segments > 0: a segmented query, request
@@ -351,6 +353,7 @@ class Engine {
   uint32_t win_slices_ = 0, win_weights_ = 0;
   bool win_b16_ = false;  // 16-bit fields of single-member groups
   uint64_t win_min_keys_ = ~0ull;
+  uint64_t round_bases_ = 0;  // set_round_bases; kRoundKeys once loaded
   std::vector<void*> allocations_;
   uint64_t resident_bytes_ = 0;
   std::unique_ptr<Workspace> ws_;
