@@ -41,3 +41,54 @@ def test_records_past_and_below_the_round_limit(gpu, oracle, tmp_path):
         got, total = index.query_records(two, two_offsets, plain=True)
         assert total == want_two_total
         np.testing.assert_array_equal(got, want_two)
+
+
+@pytest.mark.parametrize("opts", [dict(), dict(mode="findere", k=31, z=10), dict(homopolymer=True),
+                                  dict(mode="minimizers", k=31, m=21)],
+                         ids=["kmers", "findere", "homopolymer", "minimizers"])
+@pytest.mark.parametrize("colors", [12, 270], ids=["narrow", "wide"])
+def test_overlapping_records_stay_inside_the_lists(gpu, oracle, tmp_path, opts, colors):
+    """Offsets that go back to 0 again and again: every other record is the
+    whole batch, so the records hold many times the batch's tiles and seeds.
+    They are reported, no count is higher than those records' own, and the
+    index keeps answering correctly."""
+    import torch
+
+    import zindex_b200 as zx
+
+    fof = make_genomes(tmp_path / "g", colors, 3000, 31)
+    ix = build_index(fof, tmp_path / "index", **{**dict(k=31, H=4, b=8, min_docs=1), **opts})
+    genomes = [dna(3000, 31 + c) for c in range(colors)]
+    rng = np.random.default_rng(12)
+    dev = torch.device("cuda", 0)
+    with zx.Index(ix) as index:
+        for nbases, records in ((300_000, 3001), (1_500_000, 801)):
+            reads = sample_reads(genomes, rng, nbases // 150, 150)
+            bases, offsets = zx.pack_records(reads)
+            one = np.array([0, len(bases)], dtype=np.uint64)
+            want, want_total = oracle.query_records(ix, bases, one)
+            bad = np.zeros(records + 1, dtype=np.int64)
+            bad[1::2] = len(bases)
+            whole = (records + 1) // 2  # records that are the whole batch
+            d_b = torch.from_numpy(bases).to(dev)
+            d_bad = torch.from_numpy(bad).to(dev)
+            counts = torch.zeros(index.colors, dtype=torch.int64, device=dev)
+            total = torch.zeros(1, dtype=torch.int64, device=dev)
+            args = (d_b.data_ptr(), len(bases), d_bad.data_ptr(), records, counts.data_ptr(),
+                    total.data_ptr())
+            calls = [lambda: index.query_device(*args, use_graph=False)]
+            if "homopolymer" not in opts:
+                calls.append(lambda: index.query_device_noalloc(*args))
+            for call in calls:
+                counts.zero_()
+                total.zero_()
+                call()
+                torch.cuda.synchronize(dev)
+                with pytest.raises(zx.ZxError) as err:
+                    index.query_status()
+                assert err.value.code == 1
+                assert 0 < int(total) <= whole * want_total
+                assert np.all(counts.cpu().numpy() <= whole * want.astype(np.int64))
+            got, got_total = index.query_records(bases, one)
+            assert got_total == want_total
+            np.testing.assert_array_equal(got, want)

@@ -515,7 +515,8 @@ class DeviceBuilder {
     tiles_.need(std::max<uint32_t>(ntiles, 1), "tiles");
     if (records)
       fill_tiles_kernel<<<grid_for(records, sms_), 256, 0, s_>>>(d_rec_off_.p, records, nbases,
-                                                                 bc_.fp.k, tile_first_.p, tiles_.p);
+                                                                 bc_.fp.k, tile_first_.p, tiles_.p,
+                                                                 std::max<uint32_t>(ntiles, 1));
     // Seeds into each dataset's region (capacity: its bases).
     raw_.need(nbases + 1, "seed regions");
     sorted_.need(nbases + 1, "sorted seeds");

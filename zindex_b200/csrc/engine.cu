@@ -58,6 +58,14 @@ void host_alloc(T** p, uint64_t count) {
   cuda_check(cudaMallocHost((void**)p, count * sizeof(T)), "cudaMallocHost");
 }
 
+// first[r] = the tiles of the records before r (n entries; SumTiles).
+cudaError_t scan_tiles(void* tmp, size_t& bytes, const uint32_t* counts, uint32_t* first,
+                       uint64_t n, cudaStream_t s) {
+  return cub::DeviceScan::ExclusiveScan(tmp, bytes, counts, first, SumTiles{}, 0u, (int)n, s);
+}
+
+uint32_t tile_cap(uint64_t tiles) { return (uint32_t)std::min<uint64_t>(tiles, 0xFFFFFFFFull); }
+
 __global__ void repack_rows_kernel(const uint8_t* __restrict__ src, uint64_t rows,
                                    uint32_t row_bytes, uint32_t stride, uint8_t* __restrict__ dst) {
   uint64_t total = rows * stride;
@@ -437,9 +445,7 @@ void Engine::query_device_noalloc(const uint8_t* bases, uint64_t nbases, const u
           : 0;
   // Scratch layout, every region 256-byte aligned.
   size_t scan_bytes = 0;
-  cuda_check(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (uint32_t*)nullptr,
-                                           (uint32_t*)nullptr, (int)(records + 1)),
-             "scan size");
+  cuda_check(scan_tiles(nullptr, scan_bytes, nullptr, nullptr, records + 1, s), "scan size");
   uint64_t at = 0;
   auto carve = [&](uint64_t bytes) {
     uint64_t off = at;
@@ -471,12 +477,10 @@ void Engine::query_device_noalloc(const uint8_t* bases, uint64_t nbases, const u
     cuda_check(cudaGetLastError(), "count_tiles_kernel");
   }
   size_t tmp = scan_bytes;
-  cuda_check(cub::DeviceScan::ExclusiveSum(scan_tmp, tmp, tile_counts, tile_first,
-                                           (int)(records + 1), s),
-             "tile scan");
+  cuda_check(scan_tiles(scan_tmp, tmp, tile_counts, tile_first, records + 1, s), "tile scan");
   if (records) {
     fill_tiles_kernel<<<rgrid, 256, 0, s>>>(offsets, records, nbases, span(), tile_first,
-                                            tile_list);
+                                            tile_list, tile_cap(tiles));
     cuda_check(cudaGetLastError(), "fill_tiles_kernel");
   }
   BatchView bv{PackedView{packed, invalid}, offsets, tile_list, tile_first + records, fstate};
@@ -1328,7 +1332,7 @@ void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, b
     dev_alloc(&ws.tile_counts, cap + 1, "tile counts");
     dev_alloc(&ws.tile_first, cap + 1, "tile offsets");
     size_t tmp = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tmp, ws.tile_counts, ws.tile_first, (int)(cap + 1));
+    cuda_check(scan_tiles(nullptr, tmp, nullptr, nullptr, cap + 1, nullptr), "scan size");
     dev_alloc((uint8_t**)&ws.scan_tmp, tmp, "scan scratch");
     ws.scan_tmp_bytes = tmp;
     ws.cap_records = cap;
@@ -1462,12 +1466,11 @@ void Engine::plan_tiles(Workspace& ws, const uint64_t* offsets, uint64_t records
     cuda_check(cudaGetLastError(), "count_tiles_kernel");
   }
   size_t tmp = ws.scan_tmp_bytes;
-  cuda_check(cub::DeviceScan::ExclusiveSum(ws.scan_tmp, tmp, ws.tile_counts, ws.tile_first,
-                                           (int)(records + 1), s),
+  cuda_check(scan_tiles(ws.scan_tmp, tmp, ws.tile_counts, ws.tile_first, records + 1, s),
              "tile scan");
   if (records) {
     fill_tiles_kernel<<<grid, 256, 0, s>>>(offsets, records, nbases, span(), ws.tile_first,
-                                           ws.tiles);
+                                           ws.tiles, tile_cap(ws.cap_tiles));
     cuda_check(cudaGetLastError(), "fill_tiles_kernel");
   }
 }
@@ -1491,8 +1494,8 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
       for (tw = 32; tw < kTileWindows && nbases / tw > kSmallTiles;) tw *= 2;
     small_plan_kernel<<<1, 1024, 0, s>>>(bases, nbases, ws.packed, ws.invalid, words, offsets,
                                          (uint32_t)records, span(), m_.index_mode == kFindere, tw,
-                                         ws.tile_first, ws.tiles, fused ? nullptr : ws.wide_cursor,
-                                         ws.error);
+                                         ws.tile_first, ws.tiles, tile_cap(ws.cap_tiles),
+                                         fused ? nullptr : ws.wide_cursor, ws.error);
     cuda_check(cudaGetLastError(), "small_plan_kernel");
     if (fused && m_.colors.size() <= kSmallColors) l.smem_counters = 0;
   } else {

@@ -65,19 +65,33 @@ __global__ void count_tiles_kernel(const uint64_t* __restrict__ offsets, uint64_
   }
 }
 
+// Sum of tile counts that stays at 2^32 - 1 instead of wrapping.
+struct SumTiles {
+  __host__ __device__ uint32_t operator()(uint32_t a, uint32_t b) const {
+    const uint32_t s = a + b;
+    return s < a ? ~0u : s;
+  }
+};
+
+// The tiles of every record from first[r] on. The list holds `cap` tiles, which
+// records one after the other never exceed; records that overlap (possible
+// only where offsets decrease, which count_tiles_kernel reports) may. The list
+// then ends after cap tiles, all of them written, and first[] says so.
 __global__ void fill_tiles_kernel(const uint64_t* __restrict__ offsets, uint64_t records,
-                                  uint64_t nbases, int span, const uint32_t* __restrict__ first,
-                                  Tile* __restrict__ tiles) {
+                                  uint64_t nbases, int span, uint32_t* __restrict__ first,
+                                  Tile* __restrict__ tiles, uint32_t cap) {
   for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < records;
        r += (uint64_t)gridDim.x * blockDim.x) {
     uint32_t w = record_windows(offsets, r, span, nbases, nullptr);
     uint32_t t = first[r];
-    for (uint32_t w0 = 0; w0 < w;) {
+    if (t > cap) first[r] = t = cap;
+    for (uint32_t w0 = 0; w0 < w && t < cap;) {
       uint32_t task = (w0 / kFindereTask) * kFindereTask;
       uint32_t end = min(w, min(w0 + kTileWindows, task + kFindereTask));
       tiles[t++] = Tile{(uint32_t)r, w0, end - w0, task};
       w0 = end;
     }
+    if (r + 1 == records && first[records] > cap) first[records] = cap;
   }
 }
 
@@ -99,8 +113,8 @@ __global__ void __launch_bounds__(1024)
                       uint64_t* __restrict__ packed, uint32_t* __restrict__ invalid,
                       uint64_t words, const uint64_t* __restrict__ offsets, uint32_t records,
                       int span, int findere, uint32_t tw, uint32_t* __restrict__ tile_first,
-                      Tile* __restrict__ tiles, unsigned long long* __restrict__ cursor,
-                      uint32_t* __restrict__ err) {
+                      Tile* __restrict__ tiles, uint32_t cap,
+                      unsigned long long* __restrict__ cursor, uint32_t* __restrict__ err) {
   __shared__ uint32_t sums[1024];
   const uint32_t T = blockDim.x, tid = threadIdx.x;
   if (cursor && tid < 2) cursor[tid] = 0;
@@ -120,18 +134,20 @@ __global__ void __launch_bounds__(1024)
     sums[tid] += v;
     __syncthreads();
   }
-  uint32_t t = tid ? sums[tid - 1] : 0u;
+  // (At most cap tiles, as in fill_tiles_kernel; 4,096 records of 1 MiB do not
+  // wrap the sums.)
+  uint32_t t = min(cap, tid ? sums[tid - 1] : 0u);
   for (uint32_t r = lo; r < hi; ++r) {
     tile_first[r] = t;
     const uint32_t w = record_windows(offsets, r, span, nbases, nullptr);
-    for (uint32_t w0 = 0; w0 < w;) {
+    for (uint32_t w0 = 0; w0 < w && t < cap;) {
       const uint32_t task = (w0 / kFindereTask) * kFindereTask;
       const uint32_t end = min(w, min(w0 + tw, task + kFindereTask));
       tiles[t++] = Tile{r, w0, end - w0, task};
       w0 = end;
     }
   }
-  if (tid == T - 1) tile_first[records] = sums[T - 1];
+  if (tid == T - 1) tile_first[records] = min(cap, sums[T - 1]);
 }
 
 struct BatchView {
