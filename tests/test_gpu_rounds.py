@@ -92,3 +92,51 @@ def test_overlapping_records_stay_inside_the_lists(gpu, oracle, tmp_path, opts, 
             got, got_total = index.query_records(bases, one)
             assert got_total == want_total
             np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("opts", [dict(k=31), dict(k=45), dict(mode="minimizers", k=25, m=21)],
+                         ids=["short", "long", "minimizers"])
+def test_a_full_key_list_has_no_holes(gpu, tmp_path, opts):
+    """Records that overlap fill the key list. The list's old keys (all in the
+    first genome) must not come back - seeds of random bases hit no 32-bit
+    fingerprint - and it is full to the last place in every run."""
+    import torch
+
+    import zindex_b200 as zx
+
+    fof = make_genomes(tmp_path / "g", 64, 3000, 31)
+    ix = build_index(fof, tmp_path / "index", **{**dict(H=4, b=32, min_docs=1), **opts})
+    rng = np.random.default_rng(13)
+    dev = torch.device("cuda", 0)
+    nbases, records = 1_500_000, 160_001
+    # (The list has a quarter more room than the batch that made it.)
+    hits = np.frombuffer(dna(3000, 31) * (nbases * 5 // 4 // 3000), dtype=np.uint8)
+    misses = np.frombuffer(b"ACGT", dtype=np.uint8)[rng.integers(0, 4, nbases)]
+    # Records of 1 to 200 windows, so that small ones still fit where larger
+    # ones no longer do.
+    bad = np.empty(records + 1, dtype=np.int64)
+    bad[0::2] = rng.integers(0, 30, len(bad[0::2]))
+    bad[1::2] = bad[0::2] + rng.integers(45, 245, len(bad[1::2]))
+    d_bad = torch.from_numpy(bad).to(dev)
+    one = torch.tensor([0, len(hits)], dtype=torch.int64, device=dev)
+    with zx.Index(ix) as index:
+        assert index.launch()["wide"]
+        counts = torch.zeros(index.colors, dtype=torch.int64, device=dev)
+        total = torch.zeros(1, dtype=torch.int64, device=dev)
+        out = (counts.data_ptr(), total.data_ptr())
+        d_hits, d_misses = torch.from_numpy(hits.copy()).to(dev), torch.from_numpy(misses).to(dev)
+        totals = []
+        for i in range(40):
+            if i:
+                index.query_device(d_hits.data_ptr(), len(hits), one.data_ptr(), 1, *out,
+                                   use_graph=False)
+            counts.zero_()
+            total.zero_()
+            index.query_device(d_misses.data_ptr(), nbases, d_bad.data_ptr(), records, *out,
+                               use_graph=False)
+            torch.cuda.synchronize(dev)
+            with pytest.raises(zx.ZxError):
+                index.query_status()
+            totals.append(int(total))
+            assert int(counts.sum()) == 0
+        assert min(totals) == max(totals) >= nbases

@@ -119,7 +119,7 @@ struct WideRound {
   // probe (window_probe.cuh).
   uint64_t max_keys = ~0ull;
   // Keys that the unsegmented list holds; more (records that overlap because
-  // offsets decrease) are dropped and reported.
+  // offsets decrease) are dropped and reported (list_is_full).
   uint64_t key_cap = ~0ull;
   uint32_t* err = nullptr;
 };
@@ -171,6 +171,16 @@ __global__ void wide_rounds_kernel(const unsigned long long* __restrict__ cursor
   if (tid == T - 1) round_first[nseg] = part[T - 1];
 }
 
+// For a warp whose keys do not all fit: it writes those that do, and the
+// cursor never goes back below the list's end, so every place before the
+// cursor is written by the one warp that got it. (Taking the cursor back by
+// the whole amount left places that nobody wrote, with an earlier batch's
+// keys.)
+__device__ __forceinline__ void list_is_full(unsigned long long* cursor, const WideRound& sg) {
+  atomicMin(cursor, (unsigned long long)sg.key_cap);
+  atomicOr(sg.err, kErrOffsets);
+}
+
 // extract_dense_kernel for canonical k-mers of k <= 32: a warp takes several
 // tiles at a time, counts their valid windows and reserves their places with
 // one atomic; tiles without an invalid base roll their k-mers (tile_kmers_run)
@@ -219,14 +229,15 @@ __device__ __forceinline__ void extract_short(const BatchView& bv, const SeedPar
     unsigned long long at = 0;
     if (lane == 0 && total) at = atomicAdd(cur, (unsigned long long)total);
     at = __shfl_sync(kFull, at, 0);
-    if (at + total > sg.key_cap) {
-      if (lane == 0) {
-        atomicAdd(cur, 0ull - total);
-        atomicOr(sg.err, kErrOffsets);
-      }
-      continue;
-    }
     dst += at;
+    const uint64_t* end = dst + total;
+    if (at + total > sg.key_cap) {
+      // The list is full: the keys that still fit, tile by tile as below.
+      if (lane == 0) list_is_full(cur, sg);
+      if (at >= sg.key_cap) continue;
+      end = dst + (sg.key_cap - at);
+      whole = 0;
+    }
     for (uint32_t j = 0; j < m; ++j) {
       const uint64_t p = __shfl_sync(kFull, first, j);
       const uint32_t w = __shfl_sync(kFull, nw, j);
@@ -249,7 +260,8 @@ __device__ __forceinline__ void extract_short(const BatchView& bv, const SeedPar
         uint64_t key = short_canonical(bv.pv, p + i0, n, sp.klen, lane);
         if (sp.spaced) key = spaced_canonical(sp.pattern, key);
         const uint32_t ballot = __ballot_sync(kFull, keep);
-        if (keep) dst[__popc(ballot & ((1u << lane) - 1u))] = key;
+        uint64_t* to = dst + __popc(ballot & ((1u << lane) - 1u));
+        if (keep && to < end) *to = key;
         dst += __popc(ballot);
       }
     }
@@ -312,11 +324,8 @@ __global__ void extract_dense_kernel(BatchView bv, SeedParams sp, uint64_t* __re
     if (lane == 0 && n) at = atomicAdd(cur, (unsigned long long)n);
     at = __shfl_sync(0xFFFFFFFFu, at, 0);
     if (at + n > sg.key_cap) {
-      if (lane == 0) {
-        atomicAdd(cur, 0ull - n);
-        atomicOr(sg.err, kErrOffsets);
-      }
-      n = 0;
+      if (lane == 0) list_is_full(cur, sg);
+      n = at < sg.key_cap ? (uint32_t)(sg.key_cap - at) : 0u;
     }
     if constexpr (MODE == 1) {
       const uint32_t* list = reinterpret_cast<const uint32_t*>(wbase);
