@@ -140,3 +140,40 @@ def test_a_full_key_list_has_no_holes(gpu, tmp_path, opts):
             totals.append(int(total))
             assert int(counts.sum()) == 0
         assert min(totals) == max(totals) >= nbases
+
+
+@pytest.mark.parametrize("colors", [12, 270], ids=["narrow", "wide"])
+def test_a_batch_without_memory_leaves_the_index_usable(gpu, oracle, tmp_path, colors):
+    """2^42 bases fit no GPU: ZX_ENOMEM before any base is read, and the calls
+    after it, of sizes seen and not seen before, answer correctly."""
+    import torch
+
+    import zindex_b200 as zx
+
+    fof = make_genomes(tmp_path / "g", colors, 3000, 31)
+    ix = build_index(fof, tmp_path / "index", k=31, H=4, b=8, min_docs=1)
+    genomes = [dna(3000, 31 + c) for c in range(colors)]
+    batches = [zx.pack_records(sample_reads(genomes, np.random.default_rng(n), n, 150))
+               for n in (200, 20, 2000)]
+    dev = torch.device("cuda", 0)
+    with zx.Index(ix) as index:
+        counts = torch.zeros(index.colors, dtype=torch.int64, device=dev)
+        total = torch.zeros(1, dtype=torch.int64, device=dev)
+        offsets = torch.tensor([0, 100], dtype=torch.int64, device=dev)
+        args = (offsets.data_ptr(), 1, counts.data_ptr(), total.data_ptr())
+        seg = np.array([0, 1], dtype=np.uint64)
+        for bases, offs in batches:
+            want, want_total = oracle.query_records(ix, bases, offs)
+            for graph in (False, True):
+                got, got_total = index.query_records(bases, offs)
+                assert got_total == want_total
+                np.testing.assert_array_equal(got, want)
+                with pytest.raises(zx.ZxError) as err:
+                    index.query_device(counts.data_ptr(), 1 << 42, *args, use_graph=graph)
+                assert err.value.code == 4
+                with pytest.raises(zx.ZxError) as err:
+                    index.query_segments(counts.data_ptr(), 1 << 42, *args[:2], seg, *args[2:])
+                assert err.value.code == 4
+            per, totals = index.query_per_record(bases, offs)
+            assert int(totals.sum()) == want_total
+            np.testing.assert_array_equal(per.sum(axis=0, dtype=np.uint64), want)

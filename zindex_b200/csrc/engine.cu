@@ -51,6 +51,22 @@ void dev_alloc(T** p, uint64_t count, const char* what) {
   }
 }
 
+// Frees buffers that are about to be allocated anew. Their pointers are cleared
+// and their capacity is zero until the last allocation has succeeded, so a
+// call that runs out of memory leaves no freed pointer and no half of a group
+// to the next one (which asks for the group's last pointer).
+template <class... T>
+void drop(uint64_t& cap, T*&... p) {
+  cap = 0;
+  ((cudaFree(p), p = nullptr), ...);
+}
+
+template <class... T>
+void drop_host(uint64_t& cap, T*&... p) {
+  cap = 0;
+  ((cudaFreeHost(p), p = nullptr), ...);
+}
+
 template <class T>
 void host_alloc(T** p, uint64_t count) {
   *p = nullptr;
@@ -1309,12 +1325,10 @@ void Engine::set_round_bases(uint64_t bases) {
 void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, bool segmented,
                              uint64_t round_bases) {
   const uint64_t colors = m_.colors.size();
-  if (nbases > ws.cap_bases || !ws.bases) {
+  if (nbases > ws.cap_bases || !ws.invalid) {
     uint64_t cap = std::max<uint64_t>({nbases, ws.cap_bases * 3 / 2, 4096});
     cap = round_up(cap, 4096);
-    if (ws.bases) cudaFree(ws.bases);
-    if (ws.packed) cudaFree(ws.packed);
-    if (ws.invalid) cudaFree(ws.invalid);
+    drop(ws.cap_bases, ws.bases, ws.packed, ws.invalid);
     dev_alloc(&ws.bases, cap + 64, "batch bases");
     dev_alloc(&ws.packed, cap / 32 + 8, "packed bases");
     dev_alloc(&ws.invalid, cap / 32 + 8, "invalid masks");
@@ -1322,12 +1336,9 @@ void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, b
     ws.cap_tiles = 0;
     ws.release_graphs();
   }
-  if (records > ws.cap_records || !ws.offsets) {
+  if (records > ws.cap_records || !ws.scan_tmp) {
     uint64_t cap = std::max<uint64_t>({records, ws.cap_records * 3 / 2, 1024});
-    if (ws.offsets) cudaFree(ws.offsets);
-    if (ws.tile_counts) cudaFree(ws.tile_counts);
-    if (ws.tile_first) cudaFree(ws.tile_first);
-    if (ws.scan_tmp) cudaFree(ws.scan_tmp);
+    drop(ws.cap_records, ws.offsets, ws.tile_counts, ws.tile_first, ws.scan_tmp);
     dev_alloc(&ws.offsets, cap + 1, "record offsets");
     dev_alloc(&ws.tile_counts, cap + 1, "tile counts");
     dev_alloc(&ws.tile_first, cap + 1, "tile offsets");
@@ -1342,7 +1353,7 @@ void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, b
   uint64_t tiles = ws.cap_bases / kTileWindows + ws.cap_bases / kFindereTask + ws.cap_records +
                    kSmallTiles + 16;
   if (tiles > ws.cap_tiles) {
-    if (ws.tiles) cudaFree(ws.tiles);
+    drop(ws.cap_tiles, ws.tiles);
     dev_alloc(&ws.tiles, tiles, "tiles");
     ws.cap_tiles = tiles;
     ws.release_graphs();
@@ -1350,7 +1361,7 @@ void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, b
   if (m_.index_mode == kFindere && !findere_dense_) {
     const uint64_t need = (uint64_t)max_blocks(launch_) * launch_.warps * 2 * std::max<uint64_t>(colors, 1);
     if (need > ws.cap_fstate) {
-      if (ws.fstate) cudaFree(ws.fstate);
+      drop(ws.cap_fstate, ws.fstate);
       dev_alloc(&ws.fstate, need, "findere colour state");
       ws.cap_fstate = need;
       ws.release_graphs();
@@ -1358,20 +1369,19 @@ void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, b
   }
   uint64_t partial = (uint64_t)max_blocks(run_launch(launch_)) * colors;
   if (partial > ws.cap_partial) {
-    if (ws.partial) cudaFree(ws.partial);
+    drop(ws.cap_partial, ws.partial);
     dev_alloc(&ws.partial, partial, "block counters");
     ws.cap_partial = partial;
     ws.release_graphs();
   }
-  if (colors > ws.cap_colors || !ws.counts) {
-    if (ws.counts) cudaFree(ws.counts);
-    if (ws.total) cudaFree(ws.total);
+  if (!ws.error) {
+    dev_alloc(&ws.error, 1, "error word");
+    cuda_check(cudaMemset(ws.error, 0, 4), "memset");
+  }
+  if (colors > ws.cap_colors || !ws.total) {
+    drop(ws.cap_colors, ws.counts, ws.total);
     dev_alloc(&ws.counts, colors, "counts");
     dev_alloc(&ws.total, 1, "total");
-    if (!ws.error) {
-      dev_alloc(&ws.error, 1, "error word");
-      cuda_check(cudaMemset(ws.error, 0, 4), "memset");
-    }
     ws.cap_colors = colors;
     ws.release_graphs();
   }
@@ -1392,32 +1402,28 @@ void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, b
 
 void Engine::ensure_host_capacity(Workspace& ws, uint64_t nbases, uint64_t records) {
   if (nbases > ws.cap_h_bases || !ws.h_bases) {
-    if (ws.h_bases) cudaFreeHost(ws.h_bases);
     uint64_t cap = round_up(std::max<uint64_t>({nbases, ws.cap_h_bases * 3 / 2, 4096}), 4096);
+    drop_host(ws.cap_h_bases, ws.h_bases);
     host_alloc(&ws.h_bases, cap);
     ws.cap_h_bases = cap;
   }
   if (records + 1 > ws.cap_h_records || !ws.h_offsets) {
-    if (ws.h_offsets) cudaFreeHost(ws.h_offsets);
     uint64_t cap = std::max<uint64_t>({records + 1, ws.cap_h_records * 3 / 2, 1024});
+    drop_host(ws.cap_h_records, ws.h_offsets);
     host_alloc(&ws.h_offsets, cap);
     ws.cap_h_records = cap;
   }
-  if (!ws.h_counts) {
-    host_alloc(&ws.h_counts, std::max<uint64_t>(m_.colors.size(), 1));
-    host_alloc(&ws.h_total, 1);
-  }
+  if (!ws.h_counts) host_alloc(&ws.h_counts, std::max<uint64_t>(m_.colors.size(), 1));
+  if (!ws.h_total) host_alloc(&ws.h_total, 1);
 }
 
 void Engine::compress_homopolymers(Workspace& ws, const uint8_t*& bases, uint64_t nbases,
                                    const uint64_t*& offsets, uint64_t records, cudaStream_t s) {
   check(nbases < (1ull << 31) - 1, kEInval,
         "homopolymer-compressed queries take batches below 2^31 bases: split the batch");
-  if (nbases > ws.cap_hp_bases || !ws.hp_bases) {
+  if (nbases > ws.cap_hp_bases || !ws.hp_scan_tmp) {
     const uint64_t cap = round_up(std::max<uint64_t>({nbases, ws.cap_hp_bases * 3 / 2, 4096}), 4096);
-    for (void* p : {(void*)ws.hp_starts, (void*)ws.hp_keep, (void*)ws.hp_pos, (void*)ws.hp_bases,
-                    ws.hp_scan_tmp})
-      if (p) cudaFree(p);
+    drop(ws.cap_hp_bases, ws.hp_starts, ws.hp_keep, ws.hp_pos, ws.hp_bases, ws.hp_scan_tmp);
     dev_alloc(&ws.hp_starts, cap / 32 + 2, "homopolymer record starts");
     dev_alloc(&ws.hp_keep, cap + 1, "homopolymer flags");
     dev_alloc(&ws.hp_pos, cap + 1, "homopolymer positions");
@@ -1432,7 +1438,7 @@ void Engine::compress_homopolymers(Workspace& ws, const uint8_t*& bases, uint64_
   }
   if (records + 1 > ws.cap_hp_records || !ws.hp_offsets) {
     const uint64_t cap = std::max<uint64_t>({records + 1, ws.cap_hp_records * 3 / 2, 1024});
-    if (ws.hp_offsets) cudaFree(ws.hp_offsets);
+    drop(ws.cap_hp_records, ws.hp_offsets);
     dev_alloc(&ws.hp_offsets, cap, "compressed offsets");
     ws.cap_hp_records = cap;
     ws.release_graphs();
@@ -1765,6 +1771,9 @@ void Engine::run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv,
 void Engine::ensure_order_capacity(Workspace& ws, int b, bool whole) {
   if (!ws.wide_hist[b]) {
     dev_alloc(&ws.wide_hist[b], order_.buckets() + 4ull, "round order buckets");
+    ws.release_graphs();
+  }
+  if (!ws.wide_next[b]) {
     dev_alloc(&ws.wide_next[b], order_.buckets(), "round order places");
     ws.release_graphs();
   }
@@ -1807,23 +1816,17 @@ bool Engine::ensure_round_capacity(Workspace& ws, uint64_t keys) {
 }
 
 void Engine::ensure_strobe_capacity(Workspace& ws, uint64_t nbases, uint64_t tiles) {
-  if (nbases > ws.cap_strobe_bases || !ws.strobe_anchors) {
+  if (nbases > ws.cap_strobe_bases || !ws.strobe_hashes) {
     const uint64_t cap = std::max<uint64_t>({nbases, ws.cap_strobe_bases * 3 / 2, 4096});
-    if (ws.strobe_anchors) cudaFree(ws.strobe_anchors);
-    if (ws.strobe_hashes) cudaFree(ws.strobe_hashes);
-    ws.strobe_anchors = nullptr;
-    ws.strobe_hashes = nullptr;
+    drop(ws.cap_strobe_bases, ws.strobe_anchors, ws.strobe_hashes);
     dev_alloc(&ws.strobe_anchors, cap / 32 + 2, "strobe candidates");
     dev_alloc(&ws.strobe_hashes, cap + 1, "strobe hashes");
     ws.cap_strobe_bases = cap;
     ws.release_graphs();
   }
-  if (tiles > ws.cap_strobe_tiles || !ws.strobe_slots) {
+  if (tiles > ws.cap_strobe_tiles || !ws.strobe_count) {
     const uint64_t cap = std::max<uint64_t>({tiles, ws.cap_strobe_tiles * 3 / 2, 1024});
-    if (ws.strobe_slots) cudaFree(ws.strobe_slots);
-    if (ws.strobe_count) cudaFree(ws.strobe_count);
-    ws.strobe_slots = nullptr;
-    ws.strobe_count = nullptr;
+    drop(ws.cap_strobe_tiles, ws.strobe_slots, ws.strobe_count);
     dev_alloc(&ws.strobe_slots, cap * kStrobeSlot, "strobe seeds");
     dev_alloc(&ws.strobe_count, cap, "strobe seed counts");
     ws.cap_strobe_tiles = cap;
@@ -1852,15 +1855,11 @@ void Engine::link_strobes(Workspace& ws, const BatchView& bv, uint64_t nbases, c
 }
 
 void Engine::ensure_segment_capacity(Workspace& ws, uint32_t segments) {
-  if (segments + 1 > ws.cap_segments || !ws.seg_blocks) {
+  if (segments + 1 > ws.cap_segments || !ws.h_seg_records) {
     const uint64_t c = std::max<uint64_t>(segments + 1, 256);
-    for (void* p : {(void*)ws.seg_blocks, (void*)ws.seg_tiles, (void*)ws.seg_records,
-                    (void*)ws.wide_seg_cursor, (void*)ws.wide_round_first})
-      if (p) cudaFree(p);
-    for (void* p : {(void*)ws.h_seg_blocks, (void*)ws.h_seg_records})
-      if (p) cudaFreeHost(p);
-    ws.wide_seg_cursor = nullptr;
-    ws.wide_round_first = nullptr;
+    drop(ws.cap_segments, ws.seg_blocks, ws.seg_tiles, ws.seg_records, ws.wide_seg_cursor,
+         ws.wide_round_first);
+    drop_host(ws.cap_segments, ws.h_seg_blocks, ws.h_seg_records);
     dev_alloc(&ws.seg_blocks, c, "segment blocks");
     dev_alloc(&ws.seg_tiles, c, "segment tiles");
     dev_alloc(&ws.seg_records, c, "segment records");
@@ -1868,27 +1867,31 @@ void Engine::ensure_segment_capacity(Workspace& ws, uint32_t segments) {
     host_alloc(&ws.h_seg_records, c);
     ws.cap_segments = c;
   }
-  if (wide_form(launch_) && !ws.wide_seg_cursor) {
-    dev_alloc(&ws.wide_seg_cursor, 2 * ws.cap_segments, "segment key cursors");
-    dev_alloc(&ws.wide_round_first, 2 * ws.cap_segments, "segment probe rounds");
+  if (wide_form(launch_)) {
+    if (!ws.wide_seg_cursor)
+      dev_alloc(&ws.wide_seg_cursor, 2 * ws.cap_segments, "segment key cursors");
+    if (!ws.wide_round_first)
+      dev_alloc(&ws.wide_round_first, 2 * ws.cap_segments, "segment probe rounds");
   }
   if (!ws.seg_staged)
     cuda_check(cudaEventCreateWithFlags(&ws.seg_staged, cudaEventDisableTiming), "cudaEventCreate");
 }
 
 void Engine::ensure_wide_pipeline(Workspace& ws) {
-  if (ws.aux_stream) return;
-  dev_alloc(&ws.wide_keys2, kSplitTiles * kTileWindows, "second dense key list");
-  cuda_check(cudaStreamCreateWithFlags(&ws.aux_stream, cudaStreamNonBlocking), "cudaStreamCreate");
+  if (ws.wide_probe[1]) return;  // (created last)
+  if (!ws.wide_keys2)
+    dev_alloc(&ws.wide_keys2, kSplitTiles * kTileWindows, "second dense key list");
+  if (!ws.aux_stream)
+    cuda_check(cudaStreamCreateWithFlags(&ws.aux_stream, cudaStreamNonBlocking), "cudaStreamCreate");
   for (cudaEvent_t* e : {&ws.wide_fork, &ws.wide_ext[0], &ws.wide_ext[1], &ws.wide_probe[0],
                          &ws.wide_probe[1]})
-    cuda_check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate");
+    if (!*e) cuda_check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate");
   ws.release_graphs();
 }
 
 void Engine::ensure_split_capacity(Workspace& ws) {
-  if (ws.split_keys) return;
-  dev_alloc(&ws.split_keys, kSplitTiles * kTileWindows, "split key slots");
+  if (ws.split_counts) return;
+  if (!ws.split_keys) dev_alloc(&ws.split_keys, kSplitTiles * kTileWindows, "split key slots");
   dev_alloc(&ws.split_counts, kSplitTiles, "split key counts");
   ws.release_graphs();
 }
@@ -1980,14 +1983,14 @@ void Engine::query_segments(Workspace& ws, const uint8_t* bases, uint64_t nbases
   ws.h_seg_records[segments] = seg_records[segments];
   const uint64_t colors = m_.colors.size();
   if (l.smem_counters && (uint64_t)blocks * colors > ws.cap_partial) {
-    if (ws.partial) cudaFree(ws.partial);
+    drop(ws.cap_partial, ws.partial);
     dev_alloc(&ws.partial, (uint64_t)blocks * colors, "block counters");
     ws.cap_partial = (uint64_t)blocks * colors;
     ws.release_graphs();
   }
   if (m_.index_mode == kFindere && !findere_dense_ &&
       (uint64_t)blocks * wpb * 2 * colors > ws.cap_fstate) {
-    if (ws.fstate) cudaFree(ws.fstate);
+    drop(ws.cap_fstate, ws.fstate);
     dev_alloc(&ws.fstate, (uint64_t)blocks * wpb * 2 * colors, "findere colour state");
     ws.cap_fstate = (uint64_t)blocks * wpb * 2 * colors;
     ws.release_graphs();
@@ -2062,14 +2065,9 @@ void Engine::record_groups(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   // 8 bytes per base (64 Mi bases).
   const bool strobes = sp_.strobe_max != 0;
   const uint64_t group_bases = strobes ? (64ull << 20) : (256ull << 20);
-  if (gmax > ws.cap_rec_totals || !ws.rec_counts) {
-    for (void* p : {(void*)ws.rec_counts, (void*)ws.rec_totals, (void*)ws.rec_hits,
-                    (void*)ws.rec_first, ws.rec_scan_tmp})
-      if (p) cudaFree(p);
-    ws.rec_counts = nullptr;
-    ws.rec_totals = nullptr;
-    ws.rec_hits = ws.rec_first = nullptr;
-    ws.rec_scan_tmp = nullptr;
+  if (gmax > ws.cap_rec_totals || !ws.rec_scan_tmp) {
+    drop(ws.cap_rec_totals, ws.rec_counts, ws.rec_totals, ws.rec_hits, ws.rec_first,
+         ws.rec_scan_tmp);
     dev_alloc(&ws.rec_counts, gmax * colors, "record counters");
     dev_alloc(&ws.rec_totals, gmax, "record totals");
     dev_alloc(&ws.rec_hits, gmax + 1, "record hit counts");
@@ -2174,21 +2172,20 @@ void Engine::query_per_record(Workspace& ws, const uint8_t* bases, uint64_t nbas
 void Engine::ensure_strand_capacity(Workspace& ws, uint64_t nbases, uint64_t records) {
   const uint64_t counts = records * std::max<uint64_t>(m_.colors.size(), 1);
   if (nbases > ws.cap_strand_bases || !ws.strand_bases) {
-    if (ws.strand_bases) cudaFree(ws.strand_bases);
-    ws.strand_bases = nullptr;
     const uint64_t cap = std::max<uint64_t>({nbases, ws.cap_strand_bases * 3 / 2, 4096});
+    drop(ws.cap_strand_bases, ws.strand_bases);
     dev_alloc(&ws.strand_bases, cap + 64, "reverse strands");
     ws.cap_strand_bases = cap;
   }
-  if (counts > ws.cap_strand_counts || records > ws.cap_strand_records || !ws.strand_counts) {
-    for (void* p : {(void*)ws.strand_counts, (void*)ws.strand_totals})
-      if (p) cudaFree(p);
-    ws.strand_counts = nullptr;
-    ws.strand_totals = nullptr;
-    ws.cap_strand_counts = std::max(counts, ws.cap_strand_counts);
-    ws.cap_strand_records = std::max(records, ws.cap_strand_records);
-    dev_alloc(&ws.strand_counts, ws.cap_strand_counts, "reverse strand counters");
-    dev_alloc(&ws.strand_totals, ws.cap_strand_records, "reverse strand totals");
+  if (counts > ws.cap_strand_counts || !ws.strand_counts) {
+    drop(ws.cap_strand_counts, ws.strand_counts);
+    dev_alloc(&ws.strand_counts, counts, "reverse strand counters");
+    ws.cap_strand_counts = counts;
+  }
+  if (records > ws.cap_strand_records || !ws.strand_totals) {
+    drop(ws.cap_strand_records, ws.strand_totals);
+    dev_alloc(&ws.strand_totals, records, "reverse strand totals");
+    ws.cap_strand_records = records;
   }
 }
 
@@ -2239,12 +2236,9 @@ void Engine::query_record_hits(Workspace& ws, const uint8_t* bases, uint64_t nba
     uint64_t hits = 0;
     cuda_check(cudaMemcpyAsync(&hits, ws.rec_first + n, 8, cudaMemcpyDeviceToHost, s), "D2H");
     cuda_check(cudaStreamSynchronize(s), "per-record hits");
-    if (hits > ws.cap_hits || !ws.hit_colors) {
-      if (ws.hit_colors) cudaFree(ws.hit_colors);
-      if (ws.hit_counts) cudaFree(ws.hit_counts);
-      ws.hit_colors = nullptr;
-      ws.hit_counts = nullptr;
+    if (hits > ws.cap_hits || !ws.hit_counts) {
       const uint64_t cap = std::max<uint64_t>({hits, ws.cap_hits * 3 / 2, 4096});
+      drop(ws.cap_hits, ws.hit_colors, ws.hit_counts);
       dev_alloc(&ws.hit_colors, cap, "record hits");
       dev_alloc(&ws.hit_counts, cap, "record hit counts");
       ws.cap_hits = cap;
@@ -2560,8 +2554,7 @@ void Engine::extract_host(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   }
   uint64_t need = (uint64_t)ntiles * kTileWindows;
   if (need > ws.cap_keys) {
-    if (ws.keys_out) cudaFree(ws.keys_out);
-    if (ws.keys_count) cudaFree(ws.keys_count);
+    drop(ws.cap_keys, ws.keys_out, ws.keys_count);
     dev_alloc(&ws.keys_out, need, "extracted keys");
     dev_alloc(&ws.keys_count, ntiles, "extracted counts");
     ws.cap_keys = need;
