@@ -177,3 +177,53 @@ def test_a_batch_without_memory_leaves_the_index_usable(gpu, oracle, tmp_path, c
             per, totals = index.query_per_record(bases, offs)
             assert int(totals.sum()) == want_total
             np.testing.assert_array_equal(per.sum(axis=0, dtype=np.uint64), want)
+
+
+def test_many_hash_partitions_keep_the_bucket_table_small(gpu, oracle, tmp_path):
+    """8,192 partitions: sorted by the first hash alone, in 2^16 buckets. One
+    read takes no more than ten times its unsorted time (with the partitions in
+    the key it was 2^23 buckets, walked by one block in every call)."""
+    import subprocess
+
+    import torch
+
+    import zindex_b200 as zx
+
+    subprocess.run([str(helpers.ZX_BUILD), "--synth", "uniform:128:40000:40000:5", "-o",
+                    str(tmp_path / "index"), "-q", "-k", "31", "-H", "2", "-b", "16", "-L", "4",
+                    "-X", "2KiB"], check=True)
+    genomes = [dna(40000, 5 + c) for c in range(128)]
+    rng = np.random.default_rng(14)
+    dev = torch.device("cuda", 0)
+    with zx.Index(tmp_path / "index") as index:
+        assert index.info.banks == 8192 and index.launch()["wide"]
+        for reads in (1, 300, 20000):
+            bases, offsets = zx.pack_records(sample_reads(genomes, rng, reads, 150))
+            want, want_total = oracle.query_records(tmp_path / "index", bases, offsets)
+            got, total = index.query_records(bases, offsets)
+            assert total == want_total
+            np.testing.assert_array_equal(got, want)
+        d_b = torch.from_numpy(np.frombuffer(genomes[7][:150], dtype=np.uint8).copy()).to(dev)
+        d_off = torch.tensor([0, 150], dtype=torch.int64, device=dev)
+        counts = torch.zeros(128, dtype=torch.int64, device=dev)
+        n = torch.zeros(1, dtype=torch.int64, device=dev)
+        stream = torch.cuda.current_stream(dev).cuda_stream
+
+        def micros():
+            best = float("inf")
+            for _ in range(20):
+                first, last = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+                first.record()
+                for _ in range(50):
+                    index.query_device(d_b.data_ptr(), 150, d_off.data_ptr(), 1,
+                                       counts.data_ptr(), n.data_ptr(), stream)
+                last.record()
+                last.synchronize()
+                best = min(best, first.elapsed_time(last) * 20)
+            return best
+
+        sorted_us = micros()
+        index.set_launch(wide=1, order=0)
+        plain_us = micros()
+        print(f"one read: {sorted_us:.1f} us sorted, {plain_us:.1f} us unsorted")
+        assert sorted_us < 10 * plain_us

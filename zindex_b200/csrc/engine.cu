@@ -977,6 +977,9 @@ void Engine::plan_windows() {
   // block counts in shared memory, where that leaves every class slices of
   // eight chunks or what finer buckets would leave it (half the slice width
   // costs the probe a tenth; counting 1.2e8 keys in L2 takes 1.1 ms more).
+  // Where more than 2^8 partitions would still need more than 2^18: no
+  // windows, and the rounds are sorted by 2^16 values of the first hash alone,
+  // which gives the wide probe its neighbours.
   order_.fbits = 10;
   while (order_.fbits + pbits < kMaxOrderBits && (1ull << order_.fbits) < 2 * most) ++order_.fbits;
   if (order_.fbits + pbits > kLocalOrderBits && pbits < kLocalOrderBits) {
@@ -986,7 +989,12 @@ void Engine::plan_windows() {
       keep &= widest(host_ix_.cls[c], coarse) >= std::min(3, widest(host_ix_.cls[c], order_.fbits));
     if (keep) order_.fbits = coarse;
   }
-  if (order_.fbits + pbits > kMaxOrderBits || !wide_eligible(8)) return;
+  if (order_.fbits + pbits > kMaxOrderBits) {
+    order_.parts = 1;
+    order_.fbits = 16;
+    return;
+  }
+  if (!wide_eligible(8)) return;
 
   // Slices of every class: as wide as fits, the remainder cut where the sum
   // of (width + 4) per slice is least (4: a slice's own hashing of a seed, in
