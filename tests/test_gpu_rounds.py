@@ -227,3 +227,42 @@ def test_many_hash_partitions_keep_the_bucket_table_small(gpu, oracle, tmp_path)
         plain_us = micros()
         print(f"one read: {sorted_us:.1f} us sorted, {plain_us:.1f} us unsorted")
         assert sorted_us < 10 * plain_us
+
+
+def test_dense_batches_of_grouped_colours(gpu, oracle, tmp_path):
+    """Narrow rows can hold many colours through multi-member groups: with six
+    classes and 32 hashes the probe's row table leaves no shared memory for
+    9,600 colour counters."""
+    import zindex_b200 as zx
+
+    per_class, members = 1600, 50
+    lengths = [60, 120, 240, 480, 960, 1920]
+    (tmp_path / "g").mkdir()
+    lines, groups = [], []
+    for i, n in enumerate(lengths):
+        first = i * per_class
+        for c in range(first, first + per_class):
+            p = tmp_path / "g" / f"g{c}.fa"
+            helpers.write_fasta(p, [dna(n, 31 + c)])
+            lines.append(f"g{c}\t{p}")
+        groups += [",".join(map(str, range(a, a + members)))
+                   for a in range(first, first + per_class, members)]
+    (tmp_path / "fof.tsv").write_text("\n".join(lines) + "\n")
+    ix = build_index(tmp_path / "fof.tsv", tmp_path / "index", k=31, H=32, b=8, seg=16, min_docs=1,
+                     groups=";".join(groups))
+    rng = np.random.default_rng(15)
+    genomes = [dna(960, 31 + int(c)) for c in rng.integers(4 * per_class, 5 * per_class, 200)]
+    reads = sample_reads(genomes, rng, 300, 150)
+    # (Past 1 MiB by bases that are no seeds.)
+    bases, offsets = zx.pack_records([r + b"N" * 3500 for r in reads])
+    assert len(bases) > 1 << 20
+    want, want_total = oracle.query_records(ix, bases, offsets)
+    with zx.Index(ix) as index:
+        assert not index.launch()["wide"] and index.info.classes == 6
+        got, total = index.query_records(bases, offsets)
+        assert total == want_total
+        np.testing.assert_array_equal(got, want)
+        index.set_launch(blocks=1000)  # no longer the default: the fused kernel
+        got, total = index.query_records(bases, offsets)
+        assert total == want_total
+        np.testing.assert_array_equal(got, want)

@@ -1172,6 +1172,8 @@ QueryLaunch Engine::dense_launch() const {
   l.order = 1;
   l.warps = 4;
   l.smem_counters = 1;
+  // (As in default_launch: narrow rows of multi-member groups hold many colours.)
+  if (m_.colors.size() > 16384 || fused_smem_bytes(l) > 110 * 1024) l.smem_counters = 0;
   return l;
 }
 
