@@ -116,3 +116,33 @@ def test_strobe_indexes_refuse_single_strand_device_paths(gpu, tmp_path_factory)
         with pytest.raises(zx.ZxError):
             index.query_device(d_bases.data_ptr(), 100, d_off.data_ptr(), 1, d_counts.data_ptr(),
                                d_total.data_ptr())
+
+
+def test_link_time_does_not_grow_with_the_distance(gpu, oracle, tmp_path_factory):
+    """A candidate's search ends at the first partner without a differing bit:
+    up to 60,000 bases downstream takes no more than three times the time of
+    up to 2,000 (a search to the end would be twenty times the compares)."""
+    import time
+
+    import zindex_b200 as zx
+
+    best = {}
+    for hi in (2000, 60000):
+        ix, genomes = strobe_index(tmp_path_factory, k=21, hi=hi)
+        rng = np.random.default_rng(7)
+        reads = [dna(100_000, int(s)) for s in rng.integers(0, 1 << 62, 40)]
+        reads[0] = (genomes[0] + genomes[1]) * 4
+        bases, offsets = zx.pack_records(reads)
+        with zx.Index(ix) as index:
+            short, short_offsets = zx.pack_records(reads[:1])
+            got, total = index.query_records(short, short_offsets)
+            want, want_total = oracle.query_records(ix, short, short_offsets)
+            assert total == want_total
+            np.testing.assert_array_equal(got, want)
+            best[hi] = float("inf")
+            for _ in range(8):
+                start = time.perf_counter()
+                index.query_records(bases, offsets)
+                best[hi] = min(best[hi], time.perf_counter() - start)
+    print({hi: f"{s * 1e3:.2f} ms" for hi, s in best.items()})
+    assert best[60000] < 3 * best[2000]
