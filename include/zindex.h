@@ -209,9 +209,12 @@ int zx_default_fused_launch(const zx_index* index, zx_launch* out);
 
 /* Most bases of an unsegmented batch whose seeds are sorted and probed as one
  * list (0: the default and the most, 2^28). The lists hold 16 to 20 bytes per
- * base of the largest such batch until the index is closed; this call gives
- * them back. A larger batch takes several rounds of 2^18 tiles (the wide-row
- * form) or the fused kernel. Never changes results. */
+ * base of the largest such batch, in at most an eighth of the device memory
+ * that is free when they are allocated, until the index is closed, another
+ * buffer of it needs their memory, or this call gives them back. A batch
+ * without lists takes several rounds of 2^18 tiles (the wide-row form) or the
+ * fused kernel. Never changes results. Graphs that a caller captured hold the
+ * index's buffers: capture them anew after this call. */
 int zx_set_round_bases(zx_index* index, uint64_t bases);
 
 /* Status of the asynchronous zx_query_device / zx_query_device_noalloc calls

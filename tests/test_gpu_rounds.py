@@ -266,3 +266,68 @@ def test_dense_batches_of_grouped_colours(gpu, oracle, tmp_path):
         got, total = index.query_records(bases, offsets)
         assert total == want_total
         np.testing.assert_array_equal(got, want)
+
+
+def test_key_lists_come_and_go_with_the_memory(gpu, oracle, tmp_path):
+    """Key lists are held while there is room for them: not while 1.4 GB are
+    free, again once the memory is back, and no longer when another buffer of
+    the index needs theirs."""
+    import torch
+
+    import zindex_b200 as zx
+
+    fof = make_genomes(tmp_path / "g", 260, 3000, 31)
+    ix = build_index(fof, tmp_path / "index", k=31, H=4, b=8, min_docs=1)
+    genomes = [dna(3000, 31 + c) for c in range(260)]
+    rng = np.random.default_rng(16)
+    reads = sample_reads(genomes, rng, 2000, 150)
+    few = zx.pack_records(reads[:50])
+    # (20 million bases, most of them no seeds: lists of 400 MB.)
+    bases, offsets = zx.pack_records([r + b"N" * (10_000 - len(r)) for r in reads])
+    want, want_total = oracle.query_records(ix, bases, offsets)
+    per_want = [oracle.query_records(ix, few[0][i * 150:(i + 1) * 150],
+                                     np.array([0, 150], dtype=np.uint64))[0] for i in range(50)]
+    dev = torch.device("cuda", 0)
+    d_b = torch.from_numpy(bases).to(dev)
+    d_off = torch.from_numpy(offsets.view(np.int64)).to(dev)
+    counts = torch.zeros(260, dtype=torch.int64, device=dev)
+    total = torch.zeros(1, dtype=torch.int64, device=dev)
+
+    def free():
+        torch.cuda.synchronize(dev)
+        torch.cuda.empty_cache()
+        return torch.cuda.mem_get_info(dev)[0]
+
+    def fill(leave):
+        return torch.empty(free() - leave, dtype=torch.uint8, device=dev)
+
+    with zx.Index(ix) as index:
+        assert index.launch()["wide"]
+
+        def query():
+            counts.zero_()
+            total.zero_()
+            index.query_device(d_b.data_ptr(), len(bases), d_off.data_ptr(), len(reads),
+                               counts.data_ptr(), total.data_ptr(), use_graph=False)
+            torch.cuda.synchronize(dev)
+            assert int(total) == want_total
+            np.testing.assert_array_equal(counts.cpu().numpy().view(np.uint64), want)
+
+        index.query_records(*few)
+        filler = fill(1400 << 20)
+        query()  # in rounds
+        query()
+        del filler
+        before = free()
+        query()
+        assert before - free() > 350 << 20
+        before = free()
+        query()
+        assert free() == before
+        filler = fill(100 << 20)
+        per, totals = index.query_per_record(*few)  # 256 MiB of counters
+        np.testing.assert_array_equal(per, np.array(per_want))
+        query()  # in rounds again
+        del filler
+        assert free() > before
+        query()

@@ -1323,17 +1323,23 @@ std::unique_ptr<Workspace> Engine::make_workspace() {
 void Engine::set_round_bases(uint64_t bases) {
   cuda_check(cudaSetDevice(device_), "cudaSetDevice");
   round_bases_ = bases ? std::min(bases, kRoundKeys) : kRoundKeys;
+  give_back_lists();
+}
+
+bool Engine::give_back_lists() {
+  if (!ws_ || !ws_->cap_round_keys) return false;
   ws_->release_graphs();
-  for (uint64_t*& p : ws_->round_keys) {
-    if (p) cudaFree(p);
-    p = nullptr;
-  }
-  ws_->cap_round_keys = 0;
-  ws_->round_refused = ~0ull;
+  drop(ws_->cap_round_keys, ws_->round_keys[0], ws_->round_keys[1]);
+  return true;
 }
 
 void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, bool segmented,
-                             uint64_t round_bases) {
+                             uint64_t round_bases, bool may_allocate) {
+  fit([&] { size_buffers(ws, nbases, records, segmented, round_bases, may_allocate); });
+}
+
+void Engine::size_buffers(Workspace& ws, uint64_t nbases, uint64_t records, bool segmented,
+                          uint64_t round_bases, bool may_allocate) {
   const uint64_t colors = m_.colors.size();
   if (nbases > ws.cap_bases || !ws.invalid) {
     uint64_t cap = std::max<uint64_t>({nbases, ws.cap_bases * 3 / 2, 4096});
@@ -1399,7 +1405,8 @@ void Engine::ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, b
   const uint64_t at_once = std::min(nbases, round_bases);
   const bool dense = !segmented && dense_batch(at_once);
   const bool wide = wide_form(launch_) || dense;
-  const bool whole = wide && !segmented && ensure_round_capacity(ws, at_once);
+  const bool whole = wide && !segmented &&
+                     (may_allocate ? ensure_round_lists(ws, at_once) : round_lists(ws, at_once));
   if (kernel_mode(launch_) == 4 || (wide_form(launch_) && !whole)) ensure_split_capacity(ws);
   const bool rounds =
       !whole && wide_form(launch_) && nbases / kTileWindows + records + nbases / kFindereTask + 1 > kSplitTiles;
@@ -1429,6 +1436,25 @@ void Engine::ensure_host_capacity(Workspace& ws, uint64_t nbases, uint64_t recor
 
 void Engine::compress_homopolymers(Workspace& ws, const uint8_t*& bases, uint64_t nbases,
                                    const uint64_t*& offsets, uint64_t records, cudaStream_t s) {
+  fit([&] { ensure_homopolymer_capacity(ws, nbases, records); });
+  const int bgrid = std::max(1, (int)std::min<uint64_t>((nbases + 256) / 256, (uint64_t)sms_ * 16));
+  const int rgrid = std::max(1, (int)std::min<uint64_t>((records + 256) / 256, (uint64_t)sms_ * 16));
+  cuda_check(cudaMemsetAsync(ws.hp_starts, 0, (nbases / 32 + 2) * 4, s), "memset");
+  if (records) hp_mark_starts_kernel<<<rgrid, 256, 0, s>>>(offsets, records, nbases, ws.hp_starts);
+  hp_keep_kernel<<<bgrid, 256, 0, s>>>(bases, nbases, ws.hp_starts, ws.hp_keep);
+  cuda_check(cudaGetLastError(), "hp_keep_kernel");
+  size_t tmp = ws.hp_scan_bytes;
+  cuda_check(cub::DeviceScan::ExclusiveSum(ws.hp_scan_tmp, tmp, ws.hp_keep, ws.hp_pos,
+                                           (int)(nbases + 1), s),
+             "homopolymer scan");
+  hp_compact_kernel<<<bgrid, 256, 0, s>>>(bases, nbases, ws.hp_pos, ws.hp_bases);
+  hp_offsets_kernel<<<rgrid, 256, 0, s>>>(offsets, records, nbases, ws.hp_pos, ws.hp_offsets);
+  cuda_check(cudaGetLastError(), "hp_offsets_kernel");
+  bases = ws.hp_bases;
+  offsets = ws.hp_offsets;
+}
+
+void Engine::ensure_homopolymer_capacity(Workspace& ws, uint64_t nbases, uint64_t records) {
   check(nbases < (1ull << 31) - 1, kEInval,
         "homopolymer-compressed queries take batches below 2^31 bases: split the batch");
   if (nbases > ws.cap_hp_bases || !ws.hp_scan_tmp) {
@@ -1453,21 +1479,6 @@ void Engine::compress_homopolymers(Workspace& ws, const uint8_t*& bases, uint64_
     ws.cap_hp_records = cap;
     ws.release_graphs();
   }
-  const int bgrid = std::max(1, (int)std::min<uint64_t>((nbases + 256) / 256, (uint64_t)sms_ * 16));
-  const int rgrid = std::max(1, (int)std::min<uint64_t>((records + 256) / 256, (uint64_t)sms_ * 16));
-  cuda_check(cudaMemsetAsync(ws.hp_starts, 0, (nbases / 32 + 2) * 4, s), "memset");
-  if (records) hp_mark_starts_kernel<<<rgrid, 256, 0, s>>>(offsets, records, nbases, ws.hp_starts);
-  hp_keep_kernel<<<bgrid, 256, 0, s>>>(bases, nbases, ws.hp_starts, ws.hp_keep);
-  cuda_check(cudaGetLastError(), "hp_keep_kernel");
-  size_t tmp = ws.hp_scan_bytes;
-  cuda_check(cub::DeviceScan::ExclusiveSum(ws.hp_scan_tmp, tmp, ws.hp_keep, ws.hp_pos,
-                                           (int)(nbases + 1), s),
-             "homopolymer scan");
-  hp_compact_kernel<<<bgrid, 256, 0, s>>>(bases, nbases, ws.hp_pos, ws.hp_bases);
-  hp_offsets_kernel<<<rgrid, 256, 0, s>>>(offsets, records, nbases, ws.hp_pos, ws.hp_offsets);
-  cuda_check(cudaGetLastError(), "hp_offsets_kernel");
-  bases = ws.hp_bases;
-  offsets = ws.hp_offsets;
 }
 
 void Engine::plan_tiles(Workspace& ws, const uint64_t* offsets, uint64_t records,
@@ -1500,7 +1511,7 @@ void Engine::enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   // Small batches: one block packs and plans (one launch for pack, count,
   // scan and fill), and with few colours the fused kernel adds into the
   // caller's counters (no reduction launch).
-  const bool dense = dense_batch(nbases) && ensure_round_capacity(ws, nbases);
+  const bool dense = dense_batch(nbases) && round_lists(ws, nbases);
   const bool fused = !wide_form(l) && kernel_mode(l) != 4;
   const bool small = records <= kSmallRecords &&
                      nbases <= (fused ? kSmallBases : wide_form(l) ? kSmallWideBases : 0);
@@ -1644,7 +1655,7 @@ void Engine::run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv,
                                    : (int)std::min<uint64_t>(blocks_cap, std::max<uint64_t>(probe_rounds, 1));
   // One round when its key lists hold every base of the batch; else rounds of
   // kSplitTiles tiles.
-  const bool whole = !segments && ensure_round_capacity(ws, max_keys);
+  const bool whole = !segments && round_lists(ws, max_keys);
   const uint64_t round_tiles = whole ? std::max<uint64_t>(tiles_bound, 1) : kSplitTiles;
   const uint64_t rounds = (tiles_bound + round_tiles - 1) / round_tiles;
   if (!whole) ensure_split_capacity(ws);
@@ -1793,32 +1804,30 @@ void Engine::ensure_order_capacity(Workspace& ws, int b, bool whole) {
   }
 }
 
-bool Engine::ensure_round_capacity(Workspace& ws, uint64_t keys) {
-  if (keys > round_bases_ || keys >= ws.round_refused) return false;
+bool Engine::round_lists(const Workspace& ws, uint64_t keys) const {
   const int lists = launch_.wide && !launch_.order ? 1 : 2;
-  bool have = true;
-  for (int i = 0; i < lists; ++i) have &= ws.round_keys[i] && ws.cap_round_keys >= keys;
-  if (have) return true;
-  // No memory for it: the smaller lists of kSplitTiles tiles a round.
+  return keys <= round_bases_ && ws.cap_round_keys >= keys && ws.round_keys[lists - 1];
+}
+
+bool Engine::ensure_round_lists(Workspace& ws, uint64_t keys) {
+  if (keys > round_bases_) return false;
+  if (round_lists(ws, keys)) return true;
+  const int lists = launch_.wide && !launch_.order ? 1 : 2;
   const uint64_t cap = std::max<uint64_t>(keys + std::min<uint64_t>(keys / 4, 1ull << 24), 1ull << 20);
-  ws.release_graphs();
-  ws.cap_round_keys = 0;
-  for (int i = 0; i < 2; ++i) {
-    if (ws.round_keys[i]) cudaFree(ws.round_keys[i]);
-    ws.round_keys[i] = nullptr;
-  }
-  // (A GiB stays free for what the caller allocates next.)
+  // At most an eighth of the memory that is free without the lists held: the
+  // rest is for what other workspaces and the caller allocate next. (Asked
+  // again by every batch that has no lists.)
   size_t free_b = 0, total_b = 0;
   cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-  const bool room = free_b >= (uint64_t)lists * cap * 8 + (1ull << 30);
+  for (uint64_t* p : ws.round_keys)
+    if (p) free_b += ws.cap_round_keys * 8;
+  if ((uint64_t)lists * cap * 8 > free_b / 8) return false;
+  ws.release_graphs();
+  drop(ws.cap_round_keys, ws.round_keys[0], ws.round_keys[1]);
   for (int i = 0; i < lists; ++i)
-    if (!room || cudaMalloc((void**)&ws.round_keys[i], cap * 8) != cudaSuccess) {
+    if (cudaMalloc((void**)&ws.round_keys[i], cap * 8) != cudaSuccess) {
       cudaGetLastError();
-      for (int j = 0; j < 2; ++j) {
-        if (ws.round_keys[j]) cudaFree(ws.round_keys[j]);
-        ws.round_keys[j] = nullptr;
-      }
-      ws.round_refused = keys;  // (not tried again: the call may be under capture)
+      drop(ws.cap_round_keys, ws.round_keys[0], ws.round_keys[1]);
       return false;
     }
   ws.cap_round_keys = cap;
@@ -1928,7 +1937,7 @@ void Engine::query_segments(Workspace& ws, const uint8_t* bases, uint64_t nbases
   for (uint32_t i = 0; i < segments; ++i)
     check(seg_records[i] <= seg_records[i + 1], kEInval, "segment records must be non-decreasing");
   ensure_capacity(ws, nbases, records, true);
-  ensure_segment_capacity(ws, segments);
+  fit([&] { ensure_segment_capacity(ws, segments); });
   // The pinned staging is reused: wait until the previous call's copies ran.
   cuda_check(cudaEventSynchronize(ws.seg_staged), "segment staging");
   if (wide_form(launch_)) {
@@ -1968,7 +1977,7 @@ void Engine::query_segments(Workspace& ws, const uint8_t* bases, uint64_t nbases
     for (uint32_t i = 0; i < segments; ++i) tiles += est_tiles[i];
     check(tiles <= kSplitTiles, kEInval,
           "a randstrobemer query holds at most 262,144 tiles (about 64 Mbases) per launch");
-    ensure_strobe_capacity(ws, nbases, std::max<uint64_t>(tiles, 1));
+    fit([&] { ensure_strobe_capacity(ws, nbases, std::max<uint64_t>(tiles, 1)); });
   }
   l = run_launch(l);
   const int cap = max_blocks(l);
@@ -1994,14 +2003,14 @@ void Engine::query_segments(Workspace& ws, const uint8_t* bases, uint64_t nbases
   const uint64_t colors = m_.colors.size();
   if (l.smem_counters && (uint64_t)blocks * colors > ws.cap_partial) {
     drop(ws.cap_partial, ws.partial);
-    dev_alloc(&ws.partial, (uint64_t)blocks * colors, "block counters");
+    fit([&] { dev_alloc(&ws.partial, (uint64_t)blocks * colors, "block counters"); });
     ws.cap_partial = (uint64_t)blocks * colors;
     ws.release_graphs();
   }
   if (m_.index_mode == kFindere && !findere_dense_ &&
       (uint64_t)blocks * wpb * 2 * colors > ws.cap_fstate) {
     drop(ws.cap_fstate, ws.fstate);
-    dev_alloc(&ws.fstate, (uint64_t)blocks * wpb * 2 * colors, "findere colour state");
+    fit([&] { dev_alloc(&ws.fstate, (uint64_t)blocks * wpb * 2 * colors, "findere colour state"); });
     ws.cap_fstate = (uint64_t)blocks * wpb * 2 * colors;
     ws.release_graphs();
   }
@@ -2076,16 +2085,18 @@ void Engine::record_groups(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   const bool strobes = sp_.strobe_max != 0;
   const uint64_t group_bases = strobes ? (64ull << 20) : (256ull << 20);
   if (gmax > ws.cap_rec_totals || !ws.rec_scan_tmp) {
-    drop(ws.cap_rec_totals, ws.rec_counts, ws.rec_totals, ws.rec_hits, ws.rec_first,
-         ws.rec_scan_tmp);
-    dev_alloc(&ws.rec_counts, gmax * colors, "record counters");
-    dev_alloc(&ws.rec_totals, gmax, "record totals");
-    dev_alloc(&ws.rec_hits, gmax + 1, "record hit counts");
-    dev_alloc(&ws.rec_first, gmax + 1, "record hit offsets");
-    size_t tmp = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tmp, ws.rec_hits, ws.rec_first, (int)(gmax + 1));
-    dev_alloc((uint8_t**)&ws.rec_scan_tmp, tmp, "record hit scan scratch");
-    ws.rec_scan_bytes = tmp;
+    fit([&] {
+      drop(ws.cap_rec_totals, ws.rec_counts, ws.rec_totals, ws.rec_hits, ws.rec_first,
+           ws.rec_scan_tmp);
+      dev_alloc(&ws.rec_counts, gmax * colors, "record counters");
+      dev_alloc(&ws.rec_totals, gmax, "record totals");
+      dev_alloc(&ws.rec_hits, gmax + 1, "record hit counts");
+      dev_alloc(&ws.rec_first, gmax + 1, "record hit offsets");
+      size_t tmp = 0;
+      cub::DeviceScan::ExclusiveSum(nullptr, tmp, ws.rec_hits, ws.rec_first, (int)(gmax + 1));
+      dev_alloc((uint8_t**)&ws.rec_scan_tmp, tmp, "record hit scan scratch");
+      ws.rec_scan_bytes = tmp;
+    });
     ws.cap_rec_counts = gmax * colors;
     ws.cap_rec_totals = gmax;
   }
@@ -2146,7 +2157,7 @@ void Engine::record_groups(Workspace& ws, const uint8_t* bases, uint64_t nbases,
       // The reverse-complement strand too, and per record and colour the
       // larger count (PreparedRead::new, query_stream.rs:516-534;
       // Scores::score, query_stream.rs:690-701).
-      ensure_strand_capacity(ws, nb, n);
+      fit([&] { ensure_strand_capacity(ws, nb, n); });
       const int bgrid = (int)std::max<uint64_t>(1, std::min<uint64_t>((nb / 16 + 256) / 256, sms_ * 16ull));
       strobe_reverse_kernel<<<bgrid, 256, 0, s>>>(ws.bases, nb, ws.offsets, n, ws.strand_bases);
       cuda_check(cudaGetLastError(), "strobe_reverse_kernel");
@@ -2248,9 +2259,11 @@ void Engine::query_record_hits(Workspace& ws, const uint8_t* bases, uint64_t nba
     cuda_check(cudaStreamSynchronize(s), "per-record hits");
     if (hits > ws.cap_hits || !ws.hit_counts) {
       const uint64_t cap = std::max<uint64_t>({hits, ws.cap_hits * 3 / 2, 4096});
-      drop(ws.cap_hits, ws.hit_colors, ws.hit_counts);
-      dev_alloc(&ws.hit_colors, cap, "record hits");
-      dev_alloc(&ws.hit_counts, cap, "record hit counts");
+      fit([&] {
+        drop(ws.cap_hits, ws.hit_colors, ws.hit_counts);
+        dev_alloc(&ws.hit_colors, cap, "record hits");
+        dev_alloc(&ws.hit_counts, cap, "record hit counts");
+      });
       ws.cap_hits = cap;
     }
     if (hits)
@@ -2323,7 +2336,13 @@ void Engine::query_device(Workspace& ws, const uint8_t* bases, uint64_t nbases,
                           bool use_graph) {
   cuda_check(cudaSetDevice(device_), "cudaSetDevice");
   check_not_strobes();
-  ensure_capacity(ws, nbases, records);
+  // (Lists that the warm-up calls found no memory for are not asked for again
+  // while the caller captures.)
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  const bool free_to_allocate = cudaStreamIsCapturing(s, &capturing) == cudaSuccess &&
+                                capturing == cudaStreamCaptureStatusNone;
+  if (!free_to_allocate) cudaGetLastError();
+  ensure_capacity(ws, nbases, records, false, nbases, free_to_allocate);
   if (!use_graph) {
     enqueue(ws, bases, nbases, offsets, records, recover, counts, total, s);
     return;
@@ -2381,9 +2400,15 @@ void Engine::query_host(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   for (uint64_t c = 0; c < chunks; ++c)
     check(offsets[bounds[c]] <= offsets[bounds[c + 1]] && offsets[bounds[c + 1]] <= nbases, kEInval,
           "offsets must be non-decreasing");
-  uint64_t most = 0;  // bases of the largest chunk
-  for (uint64_t c = 0; c < chunks; ++c)
-    most = std::max(most, offsets[bounds[c + 1]] - offsets[bounds[c]]);
+  // The largest chunk (its bases, its records) and the largest that takes one
+  // key list.
+  uint64_t most = 0, most_records = 0, most_at_once = 0;
+  for (uint64_t c = 0; c < chunks; ++c) {
+    const uint64_t nb = offsets[bounds[c + 1]] - offsets[bounds[c]];
+    most = std::max(most, nb);
+    most_records = std::max(most_records, bounds[c + 1] - bounds[c]);
+    if (nb <= round_bases_) most_at_once = std::max(most_at_once, nb);
+  }
   // Page-locked caller bases are copied directly; pageable ones through the
   // workspace's pinned staging, chunk by chunk.
   auto pinned = [](const void* p) {
@@ -2403,7 +2428,7 @@ void Engine::query_host(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   // Staging pageable memory takes longer than the probes, which then hide
   // behind it chunk by chunk.
   const bool joined = direct && chunks > 1 && nbases <= round_bases_ && (wide_form(launch_) || dense_batch(nbases));
-  ensure_capacity(ws, nbases, records + chunks, false, joined ? nbases : most);
+  ensure_capacity(ws, nbases, records + chunks, false, joined ? nbases : most_at_once);
   ensure_host_capacity(ws, nbases, records + chunks);
   const uint64_t colors = m_.colors.size();
   cudaStream_t s = ws.stream;
@@ -2419,7 +2444,10 @@ void Engine::query_host(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   cuda_check(cudaStreamWaitEvent(ws.copy_stream, ws.chunk_events[0], 0), "cudaStreamWaitEvent");
   cuda_check(cudaMemsetAsync(ws.counts, 0, colors * 8, s), "memset");
   cuda_check(cudaMemsetAsync(ws.total, 0, 8, s), "memset");
-  const bool join = joined && ensure_round_capacity(ws, nbases);
+  // (Sized here, so that nothing takes the lists back between a join's chunks.)
+  if (m_.homopolymer_compression)
+    fit([&] { ensure_homopolymer_capacity(ws, most, most_records); });
+  const bool join = joined && round_lists(ws, nbases);
   const QueryLaunch jl = wide_form(launch_) ? launch_ : dense_launch();
   for (uint64_t c = 0; c < chunks; ++c) {
     const uint64_t r0 = bounds[c], r1 = bounds[c + 1], b0 = offsets[r0], nb = offsets[r1] - b0;
@@ -2483,9 +2511,13 @@ void Engine::query_host_plain(Workspace& ws, const uint8_t* bases, uint64_t nbas
     return;
   }
   check(offsets[0] == 0 && offsets[records] == nbases, kEInval, "offsets must span the bases");
-  for (uint64_t r = 0; r < records; ++r)  // records are sliced on the host here
+  uint64_t most_at_once = 0;  // the largest record that takes one key list
+  for (uint64_t r = 0; r < records; ++r) {  // records are sliced on the host here
     check(offsets[r] <= offsets[r + 1], kEInval, "offsets must be non-decreasing");
-  ensure_capacity(ws, nbases, records);
+    const uint64_t nb = offsets[r + 1] - offsets[r];
+    if (nb <= round_bases_) most_at_once = std::max(most_at_once, nb);
+  }
+  ensure_capacity(ws, nbases, records, false, most_at_once);
   ensure_host_capacity(ws, nbases, records);
   const uint64_t colors = m_.colors.size();
   cudaStream_t s = ws.stream;
@@ -2543,7 +2575,7 @@ void Engine::extract_host(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   }
   if (sp_.strobe_max) {
     // Randstrobemer seeds of the forward strand, records and positions in order.
-    ensure_strobe_capacity(ws, nbases, ntiles);
+    fit([&] { ensure_strobe_capacity(ws, nbases, ntiles); });
     BatchView bv{PackedView{ws.packed, ws.invalid}, d_offsets, ws.tiles, ws.tile_first + records,
                  nullptr};
     link_strobes(ws, bv, nbases, s);
@@ -2564,9 +2596,11 @@ void Engine::extract_host(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   }
   uint64_t need = (uint64_t)ntiles * kTileWindows;
   if (need > ws.cap_keys) {
-    drop(ws.cap_keys, ws.keys_out, ws.keys_count);
-    dev_alloc(&ws.keys_out, need, "extracted keys");
-    dev_alloc(&ws.keys_count, ntiles, "extracted counts");
+    fit([&] {
+      drop(ws.cap_keys, ws.keys_out, ws.keys_count);
+      dev_alloc(&ws.keys_out, need, "extracted keys");
+      dev_alloc(&ws.keys_count, ntiles, "extracted counts");
+    });
     ws.cap_keys = need;
   }
   const int warps = 4;

@@ -12,6 +12,7 @@
 #include <tuple>
 #include <vector>
 
+#include "host/error.h"
 #include "host/manifest.h"
 #include "kernels/device_index.cuh"
 #include "kernels/types.cuh"
@@ -84,7 +85,7 @@ struct Workspace {
   uint32_t* wide_next[2] = {};
   // Wide-row queries of one round: the whole batch's keys, and in order.
   uint64_t* round_keys[2] = {};
-  uint64_t cap_round_keys = 0, round_refused = ~0ull;
+  uint64_t cap_round_keys = 0;
   // Randstrobemer queries: candidate bits and strobe hashes per base, each
   // tile's linked seeds (kStrobeSlot per tile) and their numbers.
   uint32_t* strobe_anchors = nullptr;
@@ -154,6 +155,20 @@ class Engine {
   // Most bases of an unsegmented batch that is sorted and probed as one list
   // (0: kRoundKeys, also the most); the lists held are given back.
   void set_round_bases(uint64_t bases);
+  // The key lists are the one buffer that a query can do without: an
+  // allocation that fails is tried again without them. allocate() starts from
+  // cleared buffers when it is called a second time, and no key list is in
+  // use between two kernels of the caller.
+  template <class F>
+  void fit(F&& allocate) {
+    try {
+      allocate();
+    } catch (const Error& e) {
+      if (e.code != kENoMem || !give_back_lists()) throw;
+      allocate();
+    }
+  }
+  bool give_back_lists();  // false: there were none
   // The fused kernel's default launch (segmented and allocation-free queries
   // run the fused kernel; a wide-row launch maps to it, keeping its cut).
   QueryLaunch default_fused_launch() const;
@@ -275,13 +290,18 @@ class Engine {
   void release();  // frees every device allocation and event of the engine
   // Device buffers of a query of nbases / records (segmented queries do not
   // sort their rounds: no ordered-round buffers).
-  // round_bases: most bases queried at once (a host query's largest chunk).
+  // round_bases: most bases queried at once that one key list may take (a host
+  // query's largest chunk within round_bases_).
+  // may_allocate = false: the key lists are left as they are.
   void ensure_capacity(Workspace& ws, uint64_t nbases, uint64_t records, bool segmented = false,
-                       uint64_t round_bases = ~0ull);
+                       uint64_t round_bases = ~0ull, bool may_allocate = true);
+  void size_buffers(Workspace& ws, uint64_t nbases, uint64_t records, bool segmented,
+                    uint64_t round_bases, bool may_allocate);
   // Homopolymer compression on the device (lib.rs:211-222 per ACGT run):
   // replaces (bases, offsets) by the compressed batch in the workspace.
   void compress_homopolymers(Workspace& ws, const uint8_t*& bases, uint64_t nbases,
                              const uint64_t*& offsets, uint64_t records, cudaStream_t s);
+  void ensure_homopolymer_capacity(Workspace& ws, uint64_t nbases, uint64_t records);
   void ensure_host_capacity(Workspace& ws, uint64_t nbases, uint64_t records);
   void enqueue(Workspace& ws, const uint8_t* bases, uint64_t nbases, const uint64_t* offsets,
                uint64_t records, bool recover, uint64_t* counts, unsigned long long* total,
@@ -299,9 +319,13 @@ class Engine {
   // Ordered wide-row rounds: sort buffers of key list b (0 or 1); whole: the
   // sorted keys go to the round lists.
   void ensure_order_capacity(Workspace& ws, int b, bool whole);
-  // Key lists of a batch in one round (up to round_bases_ keys); false: too many
-  // keys or no memory, and the batch runs in rounds of kSplitTiles tiles.
-  bool ensure_round_capacity(Workspace& ws, uint64_t keys);
+  // Key lists of a batch in one round (up to round_bases_ keys): whether the
+  // workspace holds them, and whether it does after an attempt. Without them
+  // (too many keys, or more than an eighth of the free memory) the batch runs
+  // in rounds of kSplitTiles tiles, or in the fused kernel. Kernels are
+  // enqueued on round_lists alone: nothing is allocated under capture.
+  bool round_lists(const Workspace& ws, uint64_t keys) const;
+  bool ensure_round_lists(Workspace& ws, uint64_t keys);
   // Wide-row form over the planned tiles of a packed batch: rounds of up to
   // kSplitTiles tiles, each a dense extraction and a wide probe. segments = 0:
   // one query into counts / *total; segments > 0: a segmented query, request

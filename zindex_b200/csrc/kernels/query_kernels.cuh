@@ -23,9 +23,10 @@ constexpr uint32_t kFindereTask = 16384;  // src/findere.rs:13-16
 // run lengths in shared memory (8 bytes per colour and warp).
 constexpr uint32_t kFindereSmemColors = 512;
 constexpr uint32_t kSplitTiles = 1u << 18;  // tiles per round of a split minimizer query
-// Keys of a wide-row query in one round (two lists of 8 bytes a key, 4 GiB at
-// most): a batch of up to this many bases has no rounds that might be empty,
-// and its denser buckets copy fewer windows.
+// Keys of a wide-row query in one round, at most (two lists of 8 bytes a key;
+// Engine::ensure_round_lists says when there is memory for them): a batch in
+// one round has no rounds that might be empty, and its denser buckets copy
+// fewer windows.
 constexpr uint64_t kRoundKeys = 1ull << 28;
 // Randstrobemer seeds of a tile (strobes.cuh): its windows' positions plus up
 // to kStrobeExtra minimizer positions past a record's last window start.

@@ -25,8 +25,8 @@
 //   256 random candidates on average, and the run of valid bases is followed
 //   stage by stage, so the time does not grow with strobe_max: 4 Mbases in
 //   records of 100,000, whole call on a B200, 4.6 ms for partners up to 2,000
-//   and 4.7 ms up to 60,000 (108 ms when every lane searched to the end). A tile's seeds go to its slot of kStrobeSlot keys, in position
-//   order.
+//   and 4.7 ms up to 60,000 (108 ms when every lane searched to the end). A
+//   tile's seeds go to its slot of kStrobeSlot keys, in position order.
 //
 // Both strands of a record are scored on the device: strobe_reverse_kernel
 // makes the reverse complements, strobe_best_kernel keeps the larger count.

@@ -53,8 +53,11 @@ Server::Server(Engine& engine, std::mutex& index_mu, const ServerOptions& option
       cuda_check(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming), "cudaEventCreate");
       s.d_bases = s.ws->bases;
       s.d_offsets = s.ws->offsets;
-      s.d_counts = device_array<uint64_t>((uint64_t)opt_.slot_requests * colors_, "counts");
-      s.d_totals = device_array<unsigned long long>(opt_.slot_requests, "totals");
+      engine_.fit([&] {
+        if (!s.d_counts)
+          s.d_counts = device_array<uint64_t>((uint64_t)opt_.slot_requests * colors_, "counts");
+        s.d_totals = device_array<unsigned long long>(opt_.slot_requests, "totals");
+      });
       s.h_offsets = pinned_array<uint64_t>(opt_.slot_records + 1);
       s.h_counts = pinned_array<uint64_t>((uint64_t)opt_.slot_requests * colors_);
       s.h_totals = pinned_array<unsigned long long>(opt_.slot_requests);
