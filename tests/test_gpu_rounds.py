@@ -30,12 +30,14 @@ def test_records_past_and_below_the_round_limit(gpu, oracle, tmp_path):
     want, want_total = oracle.query_records(ix, bases, offsets)
     two, two_offsets = zx.pack_records([long, long[:1_500_000]])
     want_two, want_two_total = oracle.query_records(ix, two, two_offsets)
-    with zx.Index(ix) as index:
-        assert not index.launch()["wide"]
-        index.set_round_bases(2 << 20)
-        got, total = index.query_records(bases, offsets)
-        assert total == want_total
-        np.testing.assert_array_equal(got, want)
+    # (Without a limit: dense chunks on both sides of one that is not.)
+    for limit in (2 << 20, 0):
+        with zx.Index(ix) as index:
+            assert not index.launch()["wide"]
+            index.set_round_bases(limit)
+            got, total = index.query_records(bases, offsets)
+            assert total == want_total
+            np.testing.assert_array_equal(got, want)
     with zx.Index(ix) as index:
         index.set_round_bases(2 << 20)
         got, total = index.query_records(two, two_offsets, plain=True)
@@ -331,3 +333,95 @@ def test_key_lists_come_and_go_with_the_memory(gpu, oracle, tmp_path):
         del filler
         assert free() > before
         query()
+
+
+@pytest.mark.parametrize("opts", [dict(k=25, b=8), dict(mode="minimizers", k=25, m=21, b=16)],
+                         ids=["kmers", "minimizers"])
+def test_several_unsegmented_rounds(gpu, oracle, tmp_path, opts):
+    """Three rounds of 2^18 tiles: two key lists in turn, extraction beside the
+    probe, every order, windows and the wide probe, against the oracle and
+    the batch in one round."""
+    import zindex_b200 as zx
+
+    colors = 260 if opts["b"] == 8 else 130
+    fof = make_genomes(tmp_path / "g", colors, 3000, 31)
+    ix = build_index(fof, tmp_path / "index", H=4, min_docs=1, **opts)
+    pool = np.frombuffer(b"".join(dna(3000, 31 + c) for c in range(colors)), dtype=np.uint8)
+    rng = np.random.default_rng(17)
+    records, length = 600_000, 28
+    at = rng.integers(0, len(pool) - length, records)
+    bases = pool[at[:, None] + np.arange(length)].copy()
+    bases[rng.random(records) < 0.3, 5] = ord("N")
+    bases = bases.reshape(-1)
+    offsets = np.arange(records + 1, dtype=np.uint64) * length
+    with zx.Index(ix) as index:
+        for recover in (True, False):
+            want, want_total = oracle.query_records(ix, bases, offsets, recover=recover)
+            for limit in (1 << 20, 0):
+                index.set_round_bases(limit)
+                for order in (1, 2, 0):
+                    index.set_launch(wide=1, order=order, cut=1)
+                    got, total = index.query_records(bases, offsets, recover=recover)
+                    assert total == want_total
+                    np.testing.assert_array_equal(got, want)
+
+
+def test_split_rounds_of_a_launch_that_is_not_the_default(gpu, oracle, tmp_path):
+    """Split minimizer queries of narrow rows in three rounds: with the default
+    launch the batch takes the window probe."""
+    import zindex_b200 as zx
+
+    fof = make_genomes(tmp_path / "g", 20, 3000, 31)
+    ix = build_index(fof, tmp_path / "index", mode="minimizers", k=25, m=21, H=4, b=8, min_docs=1)
+    pool = np.frombuffer(b"".join(dna(3000, 31 + c) for c in range(20)), dtype=np.uint8)
+    records, length = 600_000, 27
+    at = np.random.default_rng(18).integers(0, len(pool) - length, records)
+    bases = pool[at[:, None] + np.arange(length)].reshape(-1).copy()
+    offsets = np.arange(records + 1, dtype=np.uint64) * length
+    want, want_total = oracle.query_records(ix, bases, offsets)
+    with zx.Index(ix) as index:
+        for launch in (dict(split=1, min_blocks=3), dict(split=0)):
+            index.set_launch(cut=1, **launch)
+            assert index.launch() != {**index.default_launch(), "cut": 1}
+            got, total = index.query_records(bases, offsets)
+            assert total == want_total
+            np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("opts", [dict(k=31, homopolymer=True), dict(k=45, homopolymer=True),
+                                  dict(k=21, pattern="##_#_##_#_#_#_##_#_##"),
+                                  dict(mode="minimizers", k=21, m=21),
+                                  dict(mode="minimizers", k=31, m=15, pattern="#####_###_#####")],
+                         ids=lambda o: "-".join(f"{k}{v}" for k, v in o.items()))
+@pytest.mark.parametrize("colors", [40, 270])
+def test_seed_options_of_dense_batches(gpu, oracle, tmp_path, opts, colors):
+    """Homopolymer compression, spaced seeds and every m-mer past 1 MiB: in
+    device memory, in chunks from pageable and joined from page-locked memory."""
+    import torch
+
+    import zindex_b200 as zx
+
+    fof = make_genomes(tmp_path / "g", colors, 3000, 31)
+    ix = build_index(fof, tmp_path / "index", **{**dict(H=4, b=8, min_docs=1), **opts})
+    genomes = [dna(3000, 31 + c) for c in range(colors)]
+    reads = sample_reads(genomes, np.random.default_rng(19), 14_500, 150, n_runs=0.05)
+    reads += [genomes[3][:40] + b"A" * 2000 + genomes[4][:900]] * 20
+    bases, offsets = zx.pack_records(reads)
+    assert len(bases) > 2 << 20
+    want, want_total = oracle.query_records(ix, bases, offsets)
+    dev = torch.device("cuda", 0)
+    with zx.Index(ix) as index:
+        assert index.launch()["wide"] == (colors > 250)
+        for source in (bases, torch.from_numpy(bases).pin_memory().numpy()):
+            got, total = index.query_records(source, offsets)
+            assert total == want_total
+            np.testing.assert_array_equal(got, want)
+        d_b = torch.from_numpy(bases).to(dev)
+        d_off = torch.from_numpy(offsets.view(np.int64)).to(dev)
+        counts = torch.zeros(colors, dtype=torch.int64, device=dev)
+        n = torch.zeros(1, dtype=torch.int64, device=dev)
+        index.query_device(d_b.data_ptr(), len(bases), d_off.data_ptr(), len(reads),
+                           counts.data_ptr(), n.data_ptr(), use_graph=False)
+        torch.cuda.synchronize(dev)
+        assert int(n) == want_total
+        np.testing.assert_array_equal(counts.cpu().numpy().view(np.uint64), want)
