@@ -1,5 +1,6 @@
-"""Batches past the size that is sorted and probed as one list, against the
-oracle: chunks and records of both sides of it in one host call."""
+"""Batches that are sorted and probed as one list, and those past that size or
+without memory for it, against the oracle; the planner's and the lists' bounds
+under offsets that go back; workspaces after a failed allocation."""
 import numpy as np
 import pytest
 
@@ -9,7 +10,16 @@ from helpers import build_index, dna, make_genomes, sample_reads
 pytestmark = pytest.mark.gpu
 
 
-def _narrow_index(tmp_path, colors=40, length=5000):
+def _lists_held(index) -> int:
+    """Bytes of the key lists that the index holds (it gives them back)."""
+    import torch
+
+    before = torch.cuda.mem_get_info()[0]
+    index.set_round_bases(0)
+    return torch.cuda.mem_get_info()[0] - before
+
+
+def _narrow_index(tmp_path, colors=240, length=3000):
     fof = make_genomes(tmp_path / "g", colors, length, 31)
     return (build_index(fof, tmp_path / "index", k=31, H=4, b=8, min_docs=1),
             [dna(length, 31 + c) for c in range(colors)])
@@ -21,28 +31,31 @@ def test_records_past_and_below_the_round_limit(gpu, oracle, tmp_path):
 
     ix, genomes = _narrow_index(tmp_path)
     rng = np.random.default_rng(11)
-    long = b"".join(sample_reads(genomes, rng, 16000, 150))  # 2.4e6 bases
-    reads = sample_reads(genomes, rng, 10500, 150, n_runs=0.05)
+    long = b"".join(sample_reads(genomes, rng, 34000, 150))  # 5.1e6 bases
+    reads = sample_reads(genomes, rng, 22000, 150, n_runs=0.05)
     bases, offsets = zx.pack_records([long] + reads)
-    chunks = np.searchsorted(offsets, [len(bases) // 3, len(bases) // 3 * 2])
-    sizes = np.diff(np.concatenate(([0], offsets[chunks], offsets[-1:])).astype(np.int64))
-    assert sizes[0] > 2 << 20 > sizes[2] > 1 << 20
+    cuts = np.searchsorted(offsets, [len(bases) // 4, len(bases) // 4 * 3])
+    sizes = np.diff(np.concatenate(([0], offsets[cuts], offsets[-1:])).astype(np.int64))
+    # (The last chunk is dense; the middle one is not.)
+    assert sizes[0] > 4 << 20 > sizes[2] > 2_000_000 and sizes[1] < 1_270_000
     want, want_total = oracle.query_records(ix, bases, offsets)
-    two, two_offsets = zx.pack_records([long, long[:1_500_000]])
+    two, two_offsets = zx.pack_records([long, long[:3_000_000]])
     want_two, want_two_total = oracle.query_records(ix, two, two_offsets)
     # (Without a limit: dense chunks on both sides of one that is not.)
-    for limit in (2 << 20, 0):
+    for limit in (4 << 20, 0):
         with zx.Index(ix) as index:
             assert not index.launch()["wide"]
             index.set_round_bases(limit)
             got, total = index.query_records(bases, offsets)
             assert total == want_total
             np.testing.assert_array_equal(got, want)
+            assert _lists_held(index) >= 16 * sizes[2]
     with zx.Index(ix) as index:
-        index.set_round_bases(2 << 20)
+        index.set_round_bases(4 << 20)
         got, total = index.query_records(two, two_offsets, plain=True)
         assert total == want_two_total
         np.testing.assert_array_equal(got, want_two)
+        assert _lists_held(index) >= 16 * 3_000_000
 
 
 @pytest.mark.parametrize("opts", [dict(), dict(mode="findere", k=31, z=10), dict(homopolymer=True),
@@ -255,15 +268,16 @@ def test_dense_batches_of_grouped_colours(gpu, oracle, tmp_path):
     rng = np.random.default_rng(15)
     genomes = [dna(960, 31 + int(c)) for c in rng.integers(4 * per_class, 5 * per_class, 200)]
     reads = sample_reads(genomes, rng, 300, 150)
-    # (Past 1 MiB by bases that are no seeds.)
-    bases, offsets = zx.pack_records([r + b"N" * 3500 for r in reads])
-    assert len(bases) > 1 << 20
+    # (Dense by bases that are no seeds.)
+    bases, offsets = zx.pack_records([r + b"N" * 60_000 for r in reads])
     want, want_total = oracle.query_records(ix, bases, offsets)
     with zx.Index(ix) as index:
         assert not index.launch()["wide"] and index.info.classes == 6
+        index.set_launch(cut=1)
         got, total = index.query_records(bases, offsets)
         assert total == want_total
         np.testing.assert_array_equal(got, want)
+        assert _lists_held(index) >= 16 * len(bases)
         index.set_launch(blocks=1000)  # no longer the default: the fused kernel
         got, total = index.query_records(bases, offsets)
         assert total == want_total
@@ -393,7 +407,7 @@ def test_split_rounds_of_a_launch_that_is_not_the_default(gpu, oracle, tmp_path)
                                   dict(mode="minimizers", k=21, m=21),
                                   dict(mode="minimizers", k=31, m=15, pattern="#####_###_#####")],
                          ids=lambda o: "-".join(f"{k}{v}" for k, v in o.items()))
-@pytest.mark.parametrize("colors", [40, 270])
+@pytest.mark.parametrize("colors", [240, 270])
 def test_seed_options_of_dense_batches(gpu, oracle, tmp_path, opts, colors):
     """Homopolymer compression, spaced seeds and every m-mer past 1 MiB: in
     device memory, in chunks from pageable and joined from page-locked memory."""
@@ -406,8 +420,8 @@ def test_seed_options_of_dense_batches(gpu, oracle, tmp_path, opts, colors):
     genomes = [dna(3000, 31 + c) for c in range(colors)]
     reads = sample_reads(genomes, np.random.default_rng(19), 14_500, 150, n_runs=0.05)
     reads += [genomes[3][:40] + b"A" * 2000 + genomes[4][:900]] * 20
-    bases, offsets = zx.pack_records(reads)
-    assert len(bases) > 2 << 20
+    # (Every chunk is dense, also by bases that are no seeds.)
+    bases, offsets = zx.pack_records([r + b"N" * 2500 for r in reads])
     want, want_total = oracle.query_records(ix, bases, offsets)
     dev = torch.device("cuda", 0)
     with zx.Index(ix) as index:
@@ -416,6 +430,7 @@ def test_seed_options_of_dense_batches(gpu, oracle, tmp_path, opts, colors):
             got, total = index.query_records(source, offsets)
             assert total == want_total
             np.testing.assert_array_equal(got, want)
+            assert _lists_held(index) >= 4 * len(bases)  # 16 a base of a chunk
         d_b = torch.from_numpy(bases).to(dev)
         d_off = torch.from_numpy(offsets.view(np.int64)).to(dev)
         counts = torch.zeros(colors, dtype=torch.int64, device=dev)
@@ -425,3 +440,94 @@ def test_seed_options_of_dense_batches(gpu, oracle, tmp_path, opts, colors):
         torch.cuda.synchronize(dev)
         assert int(n) == want_total
         np.testing.assert_array_equal(counts.cpu().numpy().view(np.uint64), want)
+
+
+def test_dense_batches_only_where_they_are_faster(gpu, tmp_path):
+    """One-chunk rows that L2 holds: sorting for the window probe does not pay
+    before tens of millions of bases. The default is at most a third slower
+    than the fused kernel at 1.3e6 bases (it was twice) and faster at 8e7."""
+    import subprocess
+
+    import torch
+
+    import zindex_b200 as zx
+
+    subprocess.run([str(helpers.ZX_BUILD), "--synth", "uniform:10:100000:100000:5", "-o",
+                    str(tmp_path / "index"), "-q", "-k", "31", "-H", "4", "-b", "8"], check=True)
+    dev = torch.device("cuda", 0)
+    acgt = torch.tensor(list(b"ACGT"), dtype=torch.uint8, device=dev)
+    torch.manual_seed(20)
+    with zx.Index(tmp_path / "index") as index:
+        counts = torch.zeros(10, dtype=torch.int64, device=dev)
+        total = torch.zeros(1, dtype=torch.int64, device=dev)
+        stream = torch.cuda.current_stream(dev).cuda_stream
+
+        def micros(bases, offsets):
+            best = float("inf")
+            for _ in range(20):
+                first, last = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+                first.record()
+                index.query_device(bases.data_ptr(), bases.numel(), offsets.data_ptr(),
+                                   offsets.numel() - 1, counts.data_ptr(), total.data_ptr(),
+                                   stream, use_graph=False)
+                last.record()
+                last.synchronize()
+                best = min(best, first.elapsed_time(last) * 1e3)
+            return best
+
+        ratio = {}
+        for records in (8_700, 540_000):
+            bases = acgt[torch.randint(0, 4, (records * 150,), device=dev)]
+            offsets = torch.arange(records + 1, dtype=torch.int64, device=dev) * 150
+            index.set_launch()
+            default = micros(bases, offsets)
+            index.set_launch(blocks=10_000)  # as many as fit: the default's grid
+            fused = micros(bases, offsets)
+            print(f"{records * 150} bases: default {default:.0f} us, fused {fused:.0f} us")
+            ratio[records] = default / fused
+        assert ratio[8_700] < 4 / 3 and ratio[540_000] < 1
+
+
+@pytest.mark.parametrize("case", [dict(colors=64, H=4, b=8, k=31), dict(colors=9, H=3, b=16, k=25),
+                                  dict(colors=30, H=2, b=4, k=45, groups="0,1;5,6"),
+                                  dict(colors=5, H=4, b=32, k=31),
+                                  dict(colors=100, H=16, b=8, k=31, max_size="256KiB"),
+                                  dict(colors=100, H=8, b=8, mode="modimizers", k=31, d=4),
+                                  dict(colors=100, H=4, b=8, mode="minimizers", k=31, m=21)],
+                         ids=lambda c: "-".join(f"{k}{v}" for k, v in c.items()))
+def test_dense_batches_past_their_threshold(gpu, oracle, tmp_path, case):
+    """Narrow rows of each width, hash count and seed mode in the window probe:
+    batches of 36 million bases, most of them no seeds, whole and in chunks."""
+    import torch
+
+    import zindex_b200 as zx
+
+    opts = dict(case)
+    colors = opts.pop("colors")
+    lengths = [2000 if c % 3 == 0 else (4000 if c % 3 == 1 else 9000) for c in range(colors)]
+    genomes = [dna(n, 31 + c) for c, n in enumerate(lengths)]
+    (tmp_path / "g").mkdir()
+    lines = []
+    for c, g in enumerate(genomes):
+        p = tmp_path / "g" / f"g{c}.fa"
+        helpers.write_fasta(p, [g])
+        lines.append(f"g{c}\t{p}")
+    (tmp_path / "fof.tsv").write_text("\n".join(lines) + "\n")
+    ix = build_index(tmp_path / "fof.tsv", tmp_path / "index", min_docs=1, **opts)
+    reads = sample_reads(genomes, np.random.default_rng(21), 8000, 151, n_runs=0.05)
+    bases, offsets = zx.pack_records([r + b"N" * 4400 for r in reads])
+    locked = torch.from_numpy(bases).pin_memory().numpy()
+    with zx.Index(ix) as index:
+        assert not index.launch()["wide"]
+        for recover in (True, False):
+            want, want_total = oracle.query_records(ix, bases, offsets, recover=recover)
+            index.set_launch(cut=1)
+            got, total = index.query_records(bases, offsets, recover=recover)
+            assert total == want_total
+            np.testing.assert_array_equal(got, want)
+            assert _lists_held(index) >= 16 * len(bases)
+            index.set_launch(cut=3)  # joined
+            got, total = index.query_records(locked, offsets, recover=recover)
+            assert total == want_total
+            np.testing.assert_array_equal(got, want)
+            assert _lists_held(index) >= 16 * len(bases)

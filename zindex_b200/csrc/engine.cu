@@ -1038,8 +1038,36 @@ void Engine::plan_windows() {
     for (const GroupMeta& g : m_.banks[cls[0]].groups) win_b16_ &= g.members.size() == 1;
   win_slices_ = (uint32_t)slices.size();
   win_weights_ = weights;
-  // Windows pay once a round's row reads are a few times the rows copied.
+  // Windows pay once a round's row reads are a few times the rows copied. The
+  // line is early for cheap rows, whose batches do not repay the 0.18 ms that
+  // windows cost whatever their size, and late for none: B200, sorted wide
+  // probe / windows, 256 colours H4 (line at 1.0e6 seeds) 0.24 / 0.39 ms at
+  // 1.0e6, 0.36 / 0.44 at 2.0e6, 0.60 / 0.57 at 4.1e6; 2,048 colours H3 b16
+  // (3.9e4) 0.25 / 0.24 ms at 3.2e4, 0.40 / 0.32 at 1.3e5; 16,384 colours H8
+  // b4 (4.0e4) 0.65 / 0.78 ms at 4.0e4, 1.30 / 0.89 at 7.9e4; 300 colours of
+  // short genomes H4 0.28 / 0.26 ms at 1.0e6.
   win_min_keys_ = std::max<uint64_t>(1, 4 * chunk_rows / (row_chunks * (uint64_t)H));
+
+  // Narrow rows: a dense batch starts behind the fused kernel by 0.115 ms
+  // (sort, three more launches) and a copy of the rows at 2.8 TB/s, and gains
+  // `gain` ps a base. Fitted to 58 geometries at 1.2e6 to 8.2e7 bases on a
+  // B200 (fused / dense ps a base: 1 chunk 31 / 26, 4 chunks 43 / 28, 8 chunks
+  // 66 / 34, 15 chunks 137 / 49, 16 hashes of 7 chunks 130 / 120, minimizers 37
+  // / 20, modimizers 15 / 8): nowhere more than 5 % slower than the fused
+  // kernel, 1 % from the faster of the two on average. With the seed count
+  // alone to decide, 10 colours of 100,000 bases took 0.21 ms instead of 0.10
+  // at 1.3e6 bases.
+  const uint32_t nc = wide_chunks();
+  const double rows = (double)chunk_rows * 16, l2 = (double)(64 << 20);
+  double gain = nc <= 2 ? 5 : nc <= 4 ? 11 + H : nc <= 8 ? 28 + H : 6.0 * nc;
+  if (H > 8) gain = nc <= 4 ? 5 : nc <= 8 ? 10 : 20;
+  if (sp_.klen > 32) gain += 13;
+  // (Row reads that miss L2, in windows read once.)
+  if (rows > l2)
+    gain = std::min(90.0, gain + 0.11 * (double)gather_sector_bytes_per_seed() * (1 - l2 / rows));
+  if (sp_.mode == kMinimizers && sp_.k != sp_.m) gain = 15;
+  if (sp_.mode == kModimizers) gain = sp_.klen > 32 ? 10 : 6;
+  dense_bases_ = (uint64_t)((115e6 + rows / 2.8) / gain);
 }
 
 uint64_t Engine::gather_sector_bytes_per_seed() const {
@@ -1158,7 +1186,7 @@ bool Engine::wide_form(const QueryLaunch& l) const { return l.wide && wide_eligi
 
 bool Engine::dense_batch(uint64_t nbases) const {
   if (!launch_default_ || launch_.wide || !win_slices_ || nbases <= kSmallBases ||
-      nbases > round_bases_)
+      nbases < dense_bases_ || nbases > round_bases_)
     return false;
   uint64_t seeds = nbases;
   if (sp_.mode == kMinimizers) seeds = 2 * nbases / (uint64_t)(sp_.ocm.w + 1);

@@ -376,7 +376,9 @@ class Engine {
   WinSlice* d_win_slices_ = nullptr;  // none: no window probe for this index
   uint32_t win_slices_ = 0, win_weights_ = 0;
   bool win_b16_ = false;  // 16-bit fields of single-member groups
-  uint64_t win_min_keys_ = ~0ull;
+  // Seeds from which windows read rows a few times; bases from which an index
+  // of narrow rows uses them.
+  uint64_t win_min_keys_ = ~0ull, dense_bases_ = ~0ull;
   uint64_t round_bases_ = 0;  // set_round_bases; kRoundKeys once loaded
   std::vector<void*> allocations_;
   uint64_t resident_bytes_ = 0;
