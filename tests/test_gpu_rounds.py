@@ -531,3 +531,30 @@ def test_dense_batches_past_their_threshold(gpu, oracle, tmp_path, case):
             assert total == want_total
             np.testing.assert_array_equal(got, want)
             assert _lists_held(index) >= 16 * len(bases)
+
+
+@pytest.mark.parametrize("colors", [12, 270], ids=["narrow", "wide"])
+def test_first_graph_of_a_homopolymer_index(gpu, oracle, tmp_path, colors):
+    """The compressed batch's buffers are there before the graph is captured."""
+    import torch
+
+    import zindex_b200 as zx
+
+    fof = make_genomes(tmp_path / "g", colors, 3000, 31)
+    ix = build_index(fof, tmp_path / "index", k=31, H=4, b=8, min_docs=1, homopolymer=True)
+    genomes = [dna(3000, 31 + c) for c in range(colors)]
+    dev = torch.device("cuda", 0)
+    with zx.Index(ix) as index:
+        for n in (50, 3000):
+            bases, offsets = zx.pack_records(sample_reads(genomes, np.random.default_rng(n), n, 150))
+            want, want_total = oracle.query_records(ix, bases, offsets)
+            d_b = torch.from_numpy(bases).to(dev)
+            d_off = torch.from_numpy(offsets.view(np.int64)).to(dev)
+            counts = torch.zeros(colors, dtype=torch.int64, device=dev)
+            total = torch.zeros(1, dtype=torch.int64, device=dev)
+            for replay in (1, 2):
+                index.query_device(d_b.data_ptr(), len(bases), d_off.data_ptr(), n,
+                                   counts.data_ptr(), total.data_ptr(), use_graph=True)
+                torch.cuda.synchronize(dev)
+                assert int(total) == replay * want_total
+                np.testing.assert_array_equal(counts.cpu().numpy().view(np.uint64), replay * want)

@@ -1356,8 +1356,14 @@ void Engine::set_round_bases(uint64_t bases) {
 
 bool Engine::give_back_lists() {
   if (!ws_ || !ws_->cap_round_keys) return false;
+  // (Refused while a caller captures: the lists then stay.)
+  if (cudaFree(ws_->round_keys[0]) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  ws_->round_keys[0] = nullptr;
+  drop(ws_->cap_round_keys, ws_->round_keys[1]);
   ws_->release_graphs();
-  drop(ws_->cap_round_keys, ws_->round_keys[0], ws_->round_keys[1]);
   return true;
 }
 
@@ -2371,6 +2377,7 @@ void Engine::query_device(Workspace& ws, const uint8_t* bases, uint64_t nbases,
                                 capturing == cudaStreamCaptureStatusNone;
   if (!free_to_allocate) cudaGetLastError();
   ensure_capacity(ws, nbases, records, false, nbases, free_to_allocate);
+  if (m_.homopolymer_compression) fit([&] { ensure_homopolymer_capacity(ws, nbases, records); });
   if (!use_graph) {
     enqueue(ws, bases, nbases, offsets, records, recover, counts, total, s);
     return;
