@@ -110,11 +110,6 @@ CONFIGS = {
 CONFIG = CONFIGS["c2"]
 WORKLOAD = CONFIG["workload"]
 METRIC = "query seeds/s"
-# DRAM bytes (read + write) per seed of the dominant kernel(s) of each workload, from
-# one ncu capture over the whole batch (the window probe copies each row a few times
-# per batch, so its bytes per seed fall as the batch grows and a slice says nothing
-# about it). Workloads without a capture report no traffic.
-TRAFFIC_BYTES_PER_SEED = {}
 # Per-record form: reads counted one by one, and the compact report threshold.
 PER_RECORD_READS = 200_000
 PER_RECORD_CPU_READS = 20_000
@@ -401,6 +396,57 @@ def hbm_peak():
         return FALLBACK_HBM_GBS, "fallback"
 
 
+def query_roofline(ix, seeds: int, nbases: int, kernel_ms: float) -> dict:
+    """What bounds the timed sequence (ix.last_kernel_ms: everything between
+    the tile plan and the counters). Batches whose row reads are four times
+    the rows take the window probe, which copies each window of rows once and
+    gathers every seed's rows from shared memory: its bound is 128 bytes per
+    clock and SM. Other batches read the rows from HBM or L2 in the wide probe
+    or the fused kernel: their bound is the copy rate. The sequence's other
+    kernels (extraction, sort) are part of the time and move none of these
+    bytes. No DRAM traffic is captured for a whole batch: traffic is null."""
+    import torch
+
+    info, launch = ix.info, ix.launch()
+    rec_bytes = 8 if info.abandoned_hashes else 0
+    row_bytes = seeds * info.gather_bytes_per_seed
+    alg = row_bytes + seeds * rec_bytes + nbases * 3 // 8
+    # The same gather in whole 32-byte DRAM sectors (each row touch costs its sectors).
+    sector = (seeds * (info.gather_sector_bytes_per_seed + (32 if rec_bytes else 0))
+              + nbases * 3 // 8)
+    seconds = kernel_ms / 1e3
+    common = {"unit": "GB/s", "kernel_ms": kernel_ms, "algorithmic_bytes_per_launch": int(alg),
+              "gather_bytes_per_seed": int(info.gather_bytes_per_seed),
+              "sector_bytes_per_seed": int(info.gather_sector_bytes_per_seed), "traffic": None}
+    if launch["wide"] and launch["order"] == 1 and row_bytes >= 4 * info.resident_bytes:
+        prop = torch.cuda.get_device_properties(torch.cuda.current_device())
+        mhz = nvidia_smi_max_sm_mhz()
+        peak = prop.multi_processor_count * 128 * mhz * 1e6 / 1e9
+        achieved = row_bytes / seconds / 1e9
+        return dict(common, bound="shared memory", achieved=achieved, peak=peak,
+                    frac=achieved / peak,
+                    peak_kind=f"128 B x {prop.multi_processor_count} SMs x {mhz:.0f} MHz",
+                    kernel="extract_dense_kernel, key sort, window_probe_kernel")
+    peak, kind = hbm_peak()
+    achieved = alg / seconds / 1e9
+    kernel = ("extract_dense_kernel, key sort, wide_probe_kernel" if launch["wide"] else
+              "findere_query_kernel or fused_query_kernel" if info.index_mode == 3 else
+              "fused_query_kernel")
+    return dict(common, bound="hbm", achieved=achieved, peak=peak, frac=achieved / peak,
+                peak_kind=kind, kernel=kernel, sector_achieved=sector / seconds / 1e9,
+                sector_frac=sector / seconds / 1e9 / peak)
+
+
+def nvidia_smi_max_sm_mhz() -> float:
+    try:
+        out = subprocess.run(["nvidia-smi", "--query-gpu=clocks.max.sm",
+                              "--format=csv,noheader,nounits"], capture_output=True, text=True,
+                             timeout=30, check=True).stdout
+        return float(out.split()[0])
+    except Exception:
+        return 1965.0
+
+
 class CpuOracle:
     """The oracle (CPU restatement of the reference query) with its index
     resident in host memory, timed on all host cores. The timed queries take
@@ -542,23 +588,16 @@ def other_config(zx, torch, name, cache: Path, steps: int):
             kms.append(ix.last_kernel_ms())
         ix.set_timing(False)
         kernel_ms = statistics.median(kms)
-        rec_bytes = 8 if info.abandoned_hashes else 0
-        alg = seeds * (info.gather_bytes_per_seed + rec_bytes) + len(bases) * 3 // 8
-        peak, peak_kind = hbm_peak()
+        roofline = query_roofline(ix, seeds, len(bases), kernel_ms)
         n = min(OTHER_CONFIGS[name], records)
         got, got_total = ix.query_records(bases[: int(offsets[n])], offsets[: n + 1])
         launch = ix.launch()
     orc = CpuOracle(index_dir)
     _, _, want = orc.run(bases, offsets, n, len(got), checker=True)
     orc.close()
-    achieved = alg / (kernel_ms / 1e3) / 1e9
     return {"workload": cfg["workload"], "value": seeds / (ms / 1e3), "unit": "seeds/s",
             "ms_per_step": ms, "steps": steps, "seeds_per_step": seeds,
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "peak_kind": peak_kind, "kernel_ms": kernel_ms,
-                         "algorithmic_bytes_per_launch": int(alg),
-                         "traffic": (TRAFFIC_BYTES_PER_SEED[name] * seeds / 1e9
-                                     if name in TRAFFIC_BYTES_PER_SEED else None)},
+            "roofline": roofline,
             "launch": launch, "resident_bytes": int(info.resident_bytes),
             "parity_vs_oracle_sample": bool(np.array_equal(got, want)),
             "parity_sample_reads": n}
@@ -679,8 +718,8 @@ def ours(args):
     launches = launches_per_step(ix, len(bases), records) * args.steps
 
     log("stage: kernel timing")
-    # Dominant kernel (fused extraction + probe) timed alone with CUDA events
-    # on its launch stream.
+    # The query's kernels after the tile plan, timed alone with CUDA events on
+    # their launch stream.
     ix.set_timing(True)
     kms = []
     for _ in range(max(3, min(args.steps, 10))):
@@ -688,15 +727,7 @@ def ours(args):
         kms.append(ix.last_kernel_ms())
     ix.set_timing(False)
     kernel_ms = statistics.median(kms)
-    gather = info.gather_bytes_per_seed
-    rec_bytes = 8 if info.abandoned_hashes else 0
-    alg_bytes = seeds * (gather + rec_bytes) + len(bases) * 3 // 8
-    peak, peak_kind = hbm_peak()
-    achieved = alg_bytes / (kernel_ms / 1e3) / 1e9
-    # The same gather in whole 32-byte DRAM sectors (each row touch costs its sectors).
-    sector = info.gather_sector_bytes_per_seed
-    sector_bytes = seeds * (sector + (32 if rec_bytes else 0)) + len(bases) * 3 // 8
-    sector_achieved = sector_bytes / (kernel_ms / 1e3) / 1e9
+    roofline = query_roofline(ix, seeds, len(bases), kernel_ms)
 
     log("stage: end to end")
     # End to end through the C ABI with pinned host buffers.
@@ -883,18 +914,8 @@ def ours(args):
             "e2e": {"value": e2e_rate, "unit": "seeds/s",
                     "h2d_bytes_per_step": int(len(bases) + 8 * (records + 1)),
                     "d2h_bytes_per_step": int(8 * ix.colors + 8)},
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak,
-                         "traffic": (TRAFFIC_BYTES_PER_SEED[args.config] * seeds / 1e9
-                                     if args.config in TRAFFIC_BYTES_PER_SEED else None),
-                         "traffic_unit": "GB",
-                         "peak_kind": peak_kind,
-                         "kernel": "fused_query_kernel", "kernel_ms": kernel_ms,
-                         "algorithmic_bytes_per_launch": int(alg_bytes),
-                         "gather_bytes_per_seed": int(gather),
-                         "sector_bytes_per_seed": int(sector),
-                         "sector_achieved": sector_achieved, "sector_frac": sector_achieved / peak,
-                         "l2_resident": bool(info.resident_bytes < (126 << 20))},
+            "roofline": dict(roofline, traffic_unit="GB",
+                             l2_resident=bool(info.resident_bytes < (126 << 20))),
             "forms": {"plain_seeds_per_s": plain_rate, "batched_seeds_per_s": value / world,
                       "served_seeds_per_s": served["closed_loop"]["seeds_per_s"],
                       "planned_seeds_per_s": world * planned["seeds_per_s"],

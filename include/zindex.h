@@ -83,10 +83,13 @@ typedef struct zx_launch {
                          team, planes, stage_bytes and split are then unused */
   int order;          /* wide-row form, unsegmented queries: 1 = each round's seeds are sorted
                          by their first hash before the probe (every class's row index grows
-                         with it, so consecutive seeds read neighbouring rows), each block
-                         probing runs of 256 consecutive seeds; 2 = sorted, and block b
-                         probes seeds b, b + blocks, ... (all blocks on neighbouring seeds);
-                         0 = extraction order; ignored elsewhere. Counts do not depend on it */
+                         with it, so consecutive seeds read neighbouring rows): rounds of many
+                         more seeds than rows gather the rows from windows of them copied to
+                         shared memory, others probe runs of up to 256 consecutive seeds per
+                         block, and far fewer seeds than rows stay unsorted; 2 = sorted, and
+                         block b probes seeds b, b + blocks, ... (all blocks on neighbouring
+                         seeds); 0 = extraction order; ignored elsewhere. Counts do not depend
+                         on it */
 } zx_launch;
 
 /* Thread-local message of the last failed call on this thread. */
@@ -198,7 +201,12 @@ int zx_extract_seeds(zx_index* index, const uint8_t* bases, const uint64_t* offs
                      uint64_t records, uint64_t* out, uint64_t cap, uint64_t* count);
 
 /* Launch configuration of the batched kernels (autotuner / planner hook;
- * never changes results). */
+ * never changes results). An index whose default is not the wide-row form
+ * (wide = 0) runs unsegmented batches of many more seeds than rows through
+ * the wide-row form's sort and window probe all the same, as long as its
+ * launch is the default one (cut, stages and bulk may differ): fields set
+ * to other values than zx_default_launch's name the fused kernel, for every
+ * batch. Setting the fields of zx_get_launch restores what it described. */
 int zx_get_launch(const zx_index* index, zx_launch* out);
 int zx_set_launch(zx_index* index, const zx_launch* launch);
 int zx_default_launch(const zx_index* index, zx_launch* out);
@@ -227,9 +235,11 @@ int zx_set_round_bases(zx_index* index, uint64_t bases);
 int zx_query_status(zx_index* index);
 
 /* Measurement hook: with timing on, zx_query_device calls made with
- * use_graph == 0 record CUDA events around the fused extraction+probe kernel
- * on the launch stream; zx_last_kernel_ms waits for the last such kernel and
- * returns its duration in milliseconds. */
+ * use_graph == 0 record CUDA events around the kernels that follow the tile
+ * plan on the launch stream: the fused extraction and probe kernel, or the
+ * rounds of extraction, sort and probe of a split or wide-row query.
+ * zx_last_kernel_ms waits for the last such interval and returns its duration
+ * in milliseconds. */
 int zx_set_timing(zx_index* index, int on);
 int zx_last_kernel_ms(zx_index* index, float* ms);
 

@@ -1724,7 +1724,11 @@ void Engine::run_wide(Workspace& ws, const QueryLaunch& l, const BatchView& bv,
       sg.key_cap = ws.cap_round_keys;
       sg.err = ws.error;
     }
-    // (Seeds far fewer than the rows share none worth bringing together.)
+    // Seeds far fewer than the rows share none worth bringing together. (B200,
+    // wide probe unsorted / sorted, 256 colours, line at 1.3e5 seeds: 0.07 /
+    // 0.12 ms there, 0.14 / 0.18 at 5e5, 0.39 / 0.36 at 2.1e6, 0.68 / 0.62 at
+    // 4.2e6; 16,384 colours H8 b4, line at 5e3: 0.19 / 0.22, 1.48 / 1.30 at
+    // 7.9e4, 3.87 / 2.80 at 3.2e5. The line could lie later.)
     const bool ordered =
         !segments && (l.order == 2 || (l.order == 1 && (!win_slices_ || max_keys >= win_min_keys_ / 8)));
     if (ordered) ensure_order_capacity(ws, b, whole);
@@ -2458,10 +2462,13 @@ void Engine::query_host(Workspace& ws, const uint8_t* bases, uint64_t nbases,
   const bool direct_offsets = pinned(offsets);
   // Wide-row and dense batches in page-locked memory: every chunk's seeds join
   // one key list while the next chunk is copied, and the list is sorted and
-  // probed once (a probe per chunk copies every window again: on a B200
-  // 250,000 reads of 256 colours in four chunks took 3.66 ms, joined 2.96 ms).
-  // Staging pageable memory takes longer than the probes, which then hide
-  // behind it chunk by chunk.
+  // probed once: a probe per chunk copies every window again. B200, reads of
+  // 150 bases in four chunks, apart / joined: 256 colours 0.89 / 0.61 ms for
+  // 20,000, 1.86 / 1.05 for 60,000, 3.61 / 2.94 for 250,000, 10.04 / 10.31 for
+  // 1,000,000; 64 colours 2.71 / 2.16 for 250,000, 6.95 / 7.49 for 1,000,000
+  // (chunks of that size hide their probes behind the copy). Staging pageable
+  // memory takes longer than the probes, which then hide behind it chunk by
+  // chunk.
   const bool joined = direct && chunks > 1 && nbases <= round_bases_ && (wide_form(launch_) || dense_batch(nbases));
   ensure_capacity(ws, nbases, records + chunks, false, joined ? nbases : most_at_once);
   ensure_host_capacity(ws, nbases, records + chunks);

@@ -28,8 +28,10 @@
 // * Recovered origins are counted once per seed, when the keys are sorted
 //   (block_count_kernel).
 //
-// Bound by shared-memory bandwidth (75-81 % of 128 bytes per clock and SM; the
-// wide probe was bound by L2 latency). B200, kernel time, wide probe -> here:
+// Bound by shared-memory bandwidth: 91 % of the data pipe (128 bytes per clock
+// and SM) on rows of 512 chunks H8 b4, 93 % on 256 chunks H3 b16, 78 % on 16
+// chunks H4 b8, where the ALU is busy for 68 % (the wide probe was bound by
+// L2 latency). B200, kernel time, wide probe -> here:
 // 31.4e6 seeds of 256 colours H4 b8 3.41 -> 1.40 ms, 2.4e6 of 16,384 colours H8
 // b4 12.64 -> 6.15 ms, 9.5e6 of 2,048 colours H3 b16 15.3 -> 4.73 ms. Warps
 // take seeds and blocks take work as they get free: in fixed shares the first
